@@ -19,7 +19,7 @@
 //              pores other than the voxel's owner record, per voxel and pore, their first
 //              touch time (extensions).
 // Frontier sizes stay on the device; the next generation is compacted in event order (see
-// ws_generations).
+// ws_generations; ws_small runs the small generations).
 //
 // Voxel state: one 64-bit word per voxel holds the claim state, which is the untouched mark,
 // the smallest touch of the running generation (kTouched | event), or the claimer (pore
@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "devutil.cuh"
@@ -75,6 +76,10 @@ struct WsState {
     uint32_t* ext_next;           // [records]: the voxel's next record + 1, 0 = none
     unsigned int* ext_count;
     uint32_t ext_cap;
+    ulonglong2* log;              // extending touches not recorded yet: (time, pore << 32 | voxel);
+                                  // ~0 in entries that were reserved and not used
+    unsigned long long* log_n;    // entries reserved (may pass log_cap)
+    uint32_t log_cap;
     unsigned int* pbound;         // per pore
     unsigned int* err;
     int spin_limit;               // polls of one wait on another block before giving up
@@ -83,8 +88,7 @@ struct WsState {
                                   // [192], [193]: block 0's ns resolving events, scan + look-back
     int time_shift;               // bucket entry time = (generation << time_shift) | event
     uint8_t* ev_touch;            // per event slot: phase 0 touched an unclaimed voxel
-    const unsigned long long* boff;  // bucket offsets
-    unsigned int* bfill;
+    unsigned long long* bpos;        // per depth: where its bucket's next entry goes
     unsigned long long* ent_time;
     unsigned long long* ent_val;
 };
@@ -134,6 +138,16 @@ __global__ void ws_seed_entries(const unsigned long long* __restrict__ a, size_t
         ent_time[a[k]] = a[np + k];
         ent_val[a[k]] = a[2 * np + k];
     }
+}
+
+// A frontier node: its voxel and its pore index, with kFace set when the voxel lies on a face of
+// the volume (the other nodes' neighbours are all inside: no coordinates to work out).
+constexpr uint32_t kFace = 0x80000000u;
+
+__device__ __forceinline__ uint32_t ws_node(const Grid& g, uint32_t v, uint32_t pore) {
+    int x, y, z;
+    g.coords(v, x, y, z);
+    return g.on_face(x, y, z) ? pore | kFace : pore;
 }
 
 // Voxel count per containing radius. Few distinct radii take most voxels, so counts gather
@@ -201,8 +215,13 @@ __device__ __forceinline__ uint32_t ws_follow(uint32_t* link, const WsState& s) 
 // Out of line: it is the rare path of the touch kernel. Slots fill in order along the
 // voxel's record chain, so two touches by one pore meet at the same slot.
 __device__ __noinline__ void ws_extend(const WsState& s, size_t w, uint32_t pore, unsigned long long t) {
-    uint32_t rec = ws_follow(s.ext + w, s);
-    for (int hop = 0; hop < kMaxHops && rec; ++hop) {
+    uint32_t* link = s.ext + w;
+    uint32_t rec = 0;
+#pragma unroll 1
+    for (int hop = 0; hop < kMaxHops; ++hop) {
+        rec = ws_follow(link, s);
+        if (!rec) break;
+#pragma unroll 1
         for (int k = 0; k < kSlots; ++k) {
             const size_t slot = static_cast<size_t>(rec - 1) * kSlots + k;
             const uint32_t cur = atomicCAS(&s.ext_pore[slot], kNone, pore);
@@ -211,9 +230,40 @@ __device__ __noinline__ void ws_extend(const WsState& s, size_t w, uint32_t pore
                 return;
             }
         }
-        if (hop + 1 < kMaxHops) rec = ws_follow(s.ext_next + (rec - 1), s);
+        link = s.ext_next + (rec - 1);
     }
     if (rec) atomicOr(s.err, 2u);  // more extending pores than neighbours: cannot happen
+}
+
+// The flood itself only notes extending touches in a log, and ws_record_extensions records them
+// later, one thread per entry: a record takes up to six dependent atomics, which would lengthen
+// every generation by their latency (a touch of the flood waits for one), and claims never
+// depend on extensions. A touch that finds the log full records itself in line. (640 x 600 x 672
+// spinodal: generations of 2^13 nodes 23.8 -> 17 us, of 2^16 87 -> 70; stage 361 -> 315 ms.)
+// Out of line, like ws_extend: the generation loops run once through a long way of code per
+// generation, and inlined copies of the rare paths cost them instruction cache misses.
+__device__ __noinline__ void ws_note(const WsState& s, uint32_t w, uint32_t pore, unsigned long long t) {
+    const unsigned peers = __activemask();
+    const int leader = __ffs(peers) - 1;
+    const unsigned lane = threadIdx.x & 31;
+    unsigned long long first = 0;
+    if (static_cast<int>(lane) == leader) first = atomicAdd(s.log_n, static_cast<unsigned long long>(__popc(peers)));
+    first = __shfl_sync(peers, first, leader);
+    const unsigned long long pos = first + __popc(peers & ((1u << lane) - 1u));
+    if (pos < s.log_cap) s.log[pos] = make_ulonglong2(t, (static_cast<unsigned long long>(pore) << 32) | w);
+    else ws_extend(s, w, pore, t);
+}
+
+__global__ void ws_record_extensions(WsState s, uint32_t begin, uint32_t end) {
+    PMA_GRID_STRIDE(k, end - begin) {
+        const ulonglong2 e = s.log[begin + k];
+        if (e.y != ~0ull) ws_extend(s, static_cast<uint32_t>(e.y), static_cast<uint32_t>(e.y >> 32), e.x);
+    }
+}
+
+// The neighbour of v at an offset that stays inside the volume (indices fit 32 bits).
+__device__ __forceinline__ uint32_t ws_neighbour(const WsState& s, uint32_t v, int dx, int dy, int dz) {
+    return v + (static_cast<uint32_t>(dz) * s.g.SX + dx) * s.g.SY + dy;  // modulo 2^32
 }
 
 // Touch events of the generation's nodes. Phase 0 claims: the smallest touch time of each
@@ -235,14 +285,17 @@ __device__ __forceinline__ void ws_claim_event(const WsState& s, const uint32_t*
     int dx, dy, dz;
     if (stencil_offset(j, s.d3q7, dx, dy, dz)) {
         const uint32_t v = __ldcg(gv + i);
-        const uint32_t pore = __ldcg(gp + i);
-        int x, y, z;
-        s.g.coords(v, x, y, z);
-        const int nx = x + dx, ny = y + dy, nz = z + dz;
-        if (!s.g.inside(nx, ny, nz)) {  // WC.cpp:140-144
+        const uint32_t node = __ldcg(gp + i), pore = node & ~kFace;
+        bool inside = true;
+        if (node & kFace) {
+            int x, y, z;
+            s.g.coords(v, x, y, z);
+            inside = s.g.inside(x + dx, y + dy, z + dz);
+        }
+        if (!inside) {  // WC.cpp:140-144
             s.pbound[pore] = 1;
         } else {
-            const size_t w = s.g.idx(nx, ny, nz);
+            const uint32_t w = ws_neighbour(s, v, dx, dy, dz);
             uint32_t r;
             unsigned long long st;
             ws_load(s, w, r, st);
@@ -251,7 +304,7 @@ __device__ __forceinline__ void ws_claim_event(const WsState& s, const uint32_t*
                     atomicMin(&s.state[w], ws_word(s.packed, kTouched | seq, r));
                     touched = 1;
                 } else if (st - 1 != pore) {
-                    ws_extend(s, w, pore, (gen << 40) | seq);
+                    ws_note(s, w, pore, (gen << 40) | seq);
                 }
             }
         }
@@ -259,53 +312,62 @@ __device__ __forceinline__ void ws_claim_event(const WsState& s, const uint32_t*
     s.ev_touch[seq] = touched;
 }
 
-// Returns true when the event claims a voxel of the same depth (a node of the next
-// generation: voxel nw of pore np_out).
+// Appends the claim of voxel w (radius r, below the running depth) to its depth's bucket. Lanes
+// appending to the same depth take their slots with one atomic: a generation's claims of
+// shallower voxels mostly go to a few depths, and one counter per depth would serialise them.
+__device__ __forceinline__ void ws_append(const WsState& s, unsigned lanes, uint32_t w, uint32_t pore, uint32_t r,
+                                          unsigned long long seq, unsigned long long gen) {
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(lanes, r);
+    const int leader = __ffs(peers) - 1;
+    unsigned long long first = 0;
+    if (static_cast<int>(lane) == leader) first = atomicAdd(&s.bpos[r], static_cast<unsigned long long>(__popc(peers)));
+    first = __shfl_sync(peers, first, leader);
+    const unsigned long long at = first + __popc(peers & ((1u << lane) - 1u));
+    s.ent_time[at] = (gen << s.time_shift) | seq;
+    s.ent_val[at] = (static_cast<unsigned long long>(pore) << 32) | w;
+}
+
+// Resolves event seq if it touched an unclaimed voxel: the winner records its claim, every other
+// touch by a pore other than the winner's is an extension. Returns true when the event claims a
+// voxel of the same depth (a node of the next generation).
 __device__ __forceinline__ bool ws_resolve_event(const WsState& s, const uint32_t* gv, const uint32_t* gp,
-                                                 unsigned long long seq, uint32_t depth, unsigned long long gen,
-                                                 uint32_t& nw, uint32_t& np_out) {
+                                                 unsigned long long seq, uint32_t depth, unsigned long long gen) {
     const unsigned long long i = seq / 27;
     const int j = static_cast<int>(seq - i * 27);
     // the node (shared by the event's warp neighbours) is loaded along with the flag
     const uint8_t touched = __ldcg(s.ev_touch + seq);
     const uint32_t v = __ldcg(gv + i);
-    const uint32_t pore = __ldcg(gp + i);
+    const uint32_t pore = __ldcg(gp + i) & ~kFace;
     if (!touched) return false;
     int dx, dy, dz;
     stencil_offset(j, s.d3q7, dx, dy, dz);
     // the neighbour is inside the box (phase 0 touched it)
-    const size_t w = static_cast<size_t>(static_cast<long long>(v) +
-                                         (static_cast<long long>(dz) * s.g.SX + dx) * s.g.SY + dy);
+    const uint32_t nw = ws_neighbour(s, v, dx, dy, dz);
     uint32_t r;
     unsigned long long st;
-    ws_load(s, w, r, st);
-    if (st == (kTouched | seq)) {
-        s.state[w] = ws_word(s.packed, pore + 1, r);  // one 64-bit store: readers see either word
-        if (r == depth) {
-            nw = static_cast<uint32_t>(w);
-            np_out = pore;
-            return true;
-        }
-        // lanes of the warp appending to the same depth take their slots with one atomic: a
-        // generation's claims of shallower voxels mostly go to a few depths, and one counter
-        // per depth would serialise them
-        const unsigned active = __activemask();
-        const unsigned peers = __match_any_sync(active, r);
-        const int leader = __ffs(peers) - 1;
-        const unsigned lane = threadIdx.x & 31;
-        unsigned first = 0;
-        if (static_cast<int>(lane) == leader) first = atomicAdd(&s.bfill[r], static_cast<unsigned>(__popc(peers)));
-        first = __shfl_sync(peers, first, leader);
-        const unsigned pos = first + __popc(peers & ((1u << lane) - 1u));
-        const unsigned long long at = s.boff[r] + pos;
-        s.ent_time[at] = (gen << s.time_shift) | seq;
-        s.ent_val[at] = (static_cast<unsigned long long>(pore) << 32) | w;
+    ws_load(s, nw, r, st);
+    if (st == (kTouched | seq)) {  // the winner
+        s.state[nw] = ws_word(s.packed, pore + 1, r);  // one 64-bit store: readers see either word
+        if (r == depth) return true;
+        ws_append(s, __activemask(), nw, pore, r, seq, gen);
         return false;
     }
     // the winner's pore: already stored as the claimer, or that of the winning touch's node
-    const uint32_t owner = st < kTouched ? static_cast<uint32_t>(st - 1) : __ldcg(gp + (st & kSeqMask) / 27);
-    if (owner != pore) ws_extend(s, w, pore, (gen << 40) | seq);
+    const uint32_t owner = st < kTouched ? static_cast<uint32_t>(st - 1) : __ldcg(gp + (st & kSeqMask) / 27) & ~kFace;
+    if (owner != pore) ws_note(s, nw, pore, (gen << 40) | seq);
     return false;
+}
+
+// Writes the node that event seq gave.
+__device__ __forceinline__ void ws_put_node(const WsState& s, const uint32_t* gv, const uint32_t* gp,
+                                            unsigned long long seq, uint32_t* v_out, uint32_t* p_out) {
+    const unsigned long long i = seq / 27;
+    int dx, dy, dz;
+    stencil_offset(static_cast<int>(seq - i * 27), s.d3q7, dx, dy, dz);
+    const uint32_t w = ws_neighbour(s, __ldcg(gv + i), dx, dy, dz);
+    *v_out = w;
+    *p_out = ws_node(s.g, w, __ldcg(gp + i) & ~kFace);
 }
 
 // Ordered compaction of a generation's same-depth claims into the next frontier, in event
@@ -443,12 +505,13 @@ __device__ __forceinline__ unsigned long long ws_clock() {  // ns
 
 // Up to max_gens generations of one depth in a single cooperative launch, two grid-wide
 // barriers per generation. ng[2] holds the two frontier sizes; the frontier starts on side
-// `cur`. out[0] = generations run, out[1] = the side holding the next frontier.
+// `cur`. The launch ends early when the frontier has at most small_nodes nodes. out[0] =
+// generations run, out[1] = the side holding the next frontier.
 __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint32_t* gv0, uint32_t* gp0, uint32_t* gv1,
                                                              uint32_t* gp1, unsigned int* ng,
                                                              unsigned long long* desc, uint32_t depth,
                                                              unsigned long long gen0, int max_gens, int cur,
-                                                             unsigned long long* out) {
+                                                             unsigned small_nodes, unsigned long long* out) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
     __shared__ unsigned int part[33];
@@ -459,7 +522,7 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
     int it = 0;
     for (; it < max_gens; ++it) {
         const unsigned long long nev = static_cast<unsigned long long>(__ldcg(ng + cur)) * 27;
-        if (nev == 0) break;
+        if (nev <= static_cast<unsigned long long>(small_nodes) * 27) break;  // ws_small goes on
         ++gen;
         const int hc = min(63, 63 - __clzll(nev / 27));
         unsigned long long t_start = 0;
@@ -503,8 +566,7 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
                 unsigned cnt = 0;
                 for (unsigned long long st = w0; st < w1; ++st) {
                     const unsigned long long seq = st * 32 + lane;
-                    uint32_t wv, wp;
-                    const bool f = seq < nev && ws_resolve_event(s, gv, gp, seq, depth, gen, wv, wp);
+                    const bool f = seq < nev && ws_resolve_event(s, gv, gp, seq, depth, gen);
                     if (f) s.ev_touch[seq] = 2;
                     cnt += __popc(__ballot_sync(0xFFFFFFFFu, f));
                 }
@@ -533,36 +595,12 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
                     atomicAdd(&s.gen_hist[193], tc - tb);
                 }
                 unsigned long long pos = static_cast<unsigned long long>(part[32]) + part[warp];
-                // four steps at a time, every load issued before the stores
-                for (unsigned long long st = w0; st < w1; st += 4) {
-                    bool f[4];
-                    uint32_t v[4], pr[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const unsigned long long seq = (st + k) * 32 + lane;
-                        f[k] = st + k < w1 && seq < nev && __ldcg(s.ev_touch + seq) == 2;  // L2: no stale L1 line
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const unsigned long long i = ((st + k) * 32 + lane) / 27;
-                        v[k] = f[k] ? __ldcg(gv + i) : 0u;
-                        pr[k] = f[k] ? __ldcg(gp + i) : 0u;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const unsigned m = __ballot_sync(0xFFFFFFFFu, f[k]);
-                        if (f[k]) {
-                            const unsigned long long seq = (st + k) * 32 + lane;
-                            const int j = static_cast<int>(seq - seq / 27 * 27);
-                            int dx, dy, dz;
-                            stencil_offset(j, s.d3q7, dx, dy, dz);
-                            const unsigned long long at = pos + __popc(m & lt);
-                            nv[at] = static_cast<uint32_t>(static_cast<long long>(v[k]) +
-                                                           (static_cast<long long>(dz) * s.g.SX + dx) * s.g.SY + dy);
-                            np_[at] = pr[k];
-                        }
-                        pos += __popc(m);
-                    }
+                for (unsigned long long st = w0; st < w1; ++st) {
+                    const unsigned long long seq = st * 32 + lane;
+                    const bool f = seq < nev && __ldcg(s.ev_touch + seq) == 2;  // L2: no stale L1 line
+                    const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
+                    if (f) ws_put_node(s, gv, gp, seq, nv + (pos + __popc(m & lt)), np_ + (pos + __popc(m & lt)));
+                    pos += __popc(m);
                 }
             }
         } else
@@ -571,15 +609,14 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
         for (unsigned long long c = blockIdx.x; c < nchunks; c += gridDim.x) {
             const bool probe = s.gen_hist && blockIdx.x == 0 && threadIdx.x == 0;  // block 0's split
             const unsigned long long ta = probe ? ws_clock() : 0;
-            bool f[4];
-            uint32_t wv[4], wp[4];
-            unsigned m[4];
+            unsigned won = 0;  // bit k: the thread's k-th event gives a node of the next generation
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const unsigned long long seq = c * kChunk + k * (kChunk / 4) + threadIdx.x;
-                f[k] = seq < nev && ws_resolve_event(s, gv, gp, seq, depth, gen, wv[k], wp[k]);
-                m[k] = __ballot_sync(0xFFFFFFFFu, f[k]);
-                if (lane == 0) part[k * (kChunk / 128) + warp] = __popc(m[k]);
+                const bool f = seq < nev && ws_resolve_event(s, gv, gp, seq, depth, gen);
+                if (f) won |= 1u << k;
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
+                if (lane == 0) part[k * (kChunk / 128) + warp] = __popc(m);
             }
             __syncthreads();
             const unsigned long long tb = probe ? ws_clock() : 0;
@@ -606,12 +643,14 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
             }
             const unsigned base = part[32];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (f[k]) {
-                    const unsigned pos = base + part[k * (kChunk / 128) + warp] + __popc(m[k] & lt);
-                    nv[pos] = wv[k];
-                    np_[pos] = wp[k];
+            for (int k = 0; k < 4; ++k) {
+                const bool f = (won >> k) & 1u;
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
+                if (f) {
+                    const unsigned pos = base + part[k * (kChunk / 128) + warp] + __popc(m & lt);
+                    ws_put_node(s, gv, gp, c * kChunk + k * (kChunk / 4) + threadIdx.x, nv + pos, np_ + pos);
                 }
+            }
             __syncthreads();  // part is reused by the next chunk
         }
         grid.sync();
@@ -624,52 +663,518 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
     }
 }
 
-// A small depth bucket (n <= kSmallBucket entries) sorted by time in one block and unpacked
-// into the first generation, with its size; replaces a radix sort and two more launches.
-constexpr int kSmallBucket = 2048;
+// --- small generations --------------------------------------------------------------------
+//
+// Most generations are small (a few to a few thousand nodes) and their time is latency: in
+// ws_generations a generation of 2^6 to 2^10 nodes takes 10 to 14 us (two barriers over the whole
+// grid, the look-back, one launch and one host round trip per depth). ws_small runs them in one
+// thread-block cluster, and goes from depth to depth by itself: it sorts a depth's bucket in
+// shared memory, runs its generations and takes the next depth, until a bucket or a frontier is
+// too large for it (the host then sorts that bucket and runs ws_generations until the frontier
+// is small again). Generations of at most kSoloNodes nodes run in the cluster's first block
+// alone, with the frontier in shared memory and block barriers; larger ones split their nodes
+// over the blocks, one contiguous run each, with three cluster barriers.
+// What bounds a generation: latency (a block barrier 50 cycles, a cluster barrier 400 and with it
+// the wait for the atomics in flight, an L2 load 300 to 700), and one sector a clock and SM for the
+// scattered state words; hence 16 blocks, and 64 nodes as the most for one block alone. From about
+// 2000 nodes the whole grid is faster (2^11 nodes: 20 us here, 16 there; 2^10: 13.5 against 15.7).
+// Whole stage, before and after (ms): 40 x 48 x 44 union 15.6 -> 5.2, 128^3 union 48.5 -> 30.7,
+// 300 x 341 x 277 spinodal 135 -> 119.
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallCluster = 16;       // blocks
+constexpr int kSmallSort = 8192;        // bucket entries sorted in shared memory
+constexpr unsigned kSoloNodes = 64;
+constexpr unsigned kSmallNodes = 2048;
+constexpr int kStage = kSmallNodes / kSmallCluster;  // nodes a block holds in shared memory
+static_assert(kSoloNodes <= kStage && kStage <= kSmallThreads, "a block's nodes are staged whole, one a thread");
+static_assert((kStage * 27 + kSmallThreads - 1) / kSmallThreads + 1 <= 32, "a thread's touch flags are one 32-bit word");
+constexpr unsigned kSmallUps = 1024;    // claims of shallower voxels a block keeps until they go to their buckets
+constexpr unsigned kLogSlab = 512;      // extension log entries a block of ws_small takes at a time
 
-__global__ void __launch_bounds__(1024) ws_sort_small(const unsigned long long* __restrict__ time,
-                                                      const unsigned long long* __restrict__ val, unsigned n,
-                                                      uint32_t* __restrict__ gv, uint32_t* __restrict__ gp,
-                                                      unsigned int* __restrict__ ng) {
-    __shared__ unsigned long long st[kSmallBucket];
-    __shared__ unsigned long long sv[kSmallBucket];
-    unsigned N = 1;
-    while (N < n) N <<= 1;
-    for (unsigned i = threadIdx.x; i < N; i += blockDim.x) {
-        st[i] = i < n ? time[i] : ~0ull;
-        sv[i] = i < n ? val[i] : 0ull;
-    }
-    __syncthreads();
-    for (unsigned k = 2; k <= N; k <<= 1)  // bitonic sort by time (times are distinct)
-        for (unsigned j = k >> 1; j > 0; j >>= 1) {
-            for (unsigned i = threadIdx.x; i < N; i += blockDim.x) {
-                const unsigned q = i ^ j;
-                if (q > i) {
-                    const unsigned long long a = st[i], c = st[q];
-                    if (((i & k) == 0) ? (a > c) : (a < c)) {
-                        st[i] = c;
-                        st[q] = a;
-                        const unsigned long long t = sv[i];
-                        sv[i] = sv[q];
-                        sv[q] = t;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
-        gv[i] = static_cast<uint32_t>(sv[i]);
-        gp[i] = static_cast<uint32_t>(sv[i] >> 32);
-    }
-    if (threadIdx.x == 0) *ng = n;
+enum WsMode { kWsDone = 0, kWsRun = 1, kWsSort = 2, kWsBig = 3, kWsLimit = 4, kWsGrow = 5 };
+
+struct WsCtl {  // where the flood stands
+    unsigned long long gen;
+    uint32_t di;   // index into the depth list
+    uint32_t n;    // frontier nodes (kWsSort: entries of the bucket)
+    uint32_t cur;  // side of the frontier
+    uint32_t mode;
+};
+
+struct WsSmallArgs {
+    uint32_t *gv0, *gp0, *gv1, *gp1;
+    const uint32_t* depths;  // depths that can hold entries, deepest first
+    uint32_t ndepths;
+    const unsigned long long* boff;  // per depth: the first entry of its bucket
+    unsigned long long max_gen;
+};
+
+struct WsSmallShared {
+    uint32_t v[2][kStage], p[2][kStage];  // staged nodes
+    unsigned long long up_time[kSmallUps], up_val[kSmallUps];  // claims of shallower voxels, as in a bucket
+    uint32_t up_r[kSmallUps];                                  // their radii
+    uint32_t ups;
+    uint32_t won[kStage];    // per node: stencil positions of its same-depth claims
+    uint32_t sum[kSmallWarps];
+    uint32_t total[kSmallCluster];
+    uint32_t delta[27];      // index step of a stencil position
+    uint32_t log_base, log_used;  // the block's slab of the extension log
+    WsCtl ctl;
+};
+
+// Notes the extending touches of a warp (all 32 lanes call; ext = this lane has one) in the
+// block's slab: a shared-memory counter instead of a round trip to the log's.
+__device__ __forceinline__ void ws_small_note(const WsState& s, WsSmallShared& sh, bool ext, uint32_t w, uint32_t pore,
+                                              unsigned long long t) {
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, ext);
+    if (!m) return;
+    const unsigned lane = threadIdx.x & 31;
+    uint32_t first = 0;
+    if (lane == 0) first = atomicAdd(&sh.log_used, static_cast<uint32_t>(__popc(m)));
+    first = __shfl_sync(0xFFFFFFFFu, first, 0);
+    if (!ext) return;
+    const uint32_t pos = first + __popc(m & ((1u << lane) - 1u));
+    if (pos < kLogSlab && sh.log_base + pos < s.log_cap)
+        s.log[sh.log_base + pos] = make_ulonglong2(t, (static_cast<unsigned long long>(pore) << 32) | w);
+    else ws_note(s, w, pore, t);  // slab full
 }
 
-__global__ void ws_unpack_entries(const unsigned long long* __restrict__ val, size_t n,
+// A new slab for the block when the present one is more than half used (or there is none).
+__device__ __forceinline__ void ws_small_slab(const WsState& s, WsSmallShared& sh) {
+    if (threadIdx.x == 0 && sh.log_used > kLogSlab / 2) {
+        sh.log_base = static_cast<uint32_t>(min(atomicAdd(s.log_n, static_cast<unsigned long long>(kLogSlab)), 0x7FFFFFFFull));
+        sh.log_used = 0;
+    }
+}
+
+// Moves the block's list of claims of shallower voxels to their depths' buckets. Keeping them here
+// over many generations takes the wait for the bucket's counter out of each of them.
+__device__ __noinline__ void ws_small_flush(const WsState& s, WsSmallShared& sh) {
+    __syncthreads();
+    const uint32_t k = min(sh.ups, kSmallUps);
+    for (uint32_t i = threadIdx.x; i < k; i += kSmallThreads) {
+        const unsigned long long at = atomicAdd(&s.bpos[sh.up_r[i]], 1ull);
+        s.ent_time[at] = sh.up_time[i];
+        s.ent_val[at] = sh.up_val[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sh.ups = 0;
+    __syncthreads();
+}
+
+// One generation of n nodes; returns the next frontier's size. cl: all blocks of the cluster, each
+// a contiguous run of the nodes, staged from gv/gp; else one block, the frontier in sh.v[side].
+// A thread takes an event at a time: a warp's lanes then meet three neighbours of a row in one
+// 32-byte sector (an SM serves about one sector a clock, which bounds a block's generation).
+__device__ __noinline__ uint32_t ws_small_generation(const WsState& s, WsSmallShared& sh, bool cl, const uint32_t* gv,
+                                                     const uint32_t* gp, uint32_t* nv, uint32_t* np_, int side, uint32_t n,
+                                                     uint32_t depth, unsigned long long gen) {
+    namespace cg = cooperative_groups;
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t first = 0, m = n;  // the block's nodes
+    if (cl) {
+        const uint32_t per = (n + kSmallCluster - 1) / kSmallCluster;
+        first = min(cg::this_cluster().block_rank() * per, n);
+        m = min(per, n - first);
+        side = 0;
+        if (tid < m) {
+            sh.v[0][tid] = __ldcg(gv + first + tid);
+            sh.p[0][tid] = __ldcg(gp + first + tid);
+        }
+    }
+    if (tid < m) sh.won[tid] = 0;
+    __syncthreads();
+    const uint32_t nev = m * 27, seq0 = first * 27;
+    // claims, as ws_claim_event; bit k of touched: this thread's k-th event touched an unclaimed
+    // voxel. Two events a turn, their loads in flight together.
+    uint32_t touched = 0;
+#pragma unroll 1
+    for (unsigned k = 0; k * kSmallThreads + warp * 32 < nev; k += 2) {
+        unsigned long long word[2];
+        uint32_t rad[2], w[2], pore[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t e = (k + u) * kSmallThreads + tid, i = e < nev ? e / 27 : 0;
+            const int j = static_cast<int>(e - i * 27);
+            int dx, dy, dz;
+            word[u] = 0;  // radius 0
+            rad[u] = 0;
+            w[u] = pore[u] = 0;
+            if (e >= nev || !stencil_offset(j, s.d3q7, dx, dy, dz)) continue;
+            const uint32_t v = sh.v[side][i], node = sh.p[side][i];
+            pore[u] = node & ~kFace;
+            w[u] = v + sh.delta[j];
+            if (node & kFace) {
+                int x, y, z;
+                s.g.coords(v, x, y, z);
+                if (!s.g.inside(x + dx, y + dy, z + dz)) {  // WC.cpp:140-144
+                    s.pbound[pore[u]] = 1;
+                    continue;
+                }
+            }
+            word[u] = __ldcg(s.state + w[u]);
+            if (!s.packed) rad[u] = __ldg(s.crad + w[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t seq = seq0 + (k + u) * kSmallThreads + tid;
+            const uint32_t r = s.packed ? static_cast<uint32_t>(word[u] & 0xFFFFu) : rad[u];
+            const unsigned long long st = s.packed ? word[u] >> 16 : word[u];
+            const bool in = r != 0 && r <= depth, ext = in && st < kTouched && st - 1 != pore[u];  // WC.cpp:152-156
+            if (in && st >= kTouched) {
+                atomicMin(&s.state[w[u]], ws_word(s.packed, kTouched | seq, r));
+                touched |= 1u << (k + u);
+            }
+            if (__any_sync(0xFFFFFFFFu, ext)) ws_small_note(s, sh, ext, w[u], pore[u], (gen << 40) | seq);
+        }
+    }
+    if (cl) cg::this_cluster().sync();
+    else __syncthreads();
+    // resolve the touches, as ws_resolve_event; a claim of the same depth sets its stencil
+    // position's bit in its node's word
+#pragma unroll 1
+    for (unsigned k = 0; k * kSmallThreads + warp * 32 < nev; k += 2) {
+        if (!__any_sync(0xFFFFFFFFu, (touched >> k) & 3u)) continue;
+        unsigned long long word[2];
+        uint32_t rad[2], w[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            word[u] = 0;
+            rad[u] = w[u] = 0;
+            if (!((touched >> (k + u)) & 1u)) continue;
+            const uint32_t e = (k + u) * kSmallThreads + tid, i = e / 27;
+            w[u] = sh.v[side][i] + sh.delta[e - i * 27];
+            word[u] = __ldcg(s.state + w[u]);
+            if (!s.packed) rad[u] = __ldg(s.crad + w[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t e = (k + u) * kSmallThreads + tid, i = e / 27, seq = seq0 + e;
+            bool ext = false;
+            uint32_t pore = 0;
+            if ((touched >> (k + u)) & 1u) {
+                pore = sh.p[side][i] & ~kFace;
+                const uint32_t r = s.packed ? static_cast<uint32_t>(word[u] & 0xFFFFu) : rad[u];
+                const unsigned long long st = s.packed ? word[u] >> 16 : word[u];
+                if (st == (kTouched | seq)) {
+                    s.state[w[u]] = ws_word(s.packed, pore + 1, r);
+                    if (r == depth) {
+                        atomicOr(&sh.won[i], 1u << (e - i * 27));
+                    } else {  // to its depth's bucket, by way of the block's list
+                        const uint32_t at = atomicAdd(&sh.ups, 1u);
+                        if (at < kSmallUps) {
+                            sh.up_time[at] = (gen << s.time_shift) | seq;
+                            sh.up_val[at] = (static_cast<unsigned long long>(pore) << 32) | w[u];
+                            sh.up_r[at] = r;
+                        } else {
+                            ws_append(s, __activemask(), w[u], pore, r, seq, gen);
+                        }
+                    }
+                } else if (st < kTouched) {
+                    ext = static_cast<uint32_t>(st - 1) != pore;
+                } else {
+                    const uint32_t node = static_cast<uint32_t>((st & kSeqMask) / 27);
+                    ext = ((node - first < m ? sh.p[side][node - first] : __ldcg(gp + node)) & ~kFace) != pore;
+                }
+            }
+            if (__any_sync(0xFFFFFFFFu, ext)) ws_small_note(s, sh, ext, w[u], pore, (gen << 40) | seq);
+        }
+    }
+    __syncthreads();
+    ws_small_slab(s, sh);
+    // offsets in event order: nodes, then stencil positions
+    uint32_t won = tid < m ? sh.won[tid] : 0u;
+    uint32_t incl = __popc(won);
+    const uint32_t mine = incl;
+    if (warp * 32 < m) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= static_cast<unsigned>(o)) incl += t;
+        }
+    }
+    if (lane == 31) sh.sum[warp] = incl;
+    __syncthreads();
+    const uint32_t sums = lane < kSmallWarps ? sh.sum[lane] : 0u;
+    uint32_t next = __reduce_add_sync(0xFFFFFFFFu, sums);
+    uint32_t pos = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? sums : 0u) + incl - mine;
+    if (cl) {
+        cg::cluster_group cluster = cg::this_cluster();
+        const unsigned rank = cluster.block_rank();
+        if (tid < kSmallCluster) cluster.map_shared_rank(sh.total, tid)[rank] = next;
+        cluster.sync();
+        next = 0;
+#pragma unroll 1
+        for (unsigned b = 0; b < kSmallCluster; ++b) {
+            if (b < rank) pos += sh.total[b];
+            next += sh.total[b];
+        }
+    }
+    if (won) {
+        const uint32_t v = sh.v[side][tid], pore = sh.p[side][tid] & ~kFace;
+        for (; won; won &= won - 1, ++pos) {
+            const uint32_t w = v + sh.delta[__ffs(won) - 1], node = ws_node(s.g, w, pore);
+            nv[pos] = w;
+            np_[pos] = node;
+            if (!cl && pos < kSoloNodes) {
+                sh.v[side ^ 1][pos] = w;
+                sh.p[side ^ 1][pos] = node;
+            }
+        }
+    }
+    if (sh.ups > kSmallUps / 2) ws_small_flush(s, sh);  // the same for the whole block: nobody adds now
+    if (cl) cg::this_cluster().sync();
+    else __syncthreads();
+    return next;
+}
+
+// Shared memory of a bucket's sort, in the dynamic part (the cluster's first block uses it).
+constexpr int kSortDigit = 6;  // bits of a radix pass: 64 digits x 32 warps of counters
+struct WsSortShared {
+    unsigned long long time[2][kSmallSort];
+    uint16_t at[2][kSmallSort];
+    uint16_t rank[kSmallSort];  // within the entry's warp and digit
+    uint32_t count[(1 << kSortDigit) * (kSmallWarps + 1)];  // [digit][warp], a row of one more: fewer bank conflicts
+    unsigned long long vary[kSmallWarps];
+    uint32_t sum[kSmallWarps];
+};
+static_assert((1 << kSortDigit) * kSmallWarps == 2 * kSmallThreads, "two counters a thread");
+constexpr uint32_t kRankSort = kSmallThreads / 4;  // buckets this small are sorted by counting
+
+// Sorts the n entries of a depth's bucket by time (times are distinct) and writes the depth's
+// first generation, in shared memory too. Up to kRankSort entries: each finds its rank by
+// comparing itself with every other, four threads an entry. Larger: stable radix passes over the
+// bits in which the times differ, each warp ranking its own run of the entries by ballots. (A bitonic sort,
+// with a block barrier per step, took 5.4 us for 100 entries and 20 us for 1300.)
+__device__ __noinline__ void ws_small_bucket(const WsState& s, WsSmallShared& sh, WsSortShared& so, unsigned long long off, uint32_t n,
+                                uint32_t* gv, uint32_t* gp) {
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+    auto put = [&](uint32_t pos, uint32_t at) {  // entry `at` becomes node `pos`
+        const unsigned long long val = __ldcg(s.ent_val + off + at);
+        const uint32_t v = static_cast<uint32_t>(val), node = ws_node(s.g, v, static_cast<uint32_t>(val >> 32));
+        gv[pos] = v;
+        gp[pos] = node;
+        if (pos < kSoloNodes) {
+            sh.v[0][pos] = v;
+            sh.p[0][pos] = node;
+        }
+    };
+    if (n <= kRankSort) {
+        if (tid < n) so.time[0][tid] = __ldcg(s.ent_time + off + tid);
+        __syncthreads();
+        const uint32_t i = tid >> 2;
+        const unsigned long long mine = i < n ? so.time[0][i] : 0ull;
+        uint32_t below = 0;
+        if (warp * 8 < n)
+#pragma unroll 4
+            for (uint32_t k = tid & 3; k < n; k += 4) below += so.time[0][k] < mine ? 1u : 0u;
+        below += __shfl_xor_sync(0xFFFFFFFFu, below, 1);
+        below += __shfl_xor_sync(0xFFFFFFFFu, below, 2);
+        if (i < n && (tid & 3) == 0) put(below, i);
+        __syncthreads();
+        return;
+    }
+    // the bits in which the times differ
+    unsigned long long vary = 0;
+    const unsigned long long t0 = __ldcg(s.ent_time + off);
+    for (uint32_t i = tid; i < n; i += kSmallThreads) {
+        const unsigned long long t = __ldcg(s.ent_time + off + i);
+        so.time[0][i] = t;
+        so.at[0][i] = static_cast<uint16_t>(i);
+        vary |= t ^ t0;
+    }
+    for (int o = 16; o > 0; o >>= 1) vary |= __shfl_xor_sync(0xFFFFFFFFu, vary, o);
+    if (lane == 0) so.vary[warp] = vary;
+    __syncthreads();
+    vary = so.vary[lane % kSmallWarps];
+    for (int o = 16; o > 0; o >>= 1) vary |= __shfl_xor_sync(0xFFFFFFFFu, vary, o);
+    // warp w's run: steps of 32 entries
+    const uint32_t steps = (n + kSmallThreads - 1) / kSmallThreads, run = warp * steps * 32;
+    int src = 0;
+    for (; vary; src ^= 1) {
+        const int shift = __ffsll(static_cast<long long>(vary)) - 1;  // the next pass starts at a bit that varies
+        vary = shift + kSortDigit < 64 ? vary & (~0ull << (shift + kSortDigit)) : 0ull;
+        for (uint32_t i = tid; i < (1u << kSortDigit) * (kSmallWarps + 1); i += kSmallThreads) so.count[i] = 0;
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t k = 0; k < steps && run + k * 32 < n; ++k) {
+            const uint32_t i = run + k * 32 + lane;
+            const bool in = i < n;
+            const uint32_t d = in ? static_cast<uint32_t>(so.time[src][i] >> shift) & ((1u << kSortDigit) - 1u) : 0u;
+            unsigned peers = __ballot_sync(0xFFFFFFFFu, in);
+#pragma unroll
+            for (int b = 0; b < kSortDigit; ++b) {
+                const unsigned set = __ballot_sync(0xFFFFFFFFu, (d >> b) & 1u);
+                peers &= (d >> b) & 1u ? set : ~set;
+            }
+            const int leader = __ffs(peers) - 1;
+            uint32_t first = 0;
+            if (in && static_cast<int>(lane) == leader) {  // the warp's own counter: no other warp writes it
+                first = so.count[d * (kSmallWarps + 1) + warp];
+                so.count[d * (kSmallWarps + 1) + warp] = first + __popc(peers);
+            }
+            first = __shfl_sync(0xFFFFFFFFu, first, leader & 31) + __popc(peers & lt);
+            if (in) so.rank[i] = static_cast<uint16_t>(first);
+            __syncwarp();
+        }
+        __syncthreads();
+        // exclusive scan of the counters, digits first, then warps: two a thread
+        uint32_t* two = so.count + (2 * tid / kSmallWarps) * (kSmallWarps + 1) + 2 * tid % kSmallWarps;
+        const uint32_t c0 = two[0], c1 = two[1];
+        uint32_t incl = c0 + c1;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= static_cast<unsigned>(o)) incl += t;
+        }
+        if (lane == 31) so.sum[warp] = incl;
+        __syncthreads();
+        uint32_t before = lane < warp ? so.sum[lane] : 0u;  // lane < warp < kSmallWarps
+        before = __reduce_add_sync(0xFFFFFFFFu, before) + incl - c0 - c1;
+        two[0] = before;
+        two[1] = before + c0;
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t k = 0; k < steps; ++k) {
+            const uint32_t i = run + k * 32 + lane;
+            if (i >= n) break;
+            const unsigned long long t = so.time[src][i];
+            const uint32_t d = static_cast<uint32_t>(t >> shift) & ((1u << kSortDigit) - 1u);
+            const uint32_t pos = so.count[d * (kSmallWarps + 1) + warp] + so.rank[i];
+            so.time[src ^ 1][pos] = t;
+            so.at[src ^ 1][pos] = so.at[src][i];
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = tid; i < n; i += kSmallThreads) put(i, so.at[src][i]);
+    __syncthreads();
+}
+
+// Runs the flood from ctl (depth index, frontier) on; leaves in ctl where it stopped and why.
+__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallThreads, 1)
+    ws_small(WsState s, WsSmallArgs a, WsCtl* ctl) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ WsSmallShared sh;
+    extern __shared__ __align__(16) unsigned char dynamic[];
+    WsSortShared& so = *reinterpret_cast<WsSortShared*>(dynamic);
+    const unsigned tid = threadIdx.x, lane = tid & 31, rank = cl.block_rank();
+    if (tid < 27) {
+        int dx, dy, dz;
+        stencil_offset(static_cast<int>(tid), 0, dx, dy, dz);
+        sh.delta[tid] = static_cast<uint32_t>((dz * static_cast<long long>(s.g.SX) + dx) * s.g.SY + dy);
+    }
+    if (tid == 0) {
+        sh.log_used = kLogSlab;  // no slab yet
+        sh.ups = 0;
+    }
+    WsCtl c = *ctl;
+    bool staged = false;  // the first block: the frontier is in sh.v[cur]
+    ws_small_slab(s, sh);
+    __syncthreads();
+    auto timed = [&](unsigned long long t0, uint32_t n) {  // the generation's class and time, in the claim slot
+        if (!s.gen_hist || rank != 0 || tid != 0) return;
+        const int hc = 31 - __clz(n);
+        atomicAdd(&s.gen_hist[hc], 1ull);
+        atomicAdd(&s.gen_hist[64 + hc], ws_clock() - t0);
+    };
+    for (;;) {
+        if (rank == 0) {  // solo generations, bucket sorts and the way from depth to depth
+            c.mode = kWsDone;
+            for (;;) {
+                // the host empties the log (and adds records) before it fills up
+                if ((c.n == 0 || (c.gen & 15) == 0) && 2ull * __ldcg(s.log_n) > s.log_cap) {
+                    c.mode = kWsGrow;
+                    break;
+                }
+                if (c.n == 0) {  // the deepest depth with entries: 32 at a time
+                    uint32_t n0 = 0;
+                    for (; c.di < a.ndepths; c.di += 32) {
+                        uint32_t f = 0;
+                        if (c.di + lane < a.ndepths) {
+                            const uint32_t d = a.depths[c.di + lane];
+                            f = static_cast<uint32_t>(__ldcg(s.bpos + d) - __ldg(a.boff + d));
+                        }
+                        const unsigned m = __ballot_sync(0xFFFFFFFFu, f != 0);
+                        if (m) {
+                            const int l = __ffs(m) - 1;
+                            n0 = __shfl_sync(0xFFFFFFFFu, f, l);
+                            c.di += l;
+                            break;
+                        }
+                    }
+                    if (n0 == 0) break;  // done
+                    c.n = n0;
+                    if (n0 > kSmallSort) {
+                        c.mode = kWsSort;
+                        break;
+                    }
+                    c.cur = 0;
+                    ws_small_bucket(s, sh, so, __ldg(a.boff + a.depths[c.di]), n0, a.gv0, a.gp0);
+                    staged = true;
+                }
+                if (c.gen >= a.max_gen) {
+                    c.mode = kWsLimit;
+                    break;
+                }
+                if (c.n > kSoloNodes) {
+                    c.mode = c.n > kSmallNodes ? kWsBig : kWsRun;
+                    staged = false;
+                    break;
+                }
+                uint32_t* gv = c.cur ? a.gv1 : a.gv0;
+                uint32_t* gp = c.cur ? a.gp1 : a.gp0;
+                if (!staged) {
+                    if (tid < c.n) {
+                        sh.v[c.cur][tid] = __ldcg(gv + tid);
+                        sh.p[c.cur][tid] = __ldcg(gp + tid);
+                    }
+                    staged = true;
+                    __syncthreads();
+                }
+                ++c.gen;
+                const unsigned long long t0 = s.gen_hist ? ws_clock() : 0;
+                const uint32_t n = ws_small_generation(s, sh, false, gv, gp, c.cur ? a.gv0 : a.gv1, c.cur ? a.gp0 : a.gp1,
+                                                              static_cast<int>(c.cur), c.n, a.depths[c.di], c.gen);
+                timed(t0, c.n);
+                c.n = n;
+                c.cur ^= 1;
+                if (n == 0) {
+                    ++c.di;
+                    ws_small_flush(s, sh);
+                }
+            }
+            if (c.mode != kWsRun) ws_small_flush(s, sh);
+            if (tid == 0) sh.ctl = c;
+        }
+        cl.sync();
+        if (rank != 0) c = *cl.map_shared_rank(&sh.ctl, 0);
+        if (c.mode != kWsRun) break;
+        while (c.n > kSoloNodes && c.n <= kSmallNodes && c.gen < a.max_gen) {
+            ++c.gen;
+            const unsigned long long t0 = s.gen_hist ? ws_clock() : 0;
+            const uint32_t n = ws_small_generation(s, sh, true, c.cur ? a.gv1 : a.gv0, c.cur ? a.gp1 : a.gp0,
+                                                         c.cur ? a.gv0 : a.gv1, c.cur ? a.gp0 : a.gp1, 0, c.n,
+                                                         a.depths[c.di], c.gen);
+            timed(t0, c.n);
+            c.n = n;
+            c.cur ^= 1;
+            if ((c.gen & 15) == 0) break;  // the first block looks at the log
+        }
+        // every block's claims are in their buckets before the first block reads one
+        ws_small_flush(s, sh);
+        cl.sync();
+        if (c.n == 0) ++c.di;
+    }
+    if (rank == 0 && tid == 0) *ctl = c;
+    cl.sync();  // no block ends while another reads its shared memory
+}
+
+__global__ void ws_unpack_entries(const unsigned long long* __restrict__ val, size_t n, Grid g,
                                   uint32_t* __restrict__ gv, uint32_t* __restrict__ gp) {
     PMA_GRID_STRIDE(i, n) {
-        gv[i] = static_cast<uint32_t>(val[i]);
-        gp[i] = static_cast<uint32_t>(val[i] >> 32);
+        const uint32_t v = static_cast<uint32_t>(val[i]);
+        gv[i] = v;
+        gp[i] = ws_node(g, v, static_cast<uint32_t>(val[i] >> 32));
     }
 }
 
@@ -861,6 +1366,19 @@ __global__ void ws_group_rows(const uint32_t* __restrict__ grep, size_t ngr, con
     }
 }
 
+// The dynamic shared-memory limit is a process-wide attribute of the kernel: set once per device.
+void small_smem_attribute() {
+    static std::mutex mutex;
+    static std::vector<int> devices;
+    int dev = 0;
+    PMA_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mutex);
+    if (std::find(devices.begin(), devices.end(), dev) != devices.end()) return;
+    PMA_CUDA(cudaFuncSetAttribute(ws_small, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(WsSortShared)));
+    PMA_CUDA(cudaFuncSetAttribute(ws_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    devices.push_back(dev);
+}
+
 template <class T>
 T* buf(pma_ctx* ctx, const char* tag, size_t count) {
     return static_cast<T*>(ctx->scratch(tag, std::max<size_t>(count, 1) * sizeof(T)));
@@ -873,6 +1391,7 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     KernelTimer kt_stage(ctx, "stage_watershed");  // the whole stage, for the untimed remainder
     check_dims(d);
     PMA_REQUIRE(crad2 && labels, PMA_ERR_ARGUMENT, "pma_watershed: null device pointer");
+    PMA_REQUIRE(pt->pores.size() < kFace, PMA_ERR_ARGUMENT, "pma_watershed: too many pores");
     cudaStream_t s = ctx->stream;
     const size_t n = voxels(d);
     const Grid g{d.sx, d.sy, d.sz};
@@ -900,6 +1419,7 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
                     "pma_watershed: two pores share a seed voxel");
     }
 
+    small_smem_attribute();
     int64_t* d_count = buf<int64_t>(ctx, "ws.count", 4);
     unsigned int* d_ng = reinterpret_cast<unsigned int*>(d_count + 3);  // two frontier sizes
     WsState ws;
@@ -919,8 +1439,8 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     }
     ws.pbound = buf<unsigned int>(ctx, "ws.pbound", npores);
     // Shared-voxel records: a first guess of n/32; the pool doubles (copying the records)
-    // whenever it is more than half used at a host synchronisation point, and a flood that
-    // still runs out is redone with four times as many (up to two per voxel).
+    // whenever it is more than half used when the log is emptied, and a flood that still runs
+    // out is redone with four times as many (up to two per voxel).
     const size_t max_records = std::min<size_t>(2 * n + 4096, 0x7FFFFFFF / kSlots);
     size_t ext_cap = std::min<size_t>(std::max<size_t>(n / 32, 4096), max_records);
     int ext_side = 0;  // which of two scratch tags holds the records
@@ -949,9 +1469,36 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
         ws.ext_next = nn_;
         ws.ext_cap = static_cast<uint32_t>(cap2);
     };
+    // Extension log: emptied when it is more than half full at a host synchronisation point.
+    const size_t log_cap = std::min<size_t>(n / 8 + (1u << 16), 1u << 30);
+    ws.log = buf<ulonglong2>(ctx, "ws.log", log_cap);
+    ws.log_cap = static_cast<uint32_t>(log_cap);
+    ws.log_n = reinterpret_cast<unsigned long long*>(d_count);  // counts other things after the flood
+    size_t used = 0;  // records in use when the log was last emptied
+    auto record_extensions = [&](unsigned long long reserved) {
+        const size_t noted = static_cast<size_t>(std::min<unsigned long long>(reserved, log_cap));
+        unsigned int* h_used = static_cast<unsigned int*>(ctx->host_staging(128)) + 28;
+        size_t at = 0;
+        // each entry takes at most one new record: as many entries as records are free at a time
+        while (at < noted) {
+            size_t m = noted - at;
+            if (ws.ext_cap < max_records) m = std::min<size_t>(m, std::max<size_t>(ws.ext_cap - std::min<size_t>(used, ws.ext_cap), 1));
+            ws_record_extensions<<<grid_for(ctx, m), 256, 0, s>>>(ws, static_cast<uint32_t>(at), static_cast<uint32_t>(at + m));
+            ctx->check_launch("ws_record_extensions");
+            at += m;
+            ReadBack rb;
+            rb.add(h_used, ws.ext_count, 4);
+            read_back(ctx, rb);
+            used = *h_used;
+            grow_records(used);
+        }
+        PMA_CUDA(cudaMemsetAsync(ws.log, 0xFF, noted * sizeof(ulonglong2), s));
+        PMA_CUDA(cudaMemsetAsync(ws.log_n, 0, 8, s));
+    };
     unsigned int h_err = 0;
     for (;;) {
         const size_t start_cap = ext_cap;
+        used = 0;
         ws.ext_cap = static_cast<uint32_t>(ext_cap);
         ws.ext_pore = buf<uint32_t>(ctx, ext_tag("ws.ext_pore").c_str(), static_cast<size_t>(ws.ext_cap) * kSlots);
         ws.ext_time = buf<unsigned long long>(ctx, ext_tag("ws.ext_time").c_str(),
@@ -959,6 +1506,7 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
         ws.ext_next = buf<uint32_t>(ctx, ext_tag("ws.ext_next").c_str(), ws.ext_cap);
         PMA_CUDA(cudaMemsetAsync(ws.ext_next, 0, static_cast<size_t>(ws.ext_cap) * 4, s));
         PMA_CUDA(cudaMemsetAsync(d_count, 0, 32, s));
+        PMA_CUDA(cudaMemsetAsync(ws.log, 0xFF, log_cap * sizeof(ulonglong2), s));
         PMA_CUDA(cudaMemsetAsync(ws.ext_pore, 0xFF, static_cast<size_t>(ws.ext_cap) * kSlots * 4, s));
         PMA_CUDA(cudaMemsetAsync(ws.ext_time, 0xFF, static_cast<size_t>(ws.ext_cap) * kSlots * 8, s));
         PMA_CUDA(cudaMemsetAsync(ws.pbound, 0, std::max<size_t>(npores, 1) * 4, s));
@@ -982,8 +1530,7 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
         }
         const unsigned long long total = boff[nb];
         auto* d_boff = buf<unsigned long long>(ctx, "ws.boff", nb + 1);
-        ws.boff = d_boff;
-        ws.bfill = buf<unsigned int>(ctx, "ws.bfill", nb);
+        ws.bpos = buf<unsigned long long>(ctx, "ws.bpos", nb);
         ws.ent_time = buf<unsigned long long>(ctx, "ws.ent_time", total);
         ws.ent_val = buf<unsigned long long>(ctx, "ws.ent_val", total);
         auto* srt_time = buf<unsigned long long>(ctx, "ws.srt_time", max_bucket);
@@ -1019,7 +1566,9 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
             ctx->check_launch("ws_seed");
             ctx->sync();
         }
-        PMA_CUDA(cudaMemcpyAsync(ws.bfill, h_fill.data(), nb * 4ull, cudaMemcpyHostToDevice, s));
+        std::vector<unsigned long long> bpos(boff.begin(), boff.end() - 1);
+        for (uint32_t b = 0; b < nb; ++b) bpos[b] += h_fill[b];
+        PMA_CUDA(cudaMemcpyAsync(ws.bpos, bpos.data(), nb * 8ull, cudaMemcpyHostToDevice, s));
         ctx->sync();
 
         // Depth sweep (WatershedComputer.cpp:80-102).
@@ -1036,78 +1585,83 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
         const size_t coop_need = (max_events + 16 * (kChunk / 4) - 1) / (16 * (kChunk / 4));
         const unsigned coop_grid = static_cast<unsigned>(
             std::max<size_t>(1, std::min<size_t>(coop_need, static_cast<size_t>(ctx->num_sms) * std::min(per_sm, 8))));
-        unsigned long long gen = 0;
         // generations of this call at most: the context's bound, within the entry-time range
         const unsigned long long max_gen =
             std::min<unsigned long long>(ctx->limits.watershed_generations, kMaxGen - 1);
-        unsigned int* h_small = static_cast<unsigned int*>(ctx->host_staging(64));
+        // pinned words: frontier sizes and the record count, the launches' results, the flood's state
+        unsigned int* h_small = static_cast<unsigned int*>(ctx->host_staging(128));
+        auto* h_log_n = reinterpret_cast<unsigned long long*>(h_small + 4);
         auto* d_out = buf<unsigned long long>(ctx, "ws.coop_out", 2);
         unsigned long long* h_out = reinterpret_cast<unsigned long long*>(h_small + 8);
+        auto* d_ctl = reinterpret_cast<WsCtl*>(buf<unsigned long long>(ctx, "ws.ctl", 3));
+        static_assert(sizeof(WsCtl) == 24, "three words");
+        WsCtl* h_ctl = reinterpret_cast<WsCtl*>(h_small + 16);
         // depths that can hold entries, deepest first
-        std::vector<int64_t> depths;
+        std::vector<uint32_t> depths;
         for (int64_t depth = static_cast<int64_t>(nb) - 1; depth >= 0; --depth)
-            if (boff[depth + 1] != boff[depth]) depths.push_back(depth);
-        bool have_count = false;  // entry count of depths[di] read with the previous depth's sync
-        size_t n0 = 0;
-        for (size_t di = 0; di < depths.size(); ++di) {
-            const int64_t depth = depths[di];
-            if (!have_count) {
+            if (boff[depth + 1] != boff[depth]) depths.push_back(static_cast<uint32_t>(depth));
+        uint32_t* d_depths = buf<uint32_t>(ctx, "ws.depths", depths.size());
+        if (!depths.empty())
+            PMA_CUDA(cudaMemcpyAsync(d_depths, depths.data(), depths.size() * 4, cudaMemcpyHostToDevice, s));
+        WsSmallArgs sa{gvb[0], gpb[0], gvb[1], gpb[1], d_depths, static_cast<uint32_t>(depths.size()), d_boff, max_gen};
+        WsCtl c{0, 0, 0, 0, kWsRun};
+        for (;;) {
+            // small buckets and generations, depth after depth
+            {
+                KernelTimer kt(ctx, "ws_small");
+                *h_ctl = c;
+                PMA_CUDA(cudaMemcpyAsync(d_ctl, h_ctl, sizeof(c), cudaMemcpyHostToDevice, s));
+                ws_small<<<kSmallCluster, kSmallThreads, sizeof(WsSortShared), s>>>(ws, sa, d_ctl);
+                ctx->check_launch("ws_small");
+                ctx->count("ws.small_launches", 1);
                 ReadBack rb;
-                rb.add(h_small, ws.bfill + depth, 4);
-                rb.add(h_small + 4, ws.ext_count, 4);
+                rb.add(h_ctl, d_ctl, sizeof(c));
+                rb.add(h_log_n, ws.log_n, 8);
                 read_back(ctx, rb);
-                grow_records(h_small[4]);
-                n0 = h_small[0];
+                c = *h_ctl;
             }
-            have_count = false;
-            if (n0 == 0) continue;
-            int cur = 0;
-            auto kt_sort = std::make_unique<KernelTimer>(ctx, "ws_depth_sort");
-            if (n0 <= static_cast<size_t>(kSmallBucket)) {
-                ws_sort_small<<<1, 1024, 0, s>>>(ws.ent_time + boff[depth], ws.ent_val + boff[depth],
-                                                 static_cast<unsigned>(n0), gvb[cur], gpb[cur], d_ng + cur);
-                ctx->check_launch("ws_sort_small");
-            } else {
+            if (c.mode == kWsDone || 2 * *h_log_n > ws.log_cap) record_extensions(*h_log_n);
+            if (c.mode == kWsDone) break;
+            PMA_REQUIRE(c.mode != kWsLimit, PMA_ERR_LIMIT, "pma_watershed: generation limit reached");
+            if (c.mode == kWsGrow) continue;
+            const uint32_t dep = depths[c.di];
+            int cur = static_cast<int>(c.cur);
+            if (c.mode == kWsSort) {
+                KernelTimer kt(ctx, "ws_depth_sort");
+                cur = 0;
                 int gen_bits = 0;
-                while (gen_bits < 24 && (1ull << gen_bits) <= gen) ++gen_bits;
-                sort_pairs(ctx, ws.ent_time + boff[depth], srt_time, ws.ent_val + boff[depth], srt_val,
-                           static_cast<int64_t>(n0), std::min(64, ws.time_shift + gen_bits));
-                ws_unpack_entries<<<grid_for(ctx, n0), 256, 0, s>>>(srt_val, n0, gvb[cur], gpb[cur]);
+                while (gen_bits < 24 && (1ull << gen_bits) <= c.gen) ++gen_bits;
+                sort_pairs(ctx, ws.ent_time + boff[dep], srt_time, ws.ent_val + boff[dep], srt_val,
+                           static_cast<int64_t>(c.n), std::min(64, ws.time_shift + gen_bits));
+                ws_unpack_entries<<<grid_for(ctx, c.n), 256, 0, s>>>(srt_val, c.n, g, gvb[cur], gpb[cur]);
                 ctx->check_launch("ws_unpack_entries");
-                h_small[2] = static_cast<unsigned int>(n0);
-                PMA_CUDA(cudaMemcpyAsync(d_ng + cur, &h_small[2], 4, cudaMemcpyHostToDevice, s));
             }
-            kt_sort.reset();
-            const int64_t next_depth = di + 1 < depths.size() ? depths[di + 1] : -1;
+            h_small[2] = c.n;
+            PMA_CUDA(cudaMemcpyAsync(d_ng + cur, &h_small[2], 4, cudaMemcpyHostToDevice, s));
+            // large generations of this depth, until the frontier is small
             KernelTimer kt(ctx, "ws_generations");
-            while (true) {
-                const uint32_t dep = static_cast<uint32_t>(depth);
-                PMA_REQUIRE(gen < max_gen, PMA_ERR_LIMIT, "pma_watershed: generation limit reached");
-                int gens = static_cast<int>(std::min<unsigned long long>(kGensPerLaunch, max_gen - gen));
+            while (c.n > kSmallNodes) {
+                PMA_REQUIRE(c.gen < max_gen, PMA_ERR_LIMIT, "pma_watershed: generation limit reached");
+                int gens = static_cast<int>(std::min<unsigned long long>(kGensPerLaunch, max_gen - c.gen));
+                unsigned small_nodes = kSmallNodes;
                 void* args[] = {&ws, &gvb[0], &gpb[0], &gvb[1], &gpb[1], &d_ng, &desc,
-                                const_cast<uint32_t*>(&dep), &gen, &gens, &cur, &d_out};
+                                const_cast<uint32_t*>(&dep), &c.gen, &gens, &cur, &small_nodes, &d_out};
                 PMA_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ws_generations), coop_grid,
                                                      kChunk / 4, args, 0, s));
                 ctx->count_launch(1);
                 ctx->count("ws.cooperative_launches", 1);
-                {
-                    ReadBack rb;
-                    rb.add(h_out, d_out, 16);
-                    rb.add(h_small + 4, ws.ext_count, 4);
-                    rb.add(h_small + 6, d_ng, 8);
-                    // the next depth's entries are final once this depth is done: read them along
-                    if (next_depth >= 0) rb.add(h_small, ws.bfill + next_depth, 4);
-                    read_back(ctx, rb);
-                }
-                gen += h_out[0];
+                ReadBack rb;
+                rb.add(h_out, d_out, 16);
+                rb.add(h_log_n, ws.log_n, 8);
+                rb.add(h_small + 6, d_ng, 8);
+                read_back(ctx, rb);
+                c.gen += h_out[0];
                 cur = static_cast<int>(h_out[1]);
-                grow_records(h_small[4]);
-                if (h_small[6 + cur] == 0) break;
+                c.n = h_small[6 + cur];
+                if (2 * *h_log_n > ws.log_cap) record_extensions(*h_log_n);
             }
-            if (next_depth >= 0) {
-                n0 = h_small[0];
-                have_count = true;
-            }
+            c.cur = static_cast<uint32_t>(cur);
+            if (c.n == 0) ++c.di;
         }
         PMA_CUDA(cudaMemcpyAsync(&h_err, ws.err, 4, cudaMemcpyDeviceToHost, s));
         ctx->sync();
