@@ -15,8 +15,7 @@
 //    with an edge into p.
 //  * Plateaus are found by a union-find over equal-crad neighbours (from 2^24 voxels:
 //    pointer jumping on the initial trees, then unions of the recorded parent pairs).
-//  * Both recurrences run plateau by plateau in decreasing crad, a few launches per crad
-//    level. The ball order is std::sort's on the host (ordered_sort: libstdc++'s own
+//  * Both recurrences run plateau by plateau in decreasing crad, one launch per crad level. The ball order is std::sort's on the host (ordered_sort: libstdc++'s own
 //    introsort steps on several threads) applied to the same sequence (z, x, y scan order)
 //    with the same comparator, so equal radii tie-break exactly as in the reference.
 //  * A voxel's label is its seed's pore id when |S| = 1 and a shared type ("throat") when
@@ -33,6 +32,7 @@
 #include <memory>
 #include <chrono>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "devutil.cuh"
@@ -500,365 +500,422 @@ __global__ void level_keys(const uint32_t* __restrict__ pcrad, size_t np, uint32
     }
 }
 
-constexpr int kSmallSet = 32;            // sets this small are merged by one warp
-constexpr unsigned kHeavyDegree = 1024;  // plateaus with more in-edges are reduced by a block
-constexpr int kLevelWarps = 4;           // warps per block of the per-plateau kernels
+// --- level sweep ---------------------------------------------------------------------------
+//
+// One step per crad level: S(p) = union of S(q) over the edges q -> p, plus p's own seed. A
+// predecessor lies in an earlier level, and most plateaus take over the set of a predecessor
+// unchanged, so sets are shared: a plateau whose union equals a predecessor's set points at that
+// set, and equal predecessor sets (the same pool position) are read once. What remains is latency
+// (the loads edge -> set -> elements, once per level):
+//  * level_sweep runs one level with a warp per plateau; unions with many elements or
+//    many edges are left to the whole block, which collects them in a hash set in shared memory;
+//  * runs of small levels go through one launch of one block, a block barrier between levels;
+//  * nothing waits for the host: levels are launched one after another, and only a union too large
+//    for a block's hash set stops the sweep (later levels return at once), for the host to merge
+//    that level's such sets by expansion and a radix sort and to go on behind it.
+// (A form with the sets of a level laid out by a scan, a read-back of the level's sizes and a
+// sort for every union beyond 2048 elements took 8 launches and a host round trip a level. The
+// sweep before and after, ms: 620 levels of 2000 plateaus 70 -> 7.1, 421 levels of 15 plateaus
+// 17 -> 1.2, 125 levels of 37000 plateaus 14.9 -> 3.9.)
+constexpr int kSweepWarps = 8;       // warps a block, one level
+constexpr int kRunWarps = 16;        // warps of the block that runs small levels
+constexpr size_t kRunLevel = 64;     // plateaus of a small level at most
+constexpr unsigned kWarpSum = 512;   // elements of a warp's union at most (distinct sets)
+constexpr int kWarpCap = 128;        // distinct elements of a warp's union
+constexpr int kWarpHash = 256;       // slots (power of two, twice kWarpCap)
+constexpr int kBlockBits = 12;       // log2 of the slots of a block's hash set (one less in a run of small
+                                     // levels: more warps share the memory); half of them are used
+constexpr int kSetHash = 512;        // pool positions of the sets a block has seen (power of two)
+constexpr unsigned kSlab = 1024;     // pool elements a warp takes at a time
+constexpr unsigned kSlabMax = 256;   // larger sets take their room directly
+constexpr size_t kSweepList = 1024;  // plateaus of one block at most (its list of large unions)
+constexpr unsigned kHardDegree = 1u << 16;  // edges beyond which a union is spread over the GPU
 
-// Level sweep state. Plateaus of one level are addressed by their local index L (position
-// in `order` minus the level's first position).
 struct PlateauSets {
     const unsigned int* eoff;
-    // Read-only path: the edges, and every array entry of a predecessor (m, slen, soff, its
-    // pool elements), are read through __ldg. A predecessor has a larger radius, so it belongs
-    // to an earlier level and was written by an earlier launch; the loads need not wait for
-    // the launch's own stores to the sweep's 32-bit arrays.
-    const uint32_t* edges;  // sources, sorted by destination
+    const uint32_t* edges;            // sources, sorted by destination
     const uint32_t* order;            // plateaus in decreasing crad
     const uint32_t* minrank;
-    uint32_t* m;       // smallest ball rank reaching the plateau
-    uint32_t* seed;    // rank of the plateau's seed or kNone
-    unsigned long long* soff;
-    uint32_t* slen;
+    ulonglong2* set;                  // per plateau: pool position, length << 32 | smallest ball rank reaching it
+    uint32_t* seed;                   // rank of the plateau's seed or kNone
     uint32_t* pool;
     unsigned long long pool_cap;
+    unsigned long long* pool_n;       // elements taken (may pass pool_cap)
+    ulonglong2* slab;                 // per warp of the sweep: next element, elements left
+    unsigned nslab;
     unsigned int* err;
-    unsigned long long* cnt;     // [L] set size
-    unsigned long long* off;     // [L] exclusive scan of cnt
-    unsigned long long* first;   // [L] first merged element of a large set
-    uint8_t* big;                // [L] 1: merged by the sort path
-    uint32_t* heavy;             // local indices of high in-degree plateaus
-    uint32_t* big_list;          // local indices of the sort-path plateaus
-    unsigned long long* info;    // [0] heavy, [1] big, [2] big elements, [3] expansion fill,
-                                 // [4] fill of the medium unions' buffer
-    uint32_t* mtmp;              // sorted medium unions of the level, until level_write
-    unsigned long long mtmp_cap;
-    unsigned long long* mtoff;   // [L] position of plateau L's medium union in mtmp
+    unsigned long long* info;         // [0] level that stopped the sweep, [1] its hard sets, [2] their
+                                      // elements, [3] keys the expansion wrote
+    uint32_t* hard;                   // plateaus of the hard sets
+    unsigned long long* cnt;          // [hard] distinct elements
+    unsigned long long* first;        // [hard] first merged key
 };
 
-__device__ __forceinline__ uint32_t warp_min_u32(uint32_t v) {
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+// L2: the writer may be another warp of this launch.
+__device__ __forceinline__ ulonglong2 ldcg_set(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
     return v;
 }
 
-__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
+__device__ __forceinline__ uint32_t set_len(ulonglong2 s) { return static_cast<uint32_t>(s.y >> 32); }
 
-// Union of the predecessors' sets and the own seed when it has at most kSmallSet elements
-// (the caller checked the sum of the sizes). On return the warp holds the union sorted
-// ascending: lanes with keep = true hold element `rank`; the return value is its size.
-__device__ __forceinline__ int warp_small_union(const PlateauSets& st, unsigned e0, unsigned e1,
-                                                uint32_t seed, uint32_t* wbuf, unsigned int* wfill,
-                                                unsigned lane, uint32_t& value, bool& keep, int& rank) {
-    if (lane == 0) *wfill = 0;
-    __syncwarp();
-    for (unsigned e = e0 + lane; e < e1; e += 32) {
-        const uint32_t q = __ldg(st.edges + e);
-        const uint32_t len = __ldg(st.slen + q);
-        if (!len) continue;
-        const unsigned pos = atomicAdd(wfill, len);
-        const uint32_t* src = st.pool + __ldg(st.soff + q);
-        for (uint32_t k = 0; k < len; ++k)
-            if (pos + k < kSmallSet) wbuf[pos + k] = __ldg(src + k);
+template <int W>
+struct SweepShared {
+    uint32_t table[W][kWarpHash];
+    uint32_t sorted[W][kWarpCap];
+    unsigned int count[W];
+    // the block's large unions
+    uint32_t list[W == kRunWarps ? kRunLevel : kSweepList];
+    unsigned int nlist;
+    static constexpr int kBits = W == kRunWarps ? kBlockBits - 1 : kBlockBits;
+    static constexpr int kSlots = 1 << kBits, kCap = kSlots / 2;  // distinct elements of a block's union
+    uint32_t btable[kSlots];
+    uint32_t bsorted[kCap];
+    unsigned long long seen[kSetHash];
+    unsigned int bcount, bover;
+    uint32_t wmin[W];
+    unsigned long long wmax[W];
+    unsigned long long wsum[W];
+    unsigned long long place;
+};
+
+// Room for k elements of the pool, by warp (all lanes get it); ~0 when the pool is full.
+__device__ __forceinline__ unsigned long long sweep_room(const PlateauSets& st, ulonglong2& slab, bool has_slab,
+                                                         unsigned k, unsigned lane) {
+    unsigned long long at;
+    if (has_slab && k <= kSlabMax) {
+        if (slab.y < k) {
+            unsigned long long b = 0;
+            if (lane == 0) b = atomicAdd(st.pool_n, static_cast<unsigned long long>(kSlab));
+            slab.x = __shfl_sync(0xFFFFFFFFu, b, 0);
+            slab.y = kSlab;
+        }
+        at = slab.x;
+        slab.x += k;
+        slab.y -= k;
+    } else {
+        at = 0;
+        if (lane == 0) at = atomicAdd(st.pool_n, static_cast<unsigned long long>(k));
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
     }
-    __syncwarp();
-    const unsigned total = min(*wfill, static_cast<unsigned>(kSmallSet));
-    __syncwarp();
-    uint32_t v = lane < total ? wbuf[lane] : kNone;
-    if (seed != kNone && lane == total) v = seed;
-    // bitonic sort of the 32 lanes, ascending (kNone pads sort last)
+    if (at + k <= st.pool_cap) return at;
+    if (lane == 0) atomicOr(st.err, 2u);  // the host redoes the sweep with a larger pool
+    return ~0ull;
+}
+
+__device__ __forceinline__ uint32_t warp_bitonic(uint32_t v, unsigned lane) {  // ascending over the lanes
     for (int k = 2; k <= 32; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
             const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, v, j);
-            const bool ascending = (lane & k) == 0;
-            const bool lower = (lane & j) == 0;
-            v = (lower == ascending) ? min(v, other) : max(v, other);
+            v = (((lane & j) == 0) == ((lane & k) == 0)) ? min(v, other) : max(v, other);
         }
-    const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, v, 1);
-    keep = v != kNone && (lane == 0 || prev != v);
-    const unsigned mask = __ballot_sync(0xFFFFFFFFu, keep);
-    rank = __popc(mask & ((1u << lane) - 1u));
-    value = v;
-    return __popc(mask);
+    return v;
 }
 
-// Medium unions: predecessors whose sizes add up to at most kMedSum elements but repeat the
-// same seeds (a plateau's in-edges mostly come from plateaus reached by the same pores). One
-// warp inserts every element into a hash set of its own in shared memory; when at most kMedCap
-// distinct elements remain, they are sorted in the warp and the union stays on this path
-// instead of the expand-and-sort path of the big sets. One warp streams a union's elements
-// serially, so a long one delays its whole level: at 1024^3 the sweep took 269 ms with unions of
-// up to 8192 elements here, 261 with 4096, 257 with 2048 (the rest going to the parallel sort
-// path).
-constexpr unsigned kMedSum = 2048;
-constexpr int kMedCap = 128;
-constexpr int kMedHash = 256;  // slots (power of two, twice kMedCap)
-constexpr unsigned long long kMedSlab = 1024;  // buffer space a warp takes at a time
+// Element u of the concatenation of the warp's sets (lane l's set starts at excl, elements from
+// position off): its owner lane by a search over the lanes, then the load.
+template <bool RUN>
+__device__ __forceinline__ uint32_t warp_element(const PlateauSets& st, uint32_t u, uint32_t excl, unsigned long long off,
+                                                 uint32_t total) {
+    int owner = 0;
+    for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t e = __shfl_sync(0xFFFFFFFFu, excl, owner + step);
+        if (e <= u) owner += step;
+    }
+    const unsigned long long o = __shfl_sync(0xFFFFFFFFu, off, owner);
+    const uint32_t oe = __shfl_sync(0xFFFFFFFFu, excl, owner);
+    if (u >= total) return kNone;
+    const uint32_t* src = st.pool + o + (u - oe);
+    return RUN ? __ldcg(src) : __ldg(src);
+}
 
-struct MedBuf {
-    uint32_t table[kMedHash];
-    uint32_t sorted[kMedCap];
-    unsigned int count;
-};
+__device__ __forceinline__ uint32_t warp_exclusive(uint32_t v, unsigned lane, uint32_t& total) {
+    uint32_t incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= static_cast<unsigned>(o)) incl += t;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    return incl - v;
+}
 
-// Inserts the predecessors' elements and the seed into the warp's hash set; returns the
-// number of distinct elements, or -1 when there are more than kMedCap.
-__device__ __forceinline__ int warp_medium_insert(const PlateauSets& st, unsigned e0, unsigned e1, uint32_t seed,
-                                                  MedBuf& mb, unsigned lane) {
-    for (int i = lane; i < kMedHash; i += 32) mb.table[i] = kNone;
-    if (lane == 0) mb.count = 0;
-    __syncwarp();
-    bool over = false;
+// One plateau by one warp; false: left to the block.
+template <bool RUN, int W>
+__device__ bool sweep_plateau(const PlateauSets& st, SweepShared<W>& sh, uint32_t p, ulonglong2& slab, bool has_slab) {
+    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned e0 = __ldg(st.eoff + p), e1 = __ldg(st.eoff + p + 1);
+    if (e1 - e0 > 32) return false;
+    ulonglong2 s = make_ulonglong2(~0ull, kNone);  // no set
+    if (e0 + lane < e1) {
+        const uint32_t q = __ldg(st.edges + e0 + lane);
+        s = RUN ? ldcg_set(st.set + q) : __ldg(st.set + q);
+    }
+    const uint32_t own = __ldg(st.minrank + p);
+    uint32_t len = set_len(s);
+    const uint32_t mp = __reduce_min_sync(0xFFFFFFFFu, static_cast<uint32_t>(s.y));
+    const uint32_t seed = own < mp ? own : kNone;
+    // one lane per distinct set
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, len ? s.x : ~0ull);
+    if (len && static_cast<int>(lane) != __ffs(peers) - 1) len = 0;
+    const unsigned have = __ballot_sync(0xFFFFFFFFu, len != 0);
+    const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, len);
+    const int of = __ffs(__ballot_sync(0xFFFFFFFFu, len == longest)) - 1;  // a lane holding a longest set
+    ulonglong2 out;
+    out.x = __shfl_sync(0xFFFFFFFFu, s.x, of);
+    uint32_t k = longest;
+    if (seed != kNone || (have & (have - 1)) != 0) {
+        uint32_t total;
+        const uint32_t excl = warp_exclusive(len, lane, total);
+        if (total > kWarpSum) return false;
+        if (total + (seed != kNone ? 1u : 0u) <= 32) {
+            uint32_t v = warp_element<RUN>(st, lane, excl, s.x, total);
+            if (seed != kNone && lane == total) v = seed;
+            v = warp_bitonic(v, lane);
+            const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, v, 1);
+            const bool keep = v != kNone && (lane == 0 || prev != v);
+            const unsigned mask = __ballot_sync(0xFFFFFFFFu, keep);
+            k = __popc(mask);
+            if (k != longest) {
+                out.x = sweep_room(st, slab, has_slab, k, lane);
+                if (out.x == ~0ull) k = 0;
+                else if (keep) st.pool[out.x + __popc(mask & ((1u << lane) - 1u))] = v;
+            }
+        } else {
+            for (int i = lane; i < kWarpHash; i += 32) sh.table[w][i] = kNone;
+            if (lane == 0) sh.count[w] = 0;
+            __syncwarp();
+            auto insert = [&](uint32_t x) {
+                unsigned h = (x * 2654435761u) >> (32 - 8);  // kWarpHash = 2^8 slots
+                for (int probe = 0; probe < kWarpHash; ++probe, h = (h + 1) & (kWarpHash - 1)) {
+                    const uint32_t prev = atomicCAS(&sh.table[w][h], kNone, x);
+                    if (prev == x) return true;
+                    if (prev == kNone) return atomicAdd(&sh.count[w], 1u) < static_cast<unsigned>(kWarpCap);
+                }
+                return false;
+            };
+            bool fits = true;
+            for (uint32_t u0 = 0; u0 < total; u0 += 32) {
+                const uint32_t x = warp_element<RUN>(st, u0 + lane, excl, s.x, total);
+                if (x != kNone) fits = insert(x);
+                if (!__all_sync(0xFFFFFFFFu, fits)) return false;  // more distinct elements than a warp sorts
+            }
+            if (seed != kNone && lane == 0) fits = insert(seed);
+            if (!__all_sync(0xFFFFFFFFu, fits)) return false;
+            __syncwarp();
+            k = sh.count[w];
+            __syncwarp();
+            if (k != longest || seed != kNone) {  // a new set: sorted, then written
+                if (lane == 0) sh.count[w] = 0;
+                __syncwarp();
+                for (int i = lane; i < kWarpHash; i += 32) {
+                    const uint32_t x = sh.table[w][i];
+                    if (x != kNone) sh.sorted[w][atomicAdd(&sh.count[w], 1u)] = x;
+                }
+                __syncwarp();
+                out.x = sweep_room(st, slab, has_slab, k, lane);
+                const bool room = out.x != ~0ull;
+                if (k <= 32) {
+                    const uint32_t v = warp_bitonic(lane < k ? sh.sorted[w][lane] : kNone, lane);
+                    if (room && lane < k) st.pool[out.x + lane] = v;
+                } else {  // each element's rank among the k
+                    for (uint32_t i = lane; i < k; i += 32) {
+                        const uint32_t x = sh.sorted[w][i];
+                        uint32_t below = 0;
+                        for (uint32_t t = 0; t < k; ++t) below += sh.sorted[w][t] < x ? 1u : 0u;
+                        if (room) st.pool[out.x + below] = x;
+                    }
+                }
+                if (!room) k = 0;
+                __syncwarp();
+            }
+        }
+    }
+    if (lane == 0) {
+        st.seed[p] = seed;
+        out.y = (static_cast<unsigned long long>(k) << 32) | min(own, mp);
+        st.set[p] = out;
+    }
+    return true;
+}
+
+// One plateau by the whole block (uniform arguments).
+template <bool RUN, int W>
+__device__ void sweep_block(const PlateauSets& st, SweepShared<W>& sh, uint32_t p, unsigned long long level) {
+    const unsigned tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned e0 = __ldg(st.eoff + p), e1 = __ldg(st.eoff + p + 1);
+    constexpr int kSlots = SweepShared<W>::kSlots;
+    for (int i = tid; i < kSlots; i += W * 32) sh.btable[i] = kNone;
+    for (int i = tid; i < kSetHash; i += W * 32) sh.seen[i] = ~0ull;
+    if (tid == 0) sh.bcount = sh.bover = 0;
+    __syncthreads();
     auto insert = [&](uint32_t x) {
-        unsigned h = (x * 2654435761u) >> (32 - 8);  // kMedHash = 2^8 slots
-        for (int probe = 0; probe < kMedHash; ++probe, h = (h + 1) & (kMedHash - 1)) {
-            const uint32_t prev = atomicCAS(&mb.table[h], kNone, x);
+        unsigned h = (x * 2654435761u) >> (32 - SweepShared<W>::kBits);
+        for (int probe = 0; probe < kSlots; ++probe, h = (h + 1) & (kSlots - 1)) {
+            uint32_t prev = *reinterpret_cast<volatile uint32_t*>(&sh.btable[h]);
+            if (prev == kNone) prev = atomicCAS(&sh.btable[h], kNone, x);
             if (prev == x) return;
             if (prev == kNone) {
-                if (atomicAdd(&mb.count, 1u) >= static_cast<unsigned>(kMedCap)) over = true;
+                if (atomicAdd(&sh.bcount, 1u) >= static_cast<unsigned>(SweepShared<W>::kCap)) sh.bover = 1;
                 return;
             }
         }
-        over = true;  // table full (only after more than kMedCap insertions)
+        sh.bover = 1;
     };
-    // The warp streams through the predecessors' sets one set at a time, 32 elements a step
-    // (lanes take 32 edges' sizes and offsets at once, then broadcast them): a set of
-    // thousands of elements costs its length / 32 steps, not its length on one lane.
-    bool stop = false;
-    for (unsigned eb = e0; eb < e1 && !stop; eb += 32) {
-        uint32_t len = 0;
-        unsigned long long off = 0;
+    const bool spread = e1 - e0 > kHardDegree;  // too many edges for one block: only its seed is found here
+    uint32_t mp = kNone;
+    unsigned long long longest = 0, sum = 0;  // a longest set: length << 32 | lane's edge; all lengths
+    for (unsigned eb = e0 + w * 32; eb < e1; eb += W * 32) {
+        ulonglong2 s = make_ulonglong2(~0ull, kNone);
         if (eb + lane < e1) {
             const uint32_t q = __ldg(st.edges + eb + lane);
-            len = __ldg(st.slen + q);
-            off = __ldg(st.soff + q);
+            s = RUN ? ldcg_set(st.set + q) : __ldg(st.set + q);
         }
-        const unsigned ne = min(32u, e1 - eb);
-        for (unsigned t = 0; t < ne && !stop; ++t) {
-            const uint32_t tl = __shfl_sync(0xFFFFFFFFu, len, t);
-            const uint32_t* src = st.pool + __shfl_sync(0xFFFFFFFFu, off, t);
-            for (uint32_t b = 0; b < tl; b += 32) {  // warp-uniform steps
-                if (b + lane < tl) insert(__ldg(src + b + lane));
-                // past the cap on any lane: the union takes the sort path
-                if (__any_sync(0xFFFFFFFFu, over)) {
-                    stop = true;
-                    break;
-                }
+        uint32_t len = set_len(s);
+        mp = min(mp, static_cast<uint32_t>(s.y));
+        sum += len;
+        if (spread || *reinterpret_cast<volatile unsigned int*>(&sh.bover)) continue;  // sizes only
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, len ? s.x : ~0ull);
+        if (len && static_cast<int>(lane) != __ffs(peers) - 1) len = 0;
+        if (len) {  // sets the block has seen already
+            unsigned h = static_cast<unsigned>((s.x * 0x9E3779B97F4A7C15ull) >> 55);  // kSetHash = 2^9 slots
+            for (int probe = 0; probe < 4; ++probe, h = (h + 1) & (kSetHash - 1)) {
+                const unsigned long long prev = atomicCAS(&sh.seen[h], ~0ull, s.x);
+                if (prev == s.x) len = 0;
+                if (prev == ~0ull || prev == s.x) break;
             }
+            longest = max(longest, (static_cast<unsigned long long>(len) << 32) | (eb + lane - e0));
+        }
+        uint32_t total;
+        const uint32_t excl = warp_exclusive(len, lane, total);
+        for (uint32_t u0 = 0; u0 < total; u0 += 32) {
+            const uint32_t x = warp_element<RUN>(st, u0 + lane, excl, s.x, total);
+            if (x != kNone) insert(x);
+            if (__any_sync(0xFFFFFFFFu, *reinterpret_cast<volatile unsigned int*>(&sh.bover))) break;
         }
     }
-    if (seed != kNone && lane == 0 && !over) insert(seed);
-    if (__any_sync(0xFFFFFFFFu, over)) return -1;
-    __syncwarp();
-    const unsigned n = mb.count;
-    return n > static_cast<unsigned>(kMedCap) ? -1 : static_cast<int>(n);
-}
-
-// The union gathered by warp_medium_insert (n elements), sorted ascending: up to 32 elements
-// in the lanes' registers, more in mb.sorted. Lane l then holds element l (value, keep = l < n)
-// when n <= 32.
-__device__ __forceinline__ void warp_medium_sort(MedBuf& mb, int n, unsigned lane, uint32_t& value) {
-    if (lane == 0) mb.count = 0;
-    __syncwarp();
-    for (int i = lane; i < kMedHash; i += 32) {
-        const uint32_t x = mb.table[i];
-        if (x != kNone) mb.sorted[atomicAdd(&mb.count, 1u)] = x;
+    mp = __reduce_min_sync(0xFFFFFFFFu, mp);
+    for (int o = 16; o > 0; o >>= 1) {
+        longest = max(longest, __shfl_xor_sync(0xFFFFFFFFu, longest, o));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     }
-    __syncwarp();
-    if (n <= 32) {
-        uint32_t v = static_cast<int>(lane) < n ? mb.sorted[lane] : kNone;
-        for (int k = 2; k <= 32; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, v, j);
-                const bool ascending = (lane & k) == 0;
-                const bool lower = (lane & j) == 0;
-                v = (lower == ascending) ? min(v, other) : max(v, other);
-            }
-        value = v;
+    if (lane == 0) {
+        sh.wmin[w] = mp;
+        sh.wmax[w] = longest;
+        sh.wsum[w] = sum;
+    }
+    __syncthreads();
+    for (int i = 0; i < W; ++i) {
+        mp = min(mp, sh.wmin[i]);
+        longest = max(longest, sh.wmax[i]);
+    }
+    const uint32_t own = __ldg(st.minrank + p);
+    const uint32_t seed = own < mp ? own : kNone;
+    const uint32_t m = min(own, mp);
+    if (tid == 0 && seed != kNone) insert(seed);
+    __syncthreads();
+    if (sh.bover || spread) {  // the host merges it
+        if (tid == 0) {
+            unsigned long long all = seed != kNone ? 1 : 0;
+            for (int i = 0; i < W; ++i) all += sh.wsum[i];
+            st.seed[p] = seed;
+            st.set[p] = make_ulonglong2(0, m);
+            st.hard[atomicAdd(&st.info[1], 1ull)] = p;
+            atomicAdd(&st.info[2], all);
+            atomicMin(&st.info[0], level);
+        }
+        __syncthreads();
         return;
     }
-    int N = 64;
-    while (N < n) N <<= 1;
-    for (int i = n + lane; i < N; i += 32) mb.sorted[i] = kNone;
-    __syncwarp();
-    for (int k = 2; k <= N; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = lane; i < N; i += 32) {
-                const int q = i ^ j;
-                if (q > i) {
-                    const uint32_t a = mb.sorted[i], b = mb.sorted[q];
-                    if (((i & k) == 0) ? (a > b) : (a < b)) {
-                        mb.sorted[i] = b;
-                        mb.sorted[q] = a;
-                    }
-                }
-            }
+    const uint32_t k = sh.bcount;
+    __syncthreads();  // all have read the count
+    if (k == static_cast<uint32_t>(longest >> 32) && seed == kNone) {  // a predecessor's set
+        if (tid == 0) {
+            const uint32_t q = __ldg(st.edges + e0 + static_cast<uint32_t>(longest));
+            const ulonglong2 s = RUN ? ldcg_set(st.set + q) : __ldg(st.set + q);
+            st.seed[p] = seed;
+            st.set[p] = make_ulonglong2(s.x, (static_cast<unsigned long long>(k) << 32) | m);
+        }
+        __syncthreads();
+        return;
+    }
+    if (tid == 0) {
+        sh.bcount = 0;
+        const unsigned long long at = atomicAdd(st.pool_n, static_cast<unsigned long long>(k));
+        const bool fits = at + k <= st.pool_cap;
+        if (!fits) atomicOr(st.err, 2u);
+        sh.place = fits ? at : ~0ull;
+        st.seed[p] = seed;
+        st.set[p] = make_ulonglong2(fits ? at : 0ull, (static_cast<unsigned long long>(fits ? k : 0u) << 32) | m);
+    }
+    __syncthreads();
+    for (int i = tid; i < kSlots; i += W * 32) {
+        const uint32_t x = sh.btable[i];
+        if (x != kNone) sh.bsorted[atomicAdd(&sh.bcount, 1u)] = x;
+    }
+    __syncthreads();
+    const unsigned long long place = sh.place;
+    if (place != ~0ull) {  // each element's rank among the k
+        for (uint32_t i = tid; i < k; i += W * 32) {
+            const uint32_t x = sh.bsorted[i];
+            uint32_t below = 0;
+            for (uint32_t t = 0; t < k; ++t) below += sh.bsorted[t] < x ? 1u : 0u;
+            st.pool[place + below] = x;
+        }
+    }
+    __syncthreads();
+}
+
+// Levels l0 .. l1 - 1 (starts: the position in `order` of each level's first plateau): one level
+// over the grid, or (RUN) several by one block. Returns at once behind a level that stopped.
+template <bool RUN, int W>
+__global__ void __launch_bounds__(W * 32) level_sweep(PlateauSets st, const uint32_t* __restrict__ starts, unsigned l0,
+                                                      unsigned l1) {
+    __shared__ SweepShared<W> sh;
+    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, id = blockIdx.x * W + w;
+    const bool has_slab = id < st.nslab;
+    ulonglong2 slab = has_slab ? st.slab[id] : make_ulonglong2(0, 0);
+    for (unsigned l = l0; l < l1; ++l) {
+        if (__ldcg(st.info) < l) break;  // uniform: written by an earlier launch, or before a block barrier
+        const uint32_t b = __ldg(starts + l), e = __ldg(starts + l + 1);
+        if (threadIdx.x == 0) sh.nlist = 0;
+        __syncthreads();
+        for (uint32_t i = b + id; i < e; i += gridDim.x * W) {
+            const uint32_t p = __ldg(st.order + i);
+            if (!sweep_plateau<RUN, W>(st, sh, p, slab, has_slab) && lane == 0) sh.list[atomicAdd(&sh.nlist, 1u)] = p;
             __syncwarp();
         }
-    value = kNone;
+        __syncthreads();
+        const unsigned n = sh.nlist;
+        for (unsigned k = 0; k < n; ++k) sweep_block<RUN, W>(st, sh, sh.list[k], l);
+        __syncthreads();
+    }
+    if (has_slab && lane == 0) st.slab[id] = slab;
 }
 
-// Seeds, m and set sizes of one level, one warp per plateau. Small and medium unions are
-// merged here and kept, sorted, in mtmp until level_write copies them to the pool; larger ones
-// go to the sort path and plateaus with many in-edges to level_heavy. A union that finds no
-// room in mtmp is merged again by level_write (small) or takes the sort path (medium).
-__global__ void level_seeds(PlateauSets st, size_t begin, size_t end, unsigned slab) {
-    __shared__ uint32_t wbuf[kLevelWarps][kSmallSet];
-    __shared__ unsigned int wfill[kLevelWarps];
-    __shared__ MedBuf med[kLevelWarps];
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // The warp takes mtmp space in slabs (one atomic per slab, not one per union on a counter
-    // every warp of the level shares); returns the start of k elements, or ~0 when full.
-    unsigned long long slab_base = 0, slab_left = 0;
-    auto take = [&](unsigned long long k) -> unsigned long long {
-        if (k > slab_left) {
-            unsigned long long b = 0;
-            if (lane == 0) b = atomicAdd(&st.info[4], static_cast<unsigned long long>(slab));
-            slab_base = __shfl_sync(0xFFFFFFFFu, b, 0);
-            slab_left = slab_base + slab <= st.mtmp_cap ? slab : 0;
-        }
-        if (k > slab_left) return ~0ull;
-        const unsigned long long at = slab_base;
-        slab_base += k;
-        slab_left -= k;
-        return at;
-    };
-    const size_t stride = static_cast<size_t>(gridDim.x) * kLevelWarps;
-    for (size_t i = begin + static_cast<size_t>(blockIdx.x) * kLevelWarps + w; i < end; i += stride) {
-        const size_t L = i - begin;
-        const uint32_t p = st.order[i];
-        const unsigned e0 = st.eoff[p], e1 = st.eoff[p + 1];
-        if (e1 - e0 > kHeavyDegree) {
-            if (lane == 0) {
-                st.big[L] = 1;
-                st.cnt[L] = 0;
-                st.heavy[atomicAdd(&st.info[0], 1ull)] = static_cast<uint32_t>(L);
-            }
-            continue;
-        }
-        uint32_t mp = kNone;
-        unsigned long long u = 0;
-        for (unsigned e = e0 + lane; e < e1; e += 32) {
-            const uint32_t q = __ldg(st.edges + e);
-            mp = min(mp, __ldg(st.m + q));
-            u += __ldg(st.slen + q);
-        }
-        mp = warp_min_u32(mp);
-        u = warp_sum_u64(u);
-        const uint32_t own = st.minrank[p];
-        const uint32_t seed = own < mp ? own : kNone;
-        if (lane == 0) {
-            st.m[p] = min(own, mp);
-            st.seed[p] = seed;
-        }
-        const unsigned long long total = u + (seed != kNone ? 1u : 0u);
-        if (total <= kSmallSet) {
-            uint32_t v;
-            bool keep;
-            int rank;
-            const int k = warp_small_union(st, e0, e1, seed, wbuf[w], &wfill[w], lane, v, keep, rank);
-            const unsigned long long at = k > 0 ? take(static_cast<unsigned long long>(k)) : 0ull;
-            if (at != ~0ull) {
-                if (keep) st.mtmp[at + rank] = v;
-                if (lane == 0) st.mtoff[L] = at;
-            }
-            if (lane == 0) {
-                st.big[L] = at != ~0ull ? 2 : 0;
-                st.cnt[L] = static_cast<unsigned long long>(k);
-            }
-        } else {
-            int k = total <= kMedSum ? warp_medium_insert(st, e0, e1, seed, med[w], lane) : -1;
-            if (k >= 0) {  // a medium union: sorted now, kept in mtmp until level_write
-                uint32_t v;
-                warp_medium_sort(med[w], k, lane, v);
-                const unsigned long long at = take(static_cast<unsigned long long>(k));
-                if (at != ~0ull) {
-                    if (k <= 32) {
-                        if (static_cast<int>(lane) < k) st.mtmp[at + lane] = v;
-                    } else {
-                        for (int r = lane; r < k; r += 32) st.mtmp[at + r] = med[w].sorted[r];
-                    }
-                    if (lane == 0) st.mtoff[L] = at;
-                } else {
-                    k = -1;  // no room left: the sort path takes it
-                }
-            }
-            if (lane == 0) {
-                if (k >= 0) {
-                    st.big[L] = 2;
-                    st.cnt[L] = static_cast<unsigned long long>(k);
-                } else {
-                    st.big[L] = 1;
-                    st.cnt[L] = 0;
-                    st.big_list[atomicAdd(&st.info[1], 1ull)] = static_cast<uint32_t>(L);
-                    atomicAdd(&st.info[2], total);
-                }
-            }
-        }
+__global__ void unpack_sets(const ulonglong2* __restrict__ set, size_t np, unsigned long long* __restrict__ soff,
+                            uint32_t* __restrict__ slen) {
+    PMA_GRID_STRIDE(p, np) {
+        const ulonglong2 s = set[p];
+        soff[p] = s.x;
+        slen[p] = set_len(s);
     }
 }
 
-// Seeds and m of the high in-degree plateaus, one block each; they all take the sort path.
-__global__ void level_heavy(PlateauSets st, size_t begin) {
-    __shared__ uint32_t smin[32];
-    __shared__ unsigned long long ssum[32];
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const unsigned long long nh = st.info[0];
-    for (unsigned long long h = blockIdx.x; h < nh; h += gridDim.x) {
-        const uint32_t L = st.heavy[h];
-        const uint32_t p = st.order[begin + L];
-        const unsigned e0 = st.eoff[p], e1 = st.eoff[p + 1];
-        uint32_t mp = kNone;
-        unsigned long long u = 0;
-        for (unsigned e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-            const uint32_t q = __ldg(st.edges + e);
-            mp = min(mp, __ldg(st.m + q));
-            u += __ldg(st.slen + q);
-        }
-        mp = warp_min_u32(mp);
-        u = warp_sum_u64(u);
-        if (lane == 0) {
-            smin[w] = mp;
-            ssum[w] = u;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (unsigned k = 1; k < nw; ++k) {
-                mp = min(mp, smin[k]);
-                u += ssum[k];
-            }
-            const uint32_t own = st.minrank[p];
-            const uint32_t seed = own < mp ? own : kNone;
-            st.m[p] = min(own, mp);
-            st.seed[p] = seed;
-            st.big_list[atomicAdd(&st.info[1], 1ull)] = L;
-            atomicAdd(&st.info[2], u + (seed != kNone ? 1u : 0u));
-        }
-        __syncthreads();
-    }
-}
-
-// Sort path: every element of every predecessor set (and the own seed) of the big plateaus
-// becomes a key (plateau << shift | rank); sorting and removing duplicates yields each union.
-// The plateau of a key is its index in the level's big list, above the rank bits (32 bits
-// in the single-block merge); keys are 32-bit whenever ranks and big-list indices fit together,
-// else 64-bit, and the radix sort covers the used bits only.
-template <class K>
-__device__ __forceinline__ uint32_t key_plateau(const PlateauSets& st, K key, int shift) {
-    return st.big_list[static_cast<uint32_t>(key >> shift)];
-}
-
-// In-degrees of the big plateaus (their edges are spread over the whole grid below).
-__global__ void level_big_degrees(PlateauSets st, size_t begin, unsigned long long* __restrict__ deg) {
-    const unsigned long long nbig = st.info[1];
-    PMA_GRID_STRIDE(b, nbig) {
-        const uint32_t p = st.order[begin + st.big_list[b]];
+// --- hard sets: unions too large for a block ---
+//
+// Every element of every predecessor set (and the own seed) becomes a key (hard set << shift |
+// rank); sorting and removing duplicates yields each union. Keys are 32-bit whenever ranks and
+// set indices fit together, else 64-bit, and the radix sort covers the used bits only.
+__global__ void level_hard_degrees(PlateauSets st, unsigned long long* __restrict__ deg) {
+    const unsigned long long nh = st.info[1];
+    PMA_GRID_STRIDE(b, nh) {
+        const uint32_t p = st.hard[b];
         deg[b] = st.eoff[p + 1] - st.eoff[p];
     }
 }
 
-// One thread per in-edge of a big plateau (t over the concatenated edge lists, doff = the
+// One thread per in-edge of a hard plateau (t over the concatenated edge lists, doff = the
 // exclusive scan of the in-degrees): a giant plateau with a million in-edges is spread over
 // the whole GPU instead of one block. The in-edges of a block mostly belong to one plateau and
 // bring the same seeds many times, so each block keeps only the first copy of a key (shared-
@@ -867,14 +924,14 @@ __global__ void level_big_degrees(PlateauSets st, size_t begin, unsigned long lo
 constexpr int kMergeTable = 2048;
 
 template <class K>
-__global__ void __launch_bounds__(256) level_expand(PlateauSets st, size_t begin,
+__global__ void __launch_bounds__(256) level_expand(PlateauSets st,
                                                     const unsigned long long* __restrict__ doff,
                                                     const unsigned long long* __restrict__ deg,
-                                                    unsigned long long nbig, K* __restrict__ keys,
+                                                    unsigned long long nhard, K* __restrict__ keys,
                                                     unsigned long long cap, int shift) {
     __shared__ K table[kMergeTable];
     const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
-    const unsigned long long total = doff[nbig - 1] + deg[nbig - 1];
+    const unsigned long long total = doff[nhard - 1] + deg[nhard - 1];
     const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
     const K empty = ~static_cast<K>(0);
     // block-uniform trip count (the table is cleared between rounds)
@@ -887,17 +944,16 @@ __global__ void __launch_bounds__(256) level_expand(PlateauSets st, size_t begin
         const uint32_t* src = st.pool;
         K hi = 0;
         if (t < total) {
-            unsigned long long lo = 0, up = nbig;  // last b with doff[b] <= t
+            unsigned long long lo = 0, up = nhard;  // last b with doff[b] <= t
             while (up - lo > 1) {
                 const unsigned long long mid = (lo + up) >> 1;
                 if (doff[mid] <= t) lo = mid;
                 else up = mid;
             }
-            const uint32_t L = st.big_list[lo];
-            const uint32_t p = st.order[begin + L];
-            const uint32_t q = __ldg(st.edges + st.eoff[p] + (t - doff[lo]));
-            len = __ldg(st.slen + q);
-            src = st.pool + __ldg(st.soff + q);
+            const uint32_t p = st.hard[lo];
+            const ulonglong2 set = __ldg(st.set + __ldg(st.edges + st.eoff[p] + (t - doff[lo])));
+            len = set_len(set);
+            src = st.pool + set.x;
             hi = static_cast<K>(lo) << shift;
         }
         // The warp's 32 sets are expanded together, 32 elements per round: element u of the
@@ -948,10 +1004,9 @@ __global__ void __launch_bounds__(256) level_expand(PlateauSets st, size_t begin
         __syncthreads();
     }
     // own seeds
-    for (unsigned long long b = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; b < nbig;
+    for (unsigned long long b = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; b < nhard;
          b += stride) {
-        const uint32_t L = st.big_list[b];
-        const uint32_t p = st.order[begin + L];
+        const uint32_t p = st.hard[b];
         if (st.seed[p] == kNone) continue;
         const unsigned long long pos = atomicAdd(&st.info[3], 1ull);
         if (pos < cap) keys[pos] = (static_cast<K>(b) << shift) | static_cast<K>(st.seed[p]);
@@ -962,173 +1017,37 @@ __global__ void __launch_bounds__(256) level_expand(PlateauSets st, size_t begin
 template <class K>
 __global__ void level_runs(const K* __restrict__ keys, size_t n, PlateauSets st, int shift) {
     PMA_GRID_STRIDE(i, n) {
-        const K hi = keys[i] >> shift;
-        const uint32_t L = key_plateau(st, keys[i], shift);
-        if (i == 0 || (keys[i - 1] >> shift) != hi) st.first[L] = i;
-        atomicAdd(&st.cnt[L], 1ull);
+        const size_t b = static_cast<size_t>(keys[i] >> shift);
+        if (i == 0 || static_cast<size_t>(keys[i - 1] >> shift) != b) st.first[b] = i;
+        atomicAdd(&st.cnt[b], 1ull);
     }
 }
 
-// Sort path of a level whose big unions hold few keys in all (kSmallMerge): one block expands,
-// sorts (bitonic, shared memory) and de-duplicates them, and fills cnt/first like level_runs.
-// No host round trip: the number of merged keys stays on the device (*merged).
-constexpr int kSmallMerge = 4096;
-
-__global__ void __launch_bounds__(1024) level_merge_small(PlateauSets st, size_t begin,
-                                                          unsigned long long* __restrict__ keys,
-                                                          unsigned long long* __restrict__ merged) {
-    __shared__ unsigned long long sk[kSmallMerge];
-    __shared__ unsigned int s_count;
-    __shared__ unsigned int wsum[32];
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const unsigned long long nbig = st.info[1];
-    if (threadIdx.x == 0) s_count = 0;
-    __syncthreads();
-    for (unsigned long long b = warp; b < nbig; b += nw) {
-        const uint32_t L = st.big_list[b];
-        const uint32_t p = st.order[begin + L];
-        const unsigned e0 = st.eoff[p], e1 = st.eoff[p + 1];
-        const unsigned long long hi = static_cast<unsigned long long>(b) << 32;
-        // lanes take 32 edges' sets at once and reserve their room; the warp then copies the
-        // sets one after another, 32 elements a step
-        for (unsigned eb = e0; eb < e1; eb += 32) {
-            uint32_t len = 0;
-            unsigned long long off = 0;
-            unsigned pos = 0;
-            if (eb + lane < e1) {
-                const uint32_t q = __ldg(st.edges + eb + lane);
-                len = __ldg(st.slen + q);
-                off = __ldg(st.soff + q);
-                pos = atomicAdd(&s_count, len);
-            }
-            const unsigned ne = min(32u, e1 - eb);
-            for (unsigned t = 0; t < ne; ++t) {
-                const uint32_t tl = __shfl_sync(0xFFFFFFFFu, len, t);
-                const unsigned tp = __shfl_sync(0xFFFFFFFFu, pos, t);
-                const uint32_t* src = st.pool + __shfl_sync(0xFFFFFFFFu, off, t);
-                for (uint32_t r = lane; r < tl; r += 32)
-                    if (tp + r < kSmallMerge) sk[tp + r] = hi | __ldg(src + r);
-            }
-        }
-        if (lane == 0 && st.seed[p] != kNone) {
-            const unsigned pos = atomicAdd(&s_count, 1u);
-            if (pos < kSmallMerge) sk[pos] = hi | st.seed[p];
-        }
-    }
-    __syncthreads();
-    const unsigned n = min(s_count, static_cast<unsigned>(kSmallMerge));
-    unsigned N = 1;
-    while (N < n) N <<= 1;
-    for (unsigned i = n + threadIdx.x; i < N; i += blockDim.x) sk[i] = ~0ull;
-    __syncthreads();
-    for (unsigned k = 2; k <= N; k <<= 1)  // bitonic sort, ascending
-        for (unsigned j = k >> 1; j > 0; j >>= 1) {
-            for (unsigned i = threadIdx.x; i < N; i += blockDim.x) {
-                const unsigned q = i ^ j;
-                if (q > i) {
-                    const unsigned long long a = sk[i], c = sk[q];
-                    if (((i & k) == 0) ? (a > c) : (a < c)) {
-                        sk[i] = c;
-                        sk[q] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    // first copies, compacted in order: each thread owns a contiguous run of 4 positions
-    const unsigned per = (N + blockDim.x - 1) / blockDim.x;  // <= 4
-    const unsigned i0 = threadIdx.x * per;
-    unsigned mine = 0;
-    for (unsigned t = 0; t < per; ++t) {
-        const unsigned i = i0 + t;
-        if (i < n && (i == 0 || sk[i - 1] != sk[i])) ++mine;
-    }
-    unsigned incl = mine;
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= static_cast<unsigned>(o)) incl += v;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned run = 0;
-        for (unsigned w = 0; w < nw; ++w) {
-            const unsigned v = wsum[w];
-            wsum[w] = run;
-            run += v;
-        }
-        *merged = run;
-    }
-    __syncthreads();
-    unsigned u = wsum[warp] + incl - mine;
-    for (unsigned t = 0; t < per; ++t) {
-        const unsigned i = i0 + t;
-        if (!(i < n && (i == 0 || sk[i - 1] != sk[i]))) continue;
-        const uint32_t bhi = static_cast<uint32_t>(sk[i] >> 32);  // index in the big list
-        const uint32_t L = st.big_list[bhi];
-        keys[u] = sk[i];
-        // sk[i] is a first copy, so sk[i - 1] is the previous distinct key
-        if (i == 0 || static_cast<uint32_t>(sk[i - 1] >> 32) != bhi) st.first[L] = u;
-        atomicAdd(&st.cnt[L], 1ull);
-        ++u;
-    }
-}
-
-// Writes the small unions (recomputed) and the list offsets of all plateaus of the level.
-__global__ void level_write(PlateauSets st, size_t begin, size_t end, const unsigned long long* __restrict__ base) {
-    __shared__ uint32_t wbuf[kLevelWarps][kSmallSet];
-    __shared__ unsigned int wfill[kLevelWarps];
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const size_t stride = static_cast<size_t>(gridDim.x) * kLevelWarps;
-    const unsigned long long b0 = *base;
-    for (size_t i = begin + static_cast<size_t>(blockIdx.x) * kLevelWarps + w; i < end; i += stride) {
-        const size_t L = i - begin;
-        const uint32_t p = st.order[i];
-        const unsigned long long pos = b0 + st.off[L], k = st.cnt[L];
-        // A list that does not fit is recorded empty so later levels never read past the
-        // pool; the overflow flag makes the host redo the sweep with a larger pool.
-        const bool fits = pos + k <= st.pool_cap;
-        if (lane == 0) {
-            st.soff[p] = fits ? pos : 0;
-            st.slen[p] = fits ? static_cast<uint32_t>(k) : 0u;
-            if (!fits) atomicOr(st.err, 2u);
-        }
-        if (st.big[L] == 1) continue;
-        if (st.big[L] == 2) {  // sorted by level_seeds
-            const uint32_t* src = st.mtmp + st.mtoff[L];
-            for (unsigned long long r = lane; r < k; r += 32)
-                if (fits) st.pool[pos + r] = src[r];
-            continue;
-        }
-        uint32_t v;
-        bool keep;
-        int rank;
-        warp_small_union(st, st.eoff[p], st.eoff[p + 1], st.seed[p], wbuf[w], &wfill[w], lane, v, keep, rank);
-        if (keep && fits) st.pool[pos + rank] = v;
+__global__ void level_place_hard(PlateauSets st, size_t nhard) {
+    PMA_GRID_STRIDE(b, nhard) {
+        const uint32_t p = st.hard[b];
+        const unsigned long long k = st.cnt[b], at = atomicAdd(st.pool_n, k);
+        const bool fits = at + k <= st.pool_cap;
+        if (!fits) atomicOr(st.err, 2u);
+        const unsigned long long m = st.set[p].y & 0xFFFFFFFFull;
+        st.set[p] = make_ulonglong2(fits ? at : 0ull, ((fits ? k : 0ull) << 32) | m);
     }
 }
 
 template <class K>
-__global__ void level_copy_big(const K* __restrict__ keys, size_t n_host, PlateauSets st,
-                               const unsigned long long* __restrict__ base, int shift,
-                               const unsigned long long* __restrict__ n_dev) {
-    const unsigned long long b0 = *base;
+__global__ void level_copy_hard(const K* __restrict__ keys, size_t n, PlateauSets st, int shift) {
     const K low = (static_cast<K>(1) << shift) - 1;
-    const size_t n = n_dev ? static_cast<size_t>(*n_dev) : n_host;
     PMA_GRID_STRIDE(i, n) {
-        const uint32_t L = key_plateau(st, keys[i], shift);
-        const unsigned long long pos = b0 + st.off[L], r = i - st.first[L];  // rank within the set
-        if (r >= st.cnt[L]) {  // keys and set bounds disagree: never write outside the set
+        const size_t b = static_cast<size_t>(keys[i] >> shift);
+        const ulonglong2 s = st.set[st.hard[b]];
+        const unsigned long long r = i - st.first[b];  // rank within the set
+        if (set_len(s) == 0) continue;  // no room in the pool: the sweep is redone
+        if (r >= set_len(s)) {  // keys and set bounds disagree: never write outside the set
             atomicOr(st.err, 32u);
             continue;
         }
-        if (pos + st.cnt[L] <= st.pool_cap) st.pool[pos + r] = static_cast<uint32_t>(keys[i] & low);
+        st.pool[s.x + r] = static_cast<uint32_t>(keys[i] & low);
     }
-}
-
-__global__ void level_advance(unsigned long long* __restrict__ base, const unsigned long long* __restrict__ off,
-                              const unsigned long long* __restrict__ cnt, size_t nlev) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *base += off[nlev - 1] + cnt[nlev - 1];
 }
 
 __global__ void throat_hashes(const unsigned long long* __restrict__ soff, const uint32_t* __restrict__ slen,
@@ -1517,177 +1436,125 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     level_begin.push_back(static_cast<size_t>(np));
 
     // Level sweep.
-    size_t max_level = 1;
-    for (size_t l = 0; l + 1 < level_begin.size(); ++l)
-        max_level = std::max(max_level, level_begin[l + 1] - level_begin[l]);
+    const size_t nlevels = level_begin.size() - 1;
     PlateauSets ps;
     ps.eoff = eoff;
     ps.edges = by_dst;
     ps.order = order;
     ps.minrank = pminrank;
-    ps.m = buf<uint32_t>(ctx, "pores.m", np);
+    ps.set = buf<ulonglong2>(ctx, "pores.set", np);
     ps.seed = buf<uint32_t>(ctx, "pores.seed", np);
-    ps.soff = buf<unsigned long long>(ctx, "pores.soff", np);
-    ps.slen = buf<uint32_t>(ctx, "pores.slen", np);
     ps.err = err;
-    ps.cnt = buf<unsigned long long>(ctx, "pores.cnt", max_level);
-    ps.off = buf<unsigned long long>(ctx, "pores.off", max_level);
-    ps.first = buf<unsigned long long>(ctx, "pores.first", max_level);
-    ps.big = buf<uint8_t>(ctx, "pores.big", max_level);
-    ps.heavy = buf<uint32_t>(ctx, "pores.heavy", max_level);
-    ps.big_list = buf<uint32_t>(ctx, "pores.big_list", max_level);
     ps.info = buf<unsigned long long>(ctx, "pores.info", 5);
-    ps.mtoff = buf<unsigned long long>(ctx, "pores.mtoff", max_level);
-    // medium unions of one level: a buffer of its own (a full buffer sends the rest to the sort path)
-    ps.mtmp_cap = std::min<unsigned long long>(std::max<unsigned long long>(1ull << 22, 16ull * np), 1ull << 27);
-    ps.mtmp = buf<uint32_t>(ctx, "pores.mtmp", ps.mtmp_cap);
-    unsigned long long* base = reinterpret_cast<unsigned long long*>(d_count + 3);
-    auto* h_info = static_cast<unsigned long long*>(ctx->host_staging(32));
-    unsigned long long pool_cap = std::max<unsigned long long>(1ull << 22, 32ull * np);
+    ps.pool_n = ps.info + 4;
+    ps.hard = buf<uint32_t>(ctx, "pores.hard", np);
+    ps.nslab = static_cast<unsigned>(ctx->num_sms * 8 * kSweepWarps);
+    ps.slab = buf<ulonglong2>(ctx, "pores.slab", ps.nslab);
+    // first position of each level (lval holds the level starts found above), and the end
+    uint32_t* d_starts = buf<uint32_t>(ctx, "pores.level_starts", nlevels + 1);
+    std::vector<uint32_t> h_starts(level_begin.begin(), level_begin.end());
+    PMA_CUDA(cudaMemcpyAsync(d_starts, h_starts.data(), h_starts.size() * 4, cudaMemcpyHostToDevice, s));
+    auto* h_info = static_cast<unsigned long long*>(ctx->host_staging(64));
+    unsigned long long pool_cap = std::max<unsigned long long>(1ull << 22, 16ull * np);
     int rank_bits = 1;  // bits of a ball rank
     while (rank_bits < 32 && (1ull << rank_bits) < static_cast<unsigned long long>(nb)) ++rank_bits;
-    const unsigned heavy_grid = static_cast<unsigned>(ctx->num_sms * 2);
+    // Merges the hard sets of the level that stopped the sweep (h_info: their number and elements).
+    auto merge_hard = [&](unsigned long long nhard, unsigned long long total) {
+        KernelTimer kt2(ctx, "level_merge");
+        ctx->count("pores.hard_sets", static_cast<double>(nhard));
+        ctx->count("pores.hard_set_elements_expanded", static_cast<double>(total));
+        PMA_REQUIRE(total < (1ull << 40), PMA_ERR_MEMORY, "pma_pores: seed-set union too large");
+        int hard_bits = 0;
+        while ((1ull << hard_bits) < nhard) ++hard_bits;
+        auto* deg = buf<unsigned long long>(ctx, "pores.bdeg", nhard);
+        auto* doff = buf<unsigned long long>(ctx, "pores.bdoff", nhard);
+        ps.cnt = buf<unsigned long long>(ctx, "pores.cnt", nhard);
+        ps.first = buf<unsigned long long>(ctx, "pores.first", nhard);
+        PMA_CUDA(cudaMemsetAsync(ps.cnt, 0, nhard * 8, s));
+        level_hard_degrees<<<grid_for(ctx, nhard), 256, 0, s>>>(ps, deg);
+        ctx->check_launch("level_hard_degrees");
+        exclusive_sum(ctx, deg, doff, static_cast<int64_t>(nhard));
+        auto merge = [&](auto* k0, auto* k1) {
+            using K = std::remove_pointer_t<decltype(k0)>;
+            level_expand<K><<<static_cast<unsigned>(ctx->num_sms * 16), 256, 0, s>>>(ps, doff, deg, nhard, k0, total,
+                                                                                    rank_bits);
+            ctx->check_launch("level_expand");
+            ReadBack rb;
+            rb.add(h_info, ps.info, 32);
+            read_back(ctx, rb);
+            const int64_t emitted = static_cast<int64_t>(std::min<unsigned long long>(h_info[3], total));
+            sort_keys(ctx, k0, k1, emitted, rank_bits + hard_bits);  // radix passes over the used bits only
+            const int64_t merged = unique(ctx, k1, k0, emitted, d_count);
+            if (!merged) return;
+            level_runs<K><<<grid_for(ctx, merged), 256, 0, s>>>(k0, merged, ps, rank_bits);
+            ctx->check_launch("level_runs");
+            level_place_hard<<<grid_for(ctx, nhard), 256, 0, s>>>(ps, nhard);
+            ctx->check_launch("level_place_hard");
+            level_copy_hard<K><<<grid_for(ctx, merged), 256, 0, s>>>(k0, merged, ps, rank_bits);
+            ctx->check_launch("level_copy_hard");
+        };
+        if (rank_bits < 32 && rank_bits + hard_bits <= 32)
+            merge(buf<uint32_t>(ctx, "pores.lkeys32", total), buf<uint32_t>(ctx, "pores.lkeys32b", total));
+        else
+            merge(buf<unsigned long long>(ctx, "pores.lkeys", total), buf<unsigned long long>(ctx, "pores.lkeys2", total));
+    };
+    constexpr unsigned long long kNoStop = ~0ull;
+    constexpr unsigned kWindow = 64;  // launches between looks at the stop
     for (int attempt = 0; attempt < 3; ++attempt) {
         ps.pool = buf<uint32_t>(ctx, "pores.pool", pool_cap);
         ps.pool_cap = pool_cap;
-        PMA_CUDA(cudaMemsetAsync(base, 0, 8, s));
+        PMA_CUDA(cudaMemsetAsync(ps.info, 0, 40, s));
+        PMA_CUDA(cudaMemsetAsync(ps.info, 0xFF, 8, s));  // no stop
         PMA_CUDA(cudaMemsetAsync(err, 0, 4, s));
+        PMA_CUDA(cudaMemsetAsync(ps.slab, 0, ps.nslab * sizeof(ulonglong2), s));
         KernelTimer kt(ctx, "level_sets");
-        // per size class of the levels (plateaus in the level, log2), when timing is on
-        static const char* const kLevelClass[32] = {"levels.plateaus_2^0", "levels.plateaus_2^1", "levels.plateaus_2^2", "levels.plateaus_2^3", "levels.plateaus_2^4", "levels.plateaus_2^5", "levels.plateaus_2^6", "levels.plateaus_2^7", "levels.plateaus_2^8", "levels.plateaus_2^9", "levels.plateaus_2^10", "levels.plateaus_2^11", "levels.plateaus_2^12", "levels.plateaus_2^13", "levels.plateaus_2^14", "levels.plateaus_2^15", "levels.plateaus_2^16", "levels.plateaus_2^17", "levels.plateaus_2^18", "levels.plateaus_2^19", "levels.plateaus_2^20", "levels.plateaus_2^21", "levels.plateaus_2^22", "levels.plateaus_2^23", "levels.plateaus_2^24", "levels.plateaus_2^25", "levels.plateaus_2^26", "levels.plateaus_2^27", "levels.plateaus_2^28", "levels.plateaus_2^29", "levels.plateaus_2^30", "levels.plateaus_2^31"};
-        for (size_t l = 0; l + 1 < level_begin.size(); ++l) {
-            const size_t b = level_begin[l], e = level_begin[l + 1];
-            int lclass = 0;
-            while (lclass < 31 && (2ull << lclass) <= e - b) ++lclass;
-            KernelTimer kt_level(ctx, kLevelClass[lclass]);
-            if (ctx->timing) ctx->count(std::string(kLevelClass[lclass]) + ".count", 1);
-            const unsigned lg = grid_for(ctx, (e - b) * 32, kLevelWarps * 32);
-            PMA_CUDA(cudaMemsetAsync(ps.info, 0, 40, s));
-            {
-                KernelTimer kt2(ctx, "level_seeds");
-                // slabs small enough for every warp of the launch to get some of mtmp, and
-                // at least a medium union's largest size
-                const unsigned slab = static_cast<unsigned>(std::min<unsigned long long>(
-                    kMedSlab, std::max<unsigned long long>(kMedCap, ps.mtmp_cap / (1ull * lg * kLevelWarps))));
-                level_seeds<<<lg, kLevelWarps * 32, 0, s>>>(ps, b, e, slab);
-                level_heavy<<<heavy_grid, 512, 0, s>>>(ps, b);
-                ctx->count_launch(2);
-            }
-            {
-                ReadBack rb;
-                rb.add(h_info, ps.info, 32);
-                read_back(ctx, rb);
-            }
-            const unsigned long long nbig = h_info[1], total = h_info[2];
-            ctx->count("pores.levels", 1);
-            if (nbig) {
-                ctx->count("pores.big_sets", static_cast<double>(nbig));
-                ctx->count("pores.big_set_elements_expanded", static_cast<double>(total));
-            }
-            if (h_info[0]) ctx->count("pores.heavy_plateaus", static_cast<double>(h_info[0]));
-            int64_t merged = 0;
-            int shift = 32;
-            void* keys = nullptr;
-            bool narrow = false;
-            const unsigned long long* merged_dev = nullptr;  // merged count left on the device
-            if (nbig && total <= static_cast<unsigned long long>(kSmallMerge)) {
-                KernelTimer kt2(ctx, "level_merge");
-                auto* k64 = buf<unsigned long long>(ctx, "pores.lkeys", kSmallMerge);
-                merged_dev = ps.info + 3;
-                level_merge_small<<<1, 1024, 0, s>>>(ps, b, k64, ps.info + 3);
-                ctx->check_launch("level_merge_small");
-                keys = k64;
-                merged = kSmallMerge;  // upper bound for the copy launch below
-            } else if (nbig) {
-                KernelTimer kt2(ctx, "level_merge");
-                PMA_REQUIRE(total < (1ull << 40), PMA_ERR_MEMORY, "pma_pores: seed-set union too large");
-                int big_bits = 0;
-                while ((1ull << big_bits) < nbig) ++big_bits;
-                narrow = rank_bits < 32 && rank_bits + big_bits <= 32;
-                auto read_emitted = [&]() {
-                    ReadBack rb;
-                    rb.add(h_info, ps.info, 32);
-                    read_back(ctx, rb);
-                    return static_cast<int64_t>(std::min<unsigned long long>(h_info[3], total));
-                };
-                auto* deg = buf<unsigned long long>(ctx, "pores.bdeg", nbig);
-                auto* doff = buf<unsigned long long>(ctx, "pores.bdoff", nbig);
-                level_big_degrees<<<grid_for(ctx, nbig), 256, 0, s>>>(ps, b, deg);
-                ctx->check_launch("level_big_degrees");
-                exclusive_sum(ctx, deg, doff, static_cast<int64_t>(nbig));
-                const unsigned eg = static_cast<unsigned>(ctx->num_sms * 16);
-                if (narrow) {
-                    shift = rank_bits;
-                    auto* k32 = buf<uint32_t>(ctx, "pores.lkeys32", total);
-                    auto* k32b = buf<uint32_t>(ctx, "pores.lkeys32b", total);
-                    int64_t emitted = 0;
-                    {
-                        KernelTimer kt3(ctx, "merge_expand");
-                        level_expand<uint32_t><<<eg, 256, 0, s>>>(ps, b, doff, deg, nbig, k32, total, shift);
-                        ctx->check_launch("level_expand");
-                        emitted = read_emitted();
-                    }
-                    {
-                        KernelTimer kt3(ctx, "merge_sort");
-                        sort_keys(ctx, k32, k32b, emitted, rank_bits + big_bits);
-                        merged = unique(ctx, k32b, k32, emitted, d_count);
-                    }
-                    keys = k32;
-                    if (merged) {
-                        level_runs<uint32_t><<<grid_for(ctx, merged), 256, 0, s>>>(k32, merged, ps, shift);
-                        ctx->check_launch("level_runs");
-                    }
+        for (size_t l = 0; l < nlevels;) {
+            for (unsigned launches = 0; l < nlevels && launches < kWindow; ++launches) {
+                size_t r = l;
+                while (r < nlevels && level_begin[r + 1] - level_begin[r] <= kRunLevel) ++r;
+                if (r > l) {  // a run of small levels
+                    level_sweep<true, kRunWarps><<<1, kRunWarps * 32, 0, s>>>(ps, d_starts, static_cast<unsigned>(l),
+                                                                             static_cast<unsigned>(r));
+                    l = r;
                 } else {
-                    shift = rank_bits;
-                    auto* k64 = buf<unsigned long long>(ctx, "pores.lkeys", total);
-                    auto* k64b = buf<unsigned long long>(ctx, "pores.lkeys2", total);
-                    int64_t emitted = 0;
-                    {
-                        KernelTimer kt3(ctx, "merge_expand");
-                        level_expand<unsigned long long><<<eg, 256, 0, s>>>(ps, b, doff, deg, nbig, k64, total, shift);
-                        ctx->check_launch("level_expand");
-                        emitted = read_emitted();
-                    }
-                    const int bits = rank_bits + big_bits;  // radix passes over the used bits only
-                    {
-                        KernelTimer kt3(ctx, "merge_sort");
-                        sort_keys(ctx, k64, k64b, emitted, bits);
-                        merged = unique(ctx, k64b, k64, emitted, d_count);
-                    }
-                    keys = k64;
-                    if (merged) {
-                        level_runs<unsigned long long><<<grid_for(ctx, merged), 256, 0, s>>>(k64, merged, ps, shift);
-                        ctx->check_launch("level_runs");
-                    }
+                    const size_t k = level_begin[l + 1] - level_begin[l];
+                    const size_t blocks = std::max(std::min((k + kSweepWarps - 1) / kSweepWarps,
+                                                            static_cast<size_t>(ctx->num_sms) * 8),
+                                                   (k + kSweepList - 1) / kSweepList);
+                    level_sweep<false, kSweepWarps><<<static_cast<unsigned>(blocks), kSweepWarps * 32, 0, s>>>(
+                        ps, d_starts, static_cast<unsigned>(l), static_cast<unsigned>(l + 1));
+                    ++l;
                 }
+                ctx->count_launch();
             }
-            if (merged && !merged_dev) ctx->count("pores.big_set_elements_merged", static_cast<double>(merged));
-            KernelTimer kt3(ctx, "level_write");
-            exclusive_sum(ctx, ps.cnt, ps.off, static_cast<int64_t>(e - b));
-            level_write<<<lg, kLevelWarps * 32, 0, s>>>(ps, b, e, base);
-            ctx->count_launch(1);
-            if (merged) {
-                if (narrow)
-                    level_copy_big<uint32_t><<<grid_for(ctx, merged), 256, 0, s>>>(
-                        static_cast<uint32_t*>(keys), merged, ps, base, shift, nullptr);
-                else
-                    level_copy_big<unsigned long long><<<grid_for(ctx, merged), 256, 0, s>>>(
-                        static_cast<unsigned long long*>(keys), merged, ps, base, shift, merged_dev);
-                ctx->count_launch(1);
+            ctx->check_launch("level_sweep");
+            ReadBack rb;
+            rb.add(h_info, ps.info, 32);
+            read_back(ctx, rb);
+            if (h_info[0] != kNoStop) {  // go on behind the level that stopped
+                l = static_cast<size_t>(h_info[0]) + 1;
+                merge_hard(h_info[1], h_info[2]);
+                PMA_CUDA(cudaMemsetAsync(ps.info, 0xFF, 8, s));
+                PMA_CUDA(cudaMemsetAsync(ps.info + 1, 0, 24, s));
             }
-            level_advance<<<1, 32, 0, s>>>(base, ps.off, ps.cnt, e - b);
-            ctx->count_launch(1);
         }
-        ctx->check_launch("level_sets");
+        ctx->count("pores.levels", static_cast<double>(nlevels));
         unsigned int h_err = 0;
         unsigned long long used = 0;
         PMA_CUDA(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s));
-        PMA_CUDA(cudaMemcpyAsync(&used, base, 8, cudaMemcpyDeviceToHost, s));
+        PMA_CUDA(cudaMemcpyAsync(&used, ps.pool_n, 8, cudaMemcpyDeviceToHost, s));
         ctx->sync();
+        ctx->count("pores.pool_elements", static_cast<double>(used));
         PMA_REQUIRE(!(h_err & 32u), PMA_ERR_INTERNAL, "pma_pores: merged seed sets disagree with their bounds");
         if (!(h_err & 2u)) break;
         PMA_REQUIRE(attempt < 2, PMA_ERR_MEMORY, "pma_pores: seed-set pool overflow");
-        pool_cap = used + (used >> 2) + 1024;
+        pool_cap = 4 * used + 1024;
+    }
+    unsigned long long* soff = buf<unsigned long long>(ctx, "pores.soff", np);
+    uint32_t* slen = buf<uint32_t>(ctx, "pores.slen", np);
+    if (np) {
+        unpack_sets<<<grid_for(ctx, np), 256, 0, s>>>(ps.set, np, soff, slen);
+        ctx->check_launch("unpack_sets");
     }
 
     // Seeds -> pores in rank order.
@@ -1730,7 +1597,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     PMA_CUDA(cudaMemsetAsync(pa.pvol, 0, std::max<size_t>(npores, 1) * 8, s));
     PMA_CUDA(cudaMemsetAsync(pa.pbound, 0, std::max<size_t>(npores, 1) * 4, s));
     if (np) {
-        pore_accumulate<<<grid_for(ctx, np), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, psize, pface, np, pa);
+        pore_accumulate<<<grid_for(ctx, np), 256, 0, s>>>(soff, slen, ps.pool, psize, pface, np, pa);
         ctx->check_launch("pore_accumulate");
     }
 
@@ -1738,7 +1605,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     // Throats: plateaus with two or more seeds, grouped by equal seed sets.
     auto kt_groups = std::make_unique<KernelTimer>(ctx, "tables_groups");
     if (np) {
-        flag_multi<<<grid_for(ctx, np), 256, 0, s>>>(ps.slen, np, flags);
+        flag_multi<<<grid_for(ctx, np), 256, 0, s>>>(slen, np, flags);
         ctx->check_launch("flag_multi");
     }
     uint32_t* multi = buf<uint32_t>(ctx, "pores.multi", np);
@@ -1766,12 +1633,12 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         // equal (h1, h2) pairs side by side.
         uint32_t* gstart = buf<uint32_t>(ctx, "pores.gstart", nm);
         uint32_t* gid = buf<uint32_t>(ctx, "pores.gid", nm);
-        throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, multi, nm, h1, h2);
+        throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(soff, slen, ps.pool, multi, nm, h1, h2);
         ctx->check_launch("throat_hashes");
         sort_pairs(ctx, h1, ktmp, multi, v2, nm);
-        throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, v2, nm, h1, h2);
+        throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(soff, slen, ps.pool, v2, nm, h1, h2);
         ctx->check_launch("throat_hashes");
-        group_starts<<<grid_for(ctx, nm), 256, 0, s>>>(v2, h1, h2, nm, ps.soff, ps.slen, ps.pool, gstart, err);
+        group_starts<<<grid_for(ctx, nm), 256, 0, s>>>(v2, h1, h2, nm, soff, slen, ps.pool, gstart, err);
         ctx->check_launch("group_starts");
         {
             unsigned int h_err0 = 0;
@@ -1779,15 +1646,15 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
             ctx->sync();
             if (h_err0 & 64u) {
                 PMA_CUDA(cudaMemsetAsync(err, 0, 4, s));
-                throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, multi, nm, h1, h2);
+                throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(soff, slen, ps.pool, multi, nm, h1, h2);
                 ctx->check_launch("throat_hashes");
                 sort_pairs(ctx, h2, ktmp, multi, v1, nm);
-                throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, v1, nm, h1, h2);
+                throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(soff, slen, ps.pool, v1, nm, h1, h2);
                 ctx->check_launch("throat_hashes");
                 sort_pairs(ctx, h1, ktmp, v1, v2, nm);
-                throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, v2, nm, h1, h2);
+                throat_hashes<<<grid_for(ctx, nm), 256, 0, s>>>(soff, slen, ps.pool, v2, nm, h1, h2);
                 ctx->check_launch("throat_hashes");
-                group_starts<<<grid_for(ctx, nm), 256, 0, s>>>(v2, h1, h2, nm, ps.soff, ps.slen, ps.pool, gstart, err);
+                group_starts<<<grid_for(ctx, nm), 256, 0, s>>>(v2, h1, h2, nm, soff, slen, ps.pool, gstart, err);
                 ctx->check_launch("group_starts");
             }
         }
@@ -1821,7 +1688,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         // Representative seed lists, gathered into one buffer.
         std::vector<uint32_t> rlen(ngroups);
         uint32_t* d_rep_len = buf<uint32_t>(ctx, "pores.rlen", ngroups);
-        gather_u32<<<grid_for(ctx, ngroups), 256, 0, s>>>(ps.slen, go.grep, ngroups, d_rep_len);
+        gather_u32<<<grid_for(ctx, ngroups), 256, 0, s>>>(slen, go.grep, ngroups, d_rep_len);
         ctx->check_launch("gather_u32");
         PMA_CUDA(cudaMemcpyAsync(rlen.data(), d_rep_len, ngroups * 4, cudaMemcpyDeviceToHost, s));
         ctx->sync();
@@ -1830,7 +1697,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         auto* d_roff = buf<unsigned long long>(ctx, "pores.roff", ngroups + 1);
         uint32_t* d_rlist = buf<uint32_t>(ctx, "pores.rlist", roff[ngroups]);
         PMA_CUDA(cudaMemcpyAsync(d_roff, roff.data(), (ngroups + 1) * 8, cudaMemcpyHostToDevice, s));
-        gather_lists<<<grid_for(ctx, ngroups), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, go.grep, d_roff,
+        gather_lists<<<grid_for(ctx, ngroups), 256, 0, s>>>(soff, slen, ps.pool, go.grep, d_roff,
                                                             ngroups, d_rank2id, d_rlist);
         ctx->check_launch("gather_lists");
         flat.resize(roff[ngroups]);
@@ -1858,7 +1725,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     // Labels.
     uint32_t* plabel = buf<uint32_t>(ctx, "pores.plabel", np);
     if (np) {
-        plateau_labels<<<grid_for(ctx, np), 256, 0, s>>>(ps.soff, ps.slen, ps.pool, d_rank2id, plateau_group,
+        plateau_labels<<<grid_for(ctx, np), 256, 0, s>>>(soff, slen, ps.pool, d_rank2id, plateau_group,
                                                          group_tid, np, plabel);
         ctx->check_launch("plateau_labels");
     }
