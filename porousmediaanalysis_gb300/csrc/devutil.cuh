@@ -197,7 +197,7 @@ inline void read_back(pma_ctx* ctx, ReadBack rb) {
         PMA_CUDA(cudaHostGetDevicePointer(&d, rb.dst[k], 0));
         rb.dst[k] = d;
     }
-    read_back_kernel<<<1, 64, 0, ctx->stream>>>(rb);
+    read_back_kernel<<<1, 256, 0, ctx->stream>>>(rb);
     ctx->count_launch();
     ctx->check_launch("read_back");
     ctx->sync();
