@@ -7,14 +7,19 @@
 // relaxation that runs until nothing improves reaches it, so the parallel form below is
 // bit-identical in float32 (and in float64 against the float64 restatement).
 //
-// Bucketing: all step weights w are >= 1 (1, sqrt 2, sqrt 3, or 1 for D3Q7) and in
-// round-to-nearest fl(d + w) >= floor(d) + 1, so relaxing a voxel of bucket floor(d) = k
-// only reaches buckets k+1 and k+2. Bucket k is therefore final when it is processed and
-// one parallel sweep per bucket suffices (Dial's algorithm). Buckets are a ring of four
-// bitmaps over the voxels (a voxel is set in bucket b's bitmap when its distance drops into
-// b); before its sweep, bucket k's bitmap is compacted into a list in voxel order (per block
-// of 8192 voxels), which is also cleared for bucket k + 4. A voxel whose distance dropped to a
-// lower bucket after being set is skipped as stale.
+// Steps: all step weights w are >= 1 (1, sqrt 2, sqrt 3, or 1 for D3Q7) and in round-to-nearest
+// fl(d + w) >= floor(d) + 1, so the predecessor of a voxel of distance in [k, k + 1) has a
+// distance below k. Step k therefore settles exactly the unreached voxels whose minimum over
+// their neighbours is below k + 1, and their values are final. Each voxel pulls its own value:
+// it is written once, by one thread, with no atomics (pushing from the settled voxels instead
+// took an atomic minimum and a mark from each of up to nine neighbours that reach a voxel).
+// A neighbour settled in the same step may be seen or not: it has distance >= k and
+// gives at least k + 1, which settles nothing in step k.
+//
+// The volume is cut into bricks of 32 x 8 x 8 voxels (y, x, z). A step loads each brick of its
+// list with a one-voxel halo into shared memory and evaluates its unreached voxels. A brick
+// goes on the next step's list when it still holds unreached voxels that could be settled, or
+// when a neighbouring brick settled a voxel next to one of its unreached voxels.
 #include "devutil.cuh"
 
 #include <cfloat>
@@ -31,7 +36,11 @@ template <> struct Bits<float> {
     static __device__ __forceinline__ float from(U u) { return __uint_as_float(u); }
     static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
     static __host__ __device__ float unknown() { return FLT_MAX; }
-    static __device__ __forceinline__ int bucket(float d) { return static_cast<int>(floorf(d)); }
+    static __device__ __forceinline__ U infinity() { return 0x7F800000u; }
+    // Values in shared memory: solid (-1) becomes infinity. Distances are far below the bound used here.
+    static __device__ __forceinline__ U to_tile(U u) { return static_cast<int>(u) < 0 ? infinity() : u; }
+    static __device__ __forceinline__ bool is_settled(U u) { return u < 0x7F000000u; }
+    static __device__ __forceinline__ bool is_unreached(U u) { return u == 0x7F7FFFFFu; }
 };
 template <> struct Bits<double> {
     typedef unsigned long long U;
@@ -39,36 +48,52 @@ template <> struct Bits<double> {
     static __device__ __forceinline__ double from(U u) { return __longlong_as_double(static_cast<long long>(u)); }
     static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
     static __host__ __device__ double unknown() { return DBL_MAX; }
-    static __device__ __forceinline__ int bucket(double d) { return static_cast<int>(floor(d)); }
+    static __device__ __forceinline__ U infinity() { return 0x7FF0000000000000ull; }
+    // (the high words alone decide)
+    static __device__ __forceinline__ U to_tile(U u) { return static_cast<int>(u >> 32) < 0 ? infinity() : u; }
+    static __device__ __forceinline__ bool is_settled(U u) { return static_cast<uint32_t>(u >> 32) < 0x7FE00000u; }
+    static __device__ __forceinline__ bool is_unreached(U u) { return static_cast<uint32_t>(u >> 32) == 0x7FEFFFFFu; }
 };
 
 struct Geo {
     int SX, SY, SZ;
-    FastDiv fy, fx;  // division by SY and by SX (multiply-high)
-    Geo() = default;
-    Geo(int sx, int sy, int sz) : SX(sx), SY(sy), SZ(sz), fy(static_cast<uint32_t>(sy)), fx(static_cast<uint32_t>(sx)) {}
     __device__ __forceinline__ size_t idx(int x, int y, int z) const {
         return (static_cast<size_t>(z) * SX + x) * SY + y;
     }
 };
 
-// Compaction chunks: 256 bitmap words (8192 voxels), one block step of geo_compact.
-constexpr int kChunkWords = 256;
-constexpr int kChunkShift = 13;  // voxel index -> chunk
+constexpr int kBrickY = 32, kBrickX = 8, kBrickZ = 8;
+constexpr int kHaloY = kBrickY + 2, kHaloX = kBrickX + 2, kHaloZ = kBrickZ + 2;
+constexpr int kBrickThreads = 32 * kBrickX;
+constexpr int kRing = 4;  // lists in use at once: step k appends to those of k + 1
 
-struct Frontier {
-    uint32_t* bits;        // four bitmaps of nwords words: bucket b uses bitmap b & 3
-    size_t nwords;
-    uint8_t* dirty;        // four flag arrays of nchunks bytes: a bit was set in the chunk
-    size_t nchunks;
-    unsigned int* count;   // [4] non-zero when a voxel was marked in that bitmap
-    uint32_t* list;        // the compacted bucket being swept
-    unsigned int* list_n;  // its length
-    uint32_t cap;          // list capacity
-    unsigned int* overflow;
+struct Bricks {
+    int BY, BX, BZ;          // bricks per axis
+    uint32_t n;              // in all
+    uint32_t* list;          // kRing lists of n bricks: step k reads list k & 3
+    unsigned int* count;     // [kRing]
+    uint32_t* mark;          // per brick: the last step (of all cavities) it was listed for
     unsigned long long* settled;  // voxels settled in this cavity
     unsigned int* walls;          // bit 2i: plane axis i at 0, bit 2i+1: at size-1
 };
+
+// Lists a brick for step k (epoch0: steps before this cavity's step 0).
+__device__ __forceinline__ void geo_list(const Bricks& b, uint32_t brick, int k, uint32_t epoch0) {
+    if (atomicExch(&b.mark[brick], epoch0 + static_cast<uint32_t>(k)) == epoch0 + static_cast<uint32_t>(k)) return;
+    const unsigned at = atomicAdd(&b.count[k & (kRing - 1)], 1u);
+    if (at < b.n) b.list[static_cast<size_t>(k & (kRing - 1)) * b.n + at] = brick;
+}
+
+__device__ __forceinline__ unsigned geo_walls(const Geo& g, int x, int y, int z) {
+    unsigned w = 0;
+    if (x == 0) w |= 1u;
+    if (x == g.SX - 1 && g.SX > 1) w |= 2u;
+    if (y == 0) w |= 4u;
+    if (y == g.SY - 1 && g.SY > 1) w |= 8u;
+    if (z == 0) w |= 16u;
+    if (z == g.SZ - 1 && g.SZ > 1) w |= 32u;
+    return w;
+}
 
 template <class T>
 __global__ void geo_init(const uint8_t* __restrict__ solid, size_t n, T* __restrict__ dist,
@@ -81,156 +106,215 @@ __global__ void geo_init(const uint8_t* __restrict__ solid, size_t n, T* __restr
     }
 }
 
+// The start voxel, settled in step 0; the bricks around it go on the list of step 1.
 template <class T>
-__global__ void geo_start(Frontier f, T* dist, uint32_t v) {
-    dist[v] = static_cast<T>(0);
-    f.bits[v >> 5] |= 1u << (v & 31);  // bucket 0
-    f.dirty[v >> kChunkShift] = 1;
-    f.count[0] = 1;
-}
-
-// Bucket k's bitmap -> list (voxel order within each block's 8192 voxels), cleared behind.
-// Only chunks whose flag is set are read: a bucket is a thin shell of the volume, and reading
-// the whole bitmap for each bucket took a quarter of the geodesic kernels' time at 512^3.
-__global__ void __launch_bounds__(kChunkWords) geo_compact(Frontier f, int k) {
-    __shared__ unsigned int wsum[kChunkWords / 32];
-    __shared__ unsigned int base;
-    uint32_t* bm = f.bits + static_cast<size_t>(k & 3) * f.nwords;
-    uint8_t* dirty = f.dirty + static_cast<size_t>(k & 3) * f.nchunks;
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (size_t ch = blockIdx.x; ch < f.nchunks; ch += gridDim.x) {
-        if (!dirty[ch]) continue;  // the same byte for the whole block: a uniform skip
-        const size_t w = ch * kChunkWords + threadIdx.x;
-        uint32_t word = 0;
-        if (w < f.nwords) {
-            word = bm[w];
-            if (word) bm[w] = 0;
-        }
-        const unsigned c = __popc(word);
-        unsigned incl = c;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= static_cast<unsigned>(o)) incl += t;
-        }
-        if (lane == 31) wsum[warp] = incl;
-        __syncthreads();  // every thread has read the flag
-        if (threadIdx.x == 0) {
-            dirty[ch] = 0;
-            unsigned tot = 0;
-            for (int i = 0; i < kChunkWords / 32; ++i) {
-                const unsigned v = wsum[i];
-                wsum[i] = tot;
-                tot += v;
-            }
-            base = tot ? atomicAdd(f.list_n, tot) : 0u;
-        }
-        __syncthreads();
-        unsigned pos = base + wsum[warp] + incl - c;
-        while (word) {
-            const int bit = __ffs(word) - 1;
-            word &= word - 1;
-            if (pos < f.cap) f.list[pos] = static_cast<uint32_t>(w * 32 + bit);
-            else atomicExch(f.overflow, 1u);
-            ++pos;
-        }
-        __syncthreads();
-    }
-}
-
-// Processes bucket k: settle its voxels and relax their neighbours. One thread per list
-// entry: it reads its own distance, then issues the loads of all its neighbours' distances at
-// once (26 independent loads in flight per thread hide their latency; the list is in voxel
-// order, so a warp's loads of one stencil position fall on neighbouring addresses), then
-// lowers the neighbours it improves. Each voxel is in the list once, so a live entry
-// (bucket(dist) == k) is settled exactly once. Steps are in [1, 2), so pushes go to buckets
-// k + 1 and k + 2 only; whether a bucket got any is flagged per warp at the end (the host
-// only asks whether the next buckets are empty).
-// Four blocks per SM (64 registers; the float64 form spills about 100 bytes to L1): more
-// warps hide more of the neighbour loads' latency than the spilled registers cost (the float64
-// bucket loop of the 1024^3 spinodal: 338 ms at 120 registers, 299 ms at three blocks per SM,
-// 294 ms at four).
-template <class T, bool D3Q7>
-__global__ void __launch_bounds__(256, 4) geo_bucket(Geo g, T w1, T w2, T w3, T* __restrict__ dist,
-                                                  uint32_t* __restrict__ cavity, Frontier f, int k,
-                                                  uint32_t cavity_id) {
-    typedef typename Bits<T>::U U;
-    const unsigned n = min(*f.list_n, f.cap);
-    const uint32_t* list = f.list;
-    const long long sy = g.SY, sxy = static_cast<long long>(g.SX) * g.SY;
-    unsigned long long my_settled = 0;
-    unsigned my_walls = 0, c1 = 0, c2 = 0;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t v = list[i];
-        const T dv = dist[v];
-        if (Bits<T>::bucket(dv) != k) continue;  // stale: the voxel moved to a lower bucket
-        const uint32_t zx = g.fy.div(v);
-        const int y = static_cast<int>(v - zx * static_cast<uint32_t>(g.SY));
-        const uint32_t zz = g.fx.div(zx);
-        const int x = static_cast<int>(zx - zz * static_cast<uint32_t>(g.SX));
-        const int z = static_cast<int>(zz);
+__global__ void geo_start(Geo g, Bricks b, T* dist, uint32_t* cavity, int x, int y, int z, uint32_t cavity_id, uint32_t epoch0) {
+    const int dy = static_cast<int>(threadIdx.x) % 3 - 1, dx = static_cast<int>(threadIdx.x) / 3 % 3 - 1,
+              dz = static_cast<int>(threadIdx.x) / 9 - 1;
+    if (threadIdx.x == 0) {
+        const size_t v = g.idx(x, y, z);
+        dist[v] = static_cast<T>(0);
         cavity[v] = cavity_id;
-        ++my_settled;
-        const bool xl = x > 0, xh = x < g.SX - 1, yl = y > 0, yh = y < g.SY - 1, zl = z > 0, zh = z < g.SZ - 1;
-        if (!xl) my_walls |= 1u;
-        if (!xh && g.SX > 1) my_walls |= 2u;
-        if (!yl) my_walls |= 4u;
-        if (!yh && g.SY > 1) my_walls |= 8u;
-        if (!zl) my_walls |= 16u;
-        if (!zh && g.SZ > 1) my_walls |= 32u;
-        const T nd1 = Bits<T>::add(dv, D3Q7 ? static_cast<T>(1) : w1);
-        const T nd2 = Bits<T>::add(dv, w2), nd3 = Bits<T>::add(dv, w3);
-        T nb[27];
-#pragma unroll
-        for (int j = 0; j < 27; ++j) {
-            const int dx = j / 9 - 1, dy = (j / 3) % 3 - 1, dz = j % 3 - 1;
-            const int kk = dx * dx + dy * dy + dz * dz;
-            if (kk == 0 || (D3Q7 && kk != 1)) continue;
-            const bool ok = (dx < 0 ? xl : (dx > 0 ? xh : true)) && (dy < 0 ? yl : (dy > 0 ? yh : true)) &&
-                            (dz < 0 ? zl : (dz > 0 ? zh : true));
-            // out of the box reads as -1, like a solid voxel: never improved
-            nb[j] = ok ? dist[static_cast<long long>(v) + dz * sxy + dx * sy + dy] : static_cast<T>(-1);
-        }
-#pragma unroll
-        for (int j = 0; j < 27; ++j) {
-            const int dx = j / 9 - 1, dy = (j / 3) % 3 - 1, dz = j % 3 - 1;
-            const int kk = dx * dx + dy * dy + dz * dz;
-            if (kk == 0 || (D3Q7 && kk != 1)) continue;
-            const T nd = kk == 1 ? nd1 : (kk == 2 ? nd2 : nd3);
-            if (nd < nb[j]) {
-                // Neither update waits for its old value (reductions, no round trip): the bit
-                // marks the voxel in nd's bucket even when another thread has lowered it further
-                // meanwhile, and such an entry is skipped as stale when its bucket comes (the
-                // lowest value's bucket has its bit from the thread that wrote that value).
-                const size_t w = static_cast<size_t>(static_cast<long long>(v) + dz * sxy + dx * sy + dy);
-                atomicMin(reinterpret_cast<U*>(dist + w), Bits<T>::to(nd));
-                const int pb = Bits<T>::bucket(nd);
-                const uint32_t bit = 1u << (w & 31);
-                atomicOr(&f.bits[static_cast<size_t>(pb & 3) * f.nwords + (w >> 5)], bit);
-                f.dirty[static_cast<size_t>(pb & 3) * f.nchunks + (w >> kChunkShift)] = 1;
-                if (pb == k + 1) c1 = 1;
-                else if (pb == k + 2) c2 = 1;
-                else atomicOr(&f.count[pb & 3], 1u);  // not reachable with steps in [1, 2)
-            }
-        }
+        *b.settled = 1;
+        *b.walls = geo_walls(g, x, y, z);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        my_settled += __shfl_xor_sync(0xFFFFFFFFu, my_settled, o);
-        my_walls |= __shfl_xor_sync(0xFFFFFFFFu, my_walls, o);
-        c1 |= __shfl_xor_sync(0xFFFFFFFFu, c1, o);
-        c2 |= __shfl_xor_sync(0xFFFFFFFFu, c2, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (my_settled) atomicAdd(f.settled, my_settled);
-        if (my_walls) atomicOr(f.walls, my_walls);
-        if (c1) atomicOr(&f.count[(k + 1) & 3], 1u);
-        if (c2) atomicOr(&f.count[(k + 2) & 3], 1u);
-    }
+    const int ny = y + dy, nx = x + dx, nz = z + dz;
+    if (threadIdx.x < 27 && ny >= 0 && ny < g.SY && nx >= 0 && nx < g.SX && nz >= 0 && nz < g.SZ)
+        geo_list(b, static_cast<uint32_t>((nz / kBrickZ * b.BX + nx / kBrickX) * b.BY + ny / kBrickY), 1, epoch0);
 }
 
-// Before bucket k is compacted: empty the list and its bitmap count.
-__global__ void geo_next(Frontier f, int k) {
-    *f.list_n = 0;
-    f.count[k & 3] = 0;
+// A row of three mask words, one bit to either side (26 neighbours) or the bits themselves.
+__device__ __forceinline__ unsigned long long geo_spread(unsigned long long m) { return m | m << 1 | m >> 1; }
+
+// Neighbours of the set bits of the halo's rows (34-bit masks, [slice][row]) in row (x, z).
+template <bool D3Q7, class F>
+__device__ __forceinline__ unsigned long long geo_dilate(F mask, int x, int z) {
+    unsigned long long m = 0;
+    if (D3Q7) {
+        const unsigned long long own = mask(x, z);
+        return own << 1 | own >> 1 | mask(x - 1, z) | mask(x + 1, z) | mask(x, z - 1) | mask(x, z + 1);
+    }
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) m |= mask(x + dx, z + dz);
+    return geo_spread(m);
+}
+
+// Step k, one block per listed brick. The brick's values and its halo's go to shared memory, with
+// one bit mask per row of settled and of unreached voxels; the unreached neighbours of settled
+// voxels (a tenth of the brick's) are listed from the masks and evaluated, one thread each; the masks of
+// what was settled then say which bricks are listed for the next step. Distances are compared as
+// unsigned integers (their bits order as the values do): solid reads as infinity, unreached as
+// the largest finite value. The least neighbour per step weight is found first and only three
+// sums are formed (rounding is monotone).
+// What bounds it: the bricks' loads (27 KB of a float64 brick with its halo, once for each of the
+// about 25 steps that the front takes through a brick: 330 B a voxel) and the block's barriers.
+// Five blocks an SM (48 registers, the loads of a whole brick in flight); six spill (1024^3 spinodal,
+// float64: 121 against 157 ms). Before and after, ms: that volume 253 -> 121 (a step of 14000
+// bricks 130 us, 2.9 TB/s of brick loads); 301 x 257 x 411 field, float32, D3Q7 10.2 -> 6.6.
+template <class T, bool D3Q7>
+__global__ void __launch_bounds__(kBrickThreads, 5)
+    geo_step(Geo g, T w1, T w2, T w3, T* __restrict__ dist, uint32_t* __restrict__ cavity, Bricks b, int k, uint32_t cavity_id,
+             uint32_t epoch0) {
+    typedef typename Bits<T>::U U;
+    constexpr int kRows = kHaloX * kHaloZ, kOwnRows = kBrickX * kBrickZ;
+    __shared__ U tile[kRows * kHaloY];
+    __shared__ uint32_t settled[kRows], unreached[kRows];
+    __shared__ uint16_t todo[kOwnRows * kBrickY];                    // candidates: row * 32 + voxel
+    __shared__ uint32_t now[kOwnRows];                               // settled in this step
+    __shared__ uint8_t edge[2][kRows];                               // halo columns: bit 0 settled, bit 1 unreached
+    __shared__ unsigned s_todo, s_next;                              // s_next: bricks to list (bit 13: this one)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned n = min(b.count[k & (kRing - 1)], b.n);
+    const uint32_t* list = b.list + static_cast<size_t>(k & (kRing - 1)) * b.n;
+    if (blockIdx.x == 0 && tid == 0) b.count[(k - 1) & (kRing - 1)] = 0;  // read by the step before, written by the one after next
+    const U kSolid = Bits<T>::infinity();
+    const T end = static_cast<T>(k) + static_cast<T>(1);
+    unsigned long long my_settled = 0;
+    unsigned my_walls = 0;
+    uint32_t brick = blockIdx.x < n ? list[blockIdx.x] : 0u;
+    for (unsigned i = blockIdx.x; i < n; i += gridDim.x) {
+        const uint32_t rest = brick / static_cast<uint32_t>(b.BY);
+        const int by = static_cast<int>(brick - rest * static_cast<uint32_t>(b.BY));
+        const int bz = static_cast<int>(rest / static_cast<uint32_t>(b.BX)), bx = static_cast<int>(rest) - bz * b.BX;
+        const int y0 = by * kBrickY, x0 = bx * kBrickX, z0 = bz * kBrickZ;
+        if (i + gridDim.x < n) brick = list[i + gridDim.x];
+        // Rows of the halo's slices, a warp a row: warp w takes row w of each slice (pointers advance by
+        // a plane), then its share of rows 8 and 9. Lane q keeps the masks of the warp's q-th row.
+        {
+            const int y = y0 + lane;
+            const size_t plane = static_cast<size_t>(g.SX) * g.SY;
+            uint32_t ms = 0, mu = 0;
+            auto put = [&](int q, int r, U u) {
+                u = Bits<T>::to_tile(u);
+                tile[r * kHaloY + 1 + lane] = u;
+                const unsigned bs = __ballot_sync(0xFFFFFFFFu, Bits<T>::is_settled(u)),
+                               bu = __ballot_sync(0xFFFFFFFFu, Bits<T>::is_unreached(u));
+                if (lane == q) {
+                    ms = bs;
+                    mu = bu;
+                }
+            };
+            constexpr int kRest = 2 * kHaloZ, kMore = (kRest + 7) / 8;  // rows 8 and 9 of each slice
+            // every load first
+            U u[kHaloZ], more[kMore], e = kSolid;
+            {
+                const int x = x0 - 1 + warp;
+                const bool in = x >= 0 && x < g.SX && y < g.SY;
+                const T* p = dist + (static_cast<long long>(z0 - 1) * g.SX + x) * g.SY + y;
+#pragma unroll
+                for (int q = 0; q < kHaloZ; ++q, p += plane)
+                    u[q] = in && static_cast<unsigned>(z0 - 1 + q) < static_cast<unsigned>(g.SZ) ? Bits<T>::to(*p) : kSolid;
+            }
+#pragma unroll
+            for (int q = 0; q < kMore; ++q) {
+                const int i2 = q * 8 + warp, x = x0 - 1 + kBrickX + (i2 & 1), z = z0 - 1 + (i2 >> 1);
+                more[q] = kSolid;
+                if (i2 < kRest && x < g.SX && static_cast<unsigned>(z) < static_cast<unsigned>(g.SZ) && y < g.SY)
+                    more[q] = Bits<T>::to(dist[g.idx(x, y, z)]);
+            }
+            const int er = tid >> 1, side = tid & 1;  // the halo's columns
+            if (tid < 2 * kRows) {
+                const int x = x0 - 1 + er % kHaloX, z = z0 - 1 + er / kHaloX, ye = side ? y0 + kBrickY : y0 - 1;
+                if (static_cast<unsigned>(x) < static_cast<unsigned>(g.SX) && static_cast<unsigned>(z) < static_cast<unsigned>(g.SZ) &&
+                    static_cast<unsigned>(ye) < static_cast<unsigned>(g.SY))
+                    e = Bits<T>::to(dist[g.idx(x, ye, z)]);
+            }
+#pragma unroll
+            for (int q = 0; q < kHaloZ; ++q) put(q, q * kHaloX + warp, u[q]);
+#pragma unroll
+            for (int q = 0; q < kMore; ++q)
+                if (q * 8 + warp < kRest) put(kHaloZ + q, ((q * 8 + warp) >> 1) * kHaloX + kBrickX + (warp & 1), more[q]);
+            if (tid < 2 * kRows) {
+                e = Bits<T>::to_tile(e);
+                tile[er * kHaloY + side * (kHaloY - 1)] = e;
+                edge[side][er] = (Bits<T>::is_settled(e) ? 1 : 0) | (Bits<T>::is_unreached(e) ? 2 : 0);
+            }
+            const int own = lane < kHaloZ ? lane * kHaloX + warp : (lane - kHaloZ) * 8 + warp < kRest && lane < kHaloZ + 3
+                                ? (((lane - kHaloZ) * 8 + warp) >> 1) * kHaloX + kBrickX + (warp & 1) : -1;
+            if (own >= 0) {
+                settled[own] = ms;
+                unreached[own] = mu;
+            }
+            if (tid < kOwnRows) now[tid] = 0;
+            if (tid == 0) s_todo = s_next = 0;
+        }
+        __syncthreads();
+        // a row's mask with the halo's columns: bits 0 and 33
+        auto settled_row = [&](int x, int z) {
+            const int r = z * kHaloX + x;
+            return static_cast<unsigned long long>(settled[r]) << 1 | (edge[0][r] & 1u) | static_cast<unsigned long long>(edge[1][r] & 1u) << 33;
+        };
+        if (tid < kOwnRows) {
+            const int x = tid % kBrickX + 1, z = tid / kBrickX + 1;
+            uint32_t c = static_cast<uint32_t>(geo_dilate<D3Q7>(settled_row, x, z) >> 1) & unreached[z * kHaloX + x];
+            uint32_t at = c ? atomicAdd(&s_todo, static_cast<unsigned>(__popc(c))) : 0u;
+            for (; c; c &= c - 1) todo[at++] = static_cast<uint16_t>(tid * 32 + __ffs(c) - 1);
+        }
+        __syncthreads();
+        const unsigned m = s_todo;
+        for (unsigned c = tid; c < m; c += kBrickThreads) {
+            const int own = todo[c], ly = own & 31, r = own >> 5, lx = r % kBrickX, lz = r / kBrickX;
+            const U* q = tile + ((lz + 1) * kHaloX + lx + 1) * kHaloY + ly + 1;
+            constexpr int DX = kHaloY, DZ = kHaloX * kHaloY;
+            U face = min(min(min(q[-1], q[1]), min(q[-DX], q[DX])), min(q[-DZ], q[DZ]));
+            T t = Bits<T>::add(Bits<T>::from(face), D3Q7 ? static_cast<T>(1) : w1);
+            if (!D3Q7) {
+                U e = min(min(q[-DX - 1], q[-DX + 1]), min(q[DX - 1], q[DX + 1]));
+                e = min(e, min(min(q[-DZ - 1], q[-DZ + 1]), min(q[-DZ - DX], q[-DZ + DX])));
+                e = min(e, min(min(q[DZ - 1], q[DZ + 1]), min(q[DZ - DX], q[DZ + DX])));
+                U d = min(min(q[-DZ - DX - 1], q[-DZ - DX + 1]), min(q[-DZ + DX - 1], q[-DZ + DX + 1]));
+                d = min(d, min(min(q[DZ - DX - 1], q[DZ - DX + 1]), min(q[DZ + DX - 1], q[DZ + DX + 1])));
+                const T t2 = Bits<T>::add(Bits<T>::from(e), w2), t3 = Bits<T>::add(Bits<T>::from(d), w3);
+                t = t2 < t ? t2 : t;
+                t = t3 < t ? t3 : t;
+            }
+            if (t < end) {
+                const int y = y0 + ly, x = x0 + lx, z = z0 + lz;
+                const size_t v = g.idx(x, y, z);
+                dist[v] = t;
+                cavity[v] = cavity_id;
+                ++my_settled;
+                my_walls |= geo_walls(g, x, y, z);
+                atomicOr(&now[r], 1u << ly);
+            } else {
+                s_next = 1u << 13;  // a later step's: nothing else is in s_next yet
+            }
+        }
+        __syncthreads();
+        if (tid < kRows) {  // unreached neighbours of what was settled, row by row of the halo
+            const int px = tid % kHaloX, pz = tid / kHaloX;
+            auto mask = [&](int mx, int mz) {
+                return mx >= 1 && mx <= kBrickX && mz >= 1 && mz <= kBrickZ
+                           ? static_cast<unsigned long long>(now[(mz - 1) * kBrickX + mx - 1]) << 1
+                           : 0ull;
+            };
+            const unsigned long long open = static_cast<unsigned long long>(unreached[tid]) << 1 | (edge[0][tid] >> 1) |
+                                            static_cast<unsigned long long>(edge[1][tid] >> 1) << 33;
+            const unsigned long long hit = geo_dilate<D3Q7>(mask, px, pz) & open & ~mask(px, pz);
+            const int sz = pz == 0 ? 0 : (pz == kHaloZ - 1 ? 2 : 1), sx = px == 0 ? 0 : (px == kHaloX - 1 ? 2 : 1);
+            unsigned next = 0;
+            if (hit & 1ull) next |= 1u;
+            if (hit & 0x1FFFFFFFEull) next |= 2u;
+            if (hit >> 33) next |= 4u;
+            if (next) atomicOr(&s_next, next << (sz * 9 + sx * 3));
+        }
+        __syncthreads();
+        if (tid < 27 && ((s_next >> tid) & 1u)) {
+            const int nz = bz + tid / 9 - 1, nx = bx + tid / 3 % 3 - 1, ny = by + tid % 3 - 1;
+            if (nz >= 0 && nz < b.BZ && nx >= 0 && nx < b.BX && ny >= 0 && ny < b.BY)
+                geo_list(b, static_cast<uint32_t>((nz * b.BX + nx) * b.BY + ny), k + 1, epoch0);
+        }
+        // no barrier: what the next brick's loads overwrite was read before the last one, and the
+        // thread that clears s_next is one of those that just read it
+    }
+    for (int o = 16; o > 0; o >>= 1) my_settled += __shfl_xor_sync(0xFFFFFFFFu, my_settled, o);
+    my_walls = __reduce_or_sync(0xFFFFFFFFu, my_walls);
+    if (lane == 0) {
+        if (my_settled) atomicAdd(b.settled, my_settled);
+        if (my_walls) atomicOr(b.walls, my_walls);
+    }
 }
 
 // Start-voxel search on box shells h0 .. h0+nh-1 around the centre, in the reference's
@@ -286,28 +370,21 @@ std::vector<pma_cavity> geodesic(pma_ctx* ctx, const uint8_t* solid, pma_dims d,
             w3 = std::sqrt(static_cast<T>(3));  // SPC.cpp:31-36
     const unsigned grid = static_cast<unsigned>(std::min<size_t>(div_up(n, 256), ctx->num_sms * 16ull));
 
-    const uint32_t cap = static_cast<uint32_t>(std::min<size_t>(n, size_t(1) << 28));
-    const size_t nwords = (n + 31) / 32;
-    auto* bits = static_cast<uint32_t*>(ctx->scratch("geo.bits", 4 * nwords * 4));
-    const size_t nchunks = (nwords + kChunkWords - 1) / kChunkWords;
-    auto* dirty = static_cast<uint8_t*>(ctx->scratch("geo.dirty", 4 * nchunks));
-    auto* list = static_cast<uint32_t*>(ctx->scratch("geo.list", static_cast<size_t>(cap) * 4));
+    Bricks br;
+    br.BY = (d.sy + kBrickY - 1) / kBrickY;
+    br.BX = (d.sx + kBrickX - 1) / kBrickX;
+    br.BZ = (d.sz + kBrickZ - 1) / kBrickZ;
+    const size_t nbricks = static_cast<size_t>(br.BY) * br.BX * br.BZ;
+    br.n = static_cast<uint32_t>(nbricks);
+    br.list = static_cast<uint32_t*>(ctx->scratch("geo.list", kRing * nbricks * 4));
+    br.mark = static_cast<uint32_t*>(ctx->scratch("geo.mark", nbricks * 4));
     auto* misc = static_cast<unsigned long long*>(ctx->scratch("geo.misc", 64));
-    Frontier f;
-    f.bits = bits;
-    f.nwords = nwords;
-    f.dirty = dirty;
-    f.nchunks = nchunks;
-    f.list = list;
-    f.count = reinterpret_cast<unsigned int*>(misc);          // 4 x u32 = misc[0..1]
-    f.overflow = reinterpret_cast<unsigned int*>(misc + 2);   // misc[2] low
-    f.walls = reinterpret_cast<unsigned int*>(misc + 3);      // misc[3] low
-    f.settled = misc + 4;
+    br.count = reinterpret_cast<unsigned int*>(misc);          // 4 x u32 = misc[0..1]
+    br.walls = reinterpret_cast<unsigned int*>(misc + 3);      // misc[3] low
+    br.settled = misc + 4;
     unsigned long long* best = misc + 5;
-    f.list_n = reinterpret_cast<unsigned int*>(misc + 6);     // misc[6] low
-    f.cap = cap;
-    PMA_CUDA(cudaMemsetAsync(bits, 0, 4 * nwords * 4, s));
-    PMA_CUDA(cudaMemsetAsync(dirty, 0, 4 * nchunks, s));
+    PMA_CUDA(cudaMemsetAsync(br.mark, 0, nbricks * 4, s));
+    uint32_t epoch0 = 0;  // steps of the cavities before this one: marks of different cavities differ
 
     geo_init<T><<<grid, 256, 0, s>>>(solid, n, dist, cavity);
     ctx->check_launch("geo_init");
@@ -325,10 +402,9 @@ std::vector<pma_cavity> geodesic(pma_ctx* ctx, const uint8_t* solid, pma_dims d,
     int half = 0;
     uint32_t cavity_id = 0;
     std::vector<pma_cavity> rows;
-    const int max_buckets_per_sync = 32;
+    const int max_steps_per_sync = 32;
     const uint64_t bucket_limit = ctx->limits.geodesic_buckets ? ctx->limits.geodesic_buckets : 2ull * n + 64;
-    const unsigned bucket_grid = static_cast<unsigned>(ctx->num_sms * 8);
-    const unsigned compact_grid = static_cast<unsigned>(std::min<size_t>(nchunks, ctx->num_sms * 8ull));
+    const unsigned step_grid = static_cast<unsigned>(std::min<size_t>(nbricks, ctx->num_sms * 5ull));  // all resident
     while (true) {  // SPC.cpp:94-140
         ++half;
         // SelectStartingPosition (SPC.cpp:396-426)
@@ -386,40 +462,28 @@ std::vector<pma_cavity> geodesic(pma_ctx* ctx, const uint8_t* solid, pma_dims d,
         if (!found) break;
 
         cavity_id += 127;
-        PMA_CUDA(cudaMemsetAsync(misc, 0, 5 * 8, s));  // counts, overflow, walls, settled
-        const size_t sidx = (static_cast<size_t>(start[2]) * d.sx + start[0]) * d.sy + start[1];
-        geo_start<T><<<1, 1, 0, s>>>(f, dist, static_cast<uint32_t>(sidx));
+        PMA_CUDA(cudaMemsetAsync(misc, 0, 5 * 8, s));  // counts, walls, settled
+        geo_start<T><<<1, 32, 0, s>>>(g, br, dist, cavity, start[0], start[1], start[2], cavity_id, epoch0);
         ctx->check_launch("geo_start");
-        int k = 0;
+        int k = 1;
         while (true) {
             KernelTimer kt(ctx, "geo_bucket");
-            for (int i = 0; i < max_buckets_per_sync; ++i, ++k) {
-                geo_next<<<1, 1, 0, s>>>(f, k);
-                geo_compact<<<compact_grid, kChunkWords, 0, s>>>(f, k);
-                if (d3q7) geo_bucket<T, true><<<bucket_grid, 256, 0, s>>>(g, w1, w2, w3, dist, cavity, f, k, cavity_id);
-                else geo_bucket<T, false><<<bucket_grid, 256, 0, s>>>(g, w1, w2, w3, dist, cavity, f, k, cavity_id);
+            for (int i = 0; i < max_steps_per_sync; ++i, ++k) {
+                if (d3q7) geo_step<T, true><<<step_grid, kBrickThreads, 0, s>>>(g, w1, w2, w3, dist, cavity, br, k, cavity_id, epoch0);
+                else geo_step<T, false><<<step_grid, kBrickThreads, 0, s>>>(g, w1, w2, w3, dist, cavity, br, k, cavity_id, epoch0);
             }
-            ctx->count_launch(3 * max_buckets_per_sync - 1);
-            ctx->check_launch("geo_bucket");
-            {
-                ReadBack rb;
-                rb.add(h, misc, 3 * 8);
-                read_back(ctx, rb);
-            }
-            const unsigned* cnt = reinterpret_cast<const unsigned*>(h);
-            PMA_REQUIRE(reinterpret_cast<const unsigned*>(h)[4] == 0, PMA_ERR_LIMIT,
-                        "geodesic: frontier list overflow");
-            // after bucket k-1: lists of buckets k and k+1 hold all pending work
-            if (cnt[k & 3] == 0 && cnt[(k + 1) & 3] == 0) break;
-            // Distances are below 2 per voxel step, so no bucket index can exceed 2n.
-            PMA_REQUIRE(static_cast<uint64_t>(k) <= bucket_limit, PMA_ERR_LIMIT,
-                        "geodesic: bucket sweep did not terminate");
-        }
-        {
+            ctx->count_launch(max_steps_per_sync - 1);
+            ctx->check_launch("geo_step");
             ReadBack rb;
             rb.add(h, misc, 5 * 8);
             read_back(ctx, rb);
+            // the list of step k holds all pending work
+            if (reinterpret_cast<const unsigned*>(h)[k & (kRing - 1)] == 0) break;
+            // Distances are below 2 per voxel step, so no step can exceed 2n.
+            PMA_REQUIRE(static_cast<uint64_t>(k) <= bucket_limit, PMA_ERR_LIMIT,
+                        "geodesic: bucket sweep did not terminate");
         }
+        epoch0 += static_cast<uint32_t>(k) + 1;
         ctx->count("geo.buckets", k);
         const unsigned walls_bits = static_cast<unsigned>(h[3]);
         const unsigned long long settled = h[4];
