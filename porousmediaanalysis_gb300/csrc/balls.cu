@@ -20,9 +20,15 @@
 // the whole tile, which every voxel of the tile is covered by). One CTA per tile orders its
 // list by radius in shared memory, and each warp of voxels takes, per voxel, the largest key
 // among the entries whose ball covers it: the reference's winner. A warp only tests entries
-// that reach its 1 x 4 x 8 box and beat its lanes' smallest key so far, and stops where the
+// that reach its 2 x 4 x 4 box and beat its lanes' smallest key so far, and stops where the
 // radius order shows that no later entry can, so the work is close to the winners' ranks in
 // the list rather than the ball volumes a scatter would touch.
+//
+// What bounds it: instructions in the gather (half the issue slots), atomics in the count and the fill (1.3
+// entries per voxel of a spinodal). 704 x 768 x 811 spinodal, before and after these forms, ms: kept
+// centres 13 -> 2.9, floors and counts 23 -> 19.9, fill 19 -> 18.2, gather 117 -> 44 (least key by
+// 32-bit reductions and 2 x 4 x 4 boxes 82, centres by descending radius 73, the box of the lanes still
+// open 44); stage 170 -> 91.
 #include <thrust/iterator/counting_iterator.h>
 
 #include <vector>
@@ -69,53 +75,75 @@ __global__ void balls_containment_table(uint32_t* __restrict__ m1, uint32_t* __r
     m3[R] = b3;
 }
 
-__device__ __forceinline__ bool dominated(const uint32_t* __restrict__ edt2, Grid g, int x, int y,
-                                          int z, uint32_t R, const uint32_t* __restrict__ mtab,
-                                          uint32_t ntab) {
-    for (int dz = -1; dz <= 1; ++dz) {
-        const int nz = z + dz;
-        if (nz < 0 || nz >= g.SZ) continue;
-        for (int dx = -1; dx <= 1; ++dx) {
-            const int nx = x + dx;
-            if (nx < 0 || nx >= g.SX) continue;
-            for (int dy = -1; dy <= 1; ++dy) {
-                const int ny = y + dy;
-                if (ny < 0 || ny >= g.SY) continue;
-                const int k = dx * dx + dy * dy + dz * dz;
-                if (k == 0) continue;
-                const uint32_t Rn = __ldg(edt2 + g.idx(nx, ny, nz));
-                if (Rn <= R) continue;
-                if (R < ntab) {
-                    if (Rn >= __ldg(mtab + (k - 1) * ntab + R)) return true;
-                } else {
-                    // (sqrt(R) + sqrt(k))^2 <= Rn  <=>  t >= 0 and t^2 >= 4kR, t = Rn - R - k
-                    const long long t = static_cast<long long>(Rn) - R - k;
-                    if (t >= 0 && static_cast<unsigned long long>(t) * t >=
-                                      4ull * static_cast<unsigned long long>(k) * R)
-                        return true;
-                }
-            }
-        }
-    }
-    return false;
+// B(c, R) lies inside the ball of a neighbour at squared distance k whose r^2 is Rn: Rn >= M_k(R), or the
+// continuous bound where the table ends. Both grow with Rn: the largest Rn of each k decides.
+__device__ __forceinline__ bool contained(uint32_t R, uint32_t Rn, int k, const uint32_t* __restrict__ mtab, uint32_t ntab) {
+    if (Rn <= R) return false;
+    if (R < ntab) return Rn >= __ldg(mtab + (k - 1) * ntab + R);
+    // (sqrt(R) + sqrt(k))^2 <= Rn  <=>  t >= 0 and t^2 >= 4kR, t = Rn - R - k
+    const long long t = static_cast<long long>(Rn) - R - k;
+    return t >= 0 && static_cast<unsigned long long>(t) * t >= 4ull * static_cast<unsigned long long>(k) * R;
 }
 
-__global__ void balls_candidate_flags(const uint32_t* __restrict__ edt2, Grid g, size_t n,
-                                      const uint32_t* __restrict__ mtab, uint32_t ntab, uint32_t nR,
-                                      uint8_t* __restrict__ flags, unsigned int* __restrict__ err) {
-    PMA_GRID_STRIDE(v, n) {
-        const uint32_t R = edt2[v];
-        uint8_t f = 0;
-        if (R != 0) {
+// Kept centres (flag 1). A block takes a brick of 32 x 8 x 8 voxels (y, x, z) with its halo in shared
+// memory; a thread walks the eight slices of its (x, y), and of each slice takes its own value,
+// the largest of the four neighbours at distance 1 and the largest of the four diagonal ones:
+// three slices together give the largest neighbour at each distance. (Reading up to 26
+// neighbours and table entries a voxel through L1 took 12.4 ms on 704 x 768 x 811 voxels, this 2.9.)
+constexpr int kBrickY = 32, kBrickX = 8, kBrickZ = 8;
+constexpr int kHaloY = kBrickY + 2, kHaloX = kBrickX + 2, kHaloZ = kBrickZ + 2;
+
+__global__ void __launch_bounds__(32 * kBrickX) balls_candidate_flags(const uint32_t* __restrict__ edt2, Grid g, int BY, int BX,
+                                                                      const uint32_t* __restrict__ mtab, uint32_t ntab,
+                                                                      uint32_t nR, uint8_t* __restrict__ flags,
+                                                                      unsigned int* __restrict__ err) {
+    constexpr int kRows = kHaloX * kHaloZ;
+    __shared__ uint32_t tile[kRows * kHaloY];
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const unsigned rest = blockIdx.x / static_cast<unsigned>(BY);
+    const int y0 = static_cast<int>(blockIdx.x - rest * static_cast<unsigned>(BY)) * kBrickY;
+    const int z0 = static_cast<int>(rest / static_cast<unsigned>(BX)) * kBrickZ;
+    const int x0 = static_cast<int>(rest % static_cast<unsigned>(BX)) * kBrickX;
+    auto value = [&](int x, int y, int z) { return g.inside(x, y, z) ? __ldg(edt2 + g.idx(x, y, z)) : 0u; };
+#pragma unroll
+    for (int q = 0; q < (kRows + kBrickX - 1) / kBrickX; ++q) {
+        const int r = q * kBrickX + row;
+        if (r < kRows) tile[r * kHaloY + 1 + lane] = value(x0 - 1 + r % kHaloX, y0 + lane, z0 - 1 + r / kHaloX);
+    }
+    if (threadIdx.x < 2 * kRows) {
+        const int r = threadIdx.x >> 1, side = threadIdx.x & 1;
+        tile[r * kHaloY + side * (kHaloY - 1)] = value(x0 - 1 + r % kHaloX, side ? y0 + kBrickY : y0 - 1, z0 - 1 + r / kHaloX);
+    }
+    __syncthreads();
+    const uint32_t* col = tile + row * kHaloY + lane;  // (x - 1, y - 1) of slice z - 1
+    constexpr int kSlice = kHaloX * kHaloY;
+    const int x = x0 + row, y = y0 + lane;
+    const bool in = x < g.SX && y < g.SY;
+    uint32_t c0 = 0, f0 = 0, d0 = 0, c1 = 0, f1 = 0, d1 = 0;
+#pragma unroll
+    for (int p = 0; p < kHaloZ; ++p) {
+        const uint32_t* q = col + p * kSlice;
+        const uint32_t c2 = q[kHaloY + 1];
+        const uint32_t f2 = max(max(q[kHaloY], q[kHaloY + 2]), max(q[1], q[2 * kHaloY + 1]));
+        const uint32_t d2 = max(max(q[0], q[2]), max(q[2 * kHaloY], q[2 * kHaloY + 2]));
+        const int z = z0 + p - 2;  // the slice between c0 and c2
+        if (p >= 2 && in && z < g.SZ) {
+            const uint32_t R = c1;
+            uint8_t f = 0;
             if (R >= nR) {  // max_edt2 below the data: refuse rather than index past the table
                 atomicOr(err, 1u);
-            } else {
-                int x, y, z;
-                g.coords(v, x, y, z);
-                f = dominated(edt2, g, x, y, z, R, mtab, ntab) ? 0 : 1;
+            } else if (R != 0) {
+                f = !contained(R, max(max(c0, c2), f1), 1, mtab, ntab) && !contained(R, max(max(f0, f2), d1), 2, mtab, ntab) &&
+                    !contained(R, max(d0, d2), 3, mtab, ntab);
             }
+            flags[g.idx(x, y, z)] = f;
         }
-        flags[v] = f;
+        c0 = c1;
+        f0 = f1;
+        d0 = d1;
+        c1 = c2;
+        f1 = f2;
+        d1 = d2;
     }
 }
 
@@ -127,9 +155,7 @@ struct Tiles {
 };
 
 // Visits the tiles whose box is within sqrt(R) of centre (x, y, z), restricted to tile
-// z-range [tz0, tz1). f(tile, full): full = the ball covers the whole tile (clipped to the
-// volume), i.e. its farthest corner - a ball is convex, so covering the eight corners of a
-// box covers every lattice point in it.
+// z-range [tz0, tz1).
 template <class F>
 __device__ __forceinline__ void for_each_tile(Grid g, Tiles t, int x, int y, int z, uint32_t R,
                                               int tz0, int tz1, F f) {
@@ -140,41 +166,74 @@ __device__ __forceinline__ void for_each_tile(Grid g, Tiles t, int x, int y, int
     for (int tz = az; tz <= bz; ++tz) {
         const int lz = tz * kTile, hz = min(lz + kTile - 1, g.SZ - 1);
         const int dz = z < lz ? lz - z : (z > hz ? z - hz : 0);
-        const int fz = max(abs(z - lz), abs(hz - z));
         for (int tx = ax; tx <= bx; ++tx) {
             const int lx = tx * kTile, hx = min(lx + kTile - 1, g.SX - 1);
             const int dx = x < lx ? lx - x : (x > hx ? x - hx : 0);
             const int dxz = dx * dx + dz * dz;
             if (static_cast<uint32_t>(dxz) > R) continue;
-            const int fx = max(abs(x - lx), abs(hx - x));
-            const int fxz = fx * fx + fz * fz;
             for (int ty = ay; ty <= by; ++ty) {
                 const int ly = ty * kTile, hy = min(ly + kTile - 1, g.SY - 1);
                 const int dy = y < ly ? ly - y : (y > hy ? y - hy : 0);
                 if (static_cast<uint32_t>(dxz + dy * dy) > R) continue;
-                const int fy = max(abs(y - ly), abs(hy - y));
-                f(t.id(tx, ty, tz), static_cast<uint32_t>(fxz + fy * fy) <= R);
+                f(t.id(tx, ty, tz));
             }
         }
     }
 }
 
-// Floor of a tile: the largest key among balls covering the whole tile. Every voxel of the
+__device__ __forceinline__ unsigned long long ball_key(Grid g, int x, int y, int z, uint32_t R) {
+    const uint32_t lex = (static_cast<uint32_t>(x) * g.SY + y) * static_cast<uint32_t>(g.SZ) + z;
+    return (static_cast<unsigned long long>(R) << 32) | (0xFFFFFFFFu - lex);
+}
+
+// Squared radii of the kept centres, counted down from the largest (a sort key, descending r^2).
+__global__ void balls_radii(const uint32_t* __restrict__ edt2, const uint32_t* __restrict__ cand, size_t nc, uint32_t max_edt2,
+                            uint32_t* __restrict__ down) {
+    PMA_GRID_STRIDE(i, nc) down[i] = max_edt2 - edt2[cand[i]];
+}
+
+// Floor of a tile: the largest key among balls covering the whole tile (those found here: balls
+// of r^2 below kFloorR2 cover no whole tile except clipped ones, and are left out). Every voxel of the
 // tile is covered by that ball, so its winner's key is at least the floor, and list entries
 // below it can be left out.
-struct FloorTile {
-    unsigned long long* floor;
-    unsigned long long key;
-    __device__ void operator()(size_t tid, bool full) const {
-        if (full) atomicMax(&floor[tid], key);
+constexpr uint32_t kFloorR2 = 37;  // half the diagonal between a tile's corner voxels: 3 * 3.5^2 = 36.75
+
+__global__ void balls_tile_floor(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
+                                 size_t nc, Grid g, Tiles t, unsigned long long* __restrict__ floor) {
+    PMA_GRID_STRIDE(i, nc) {
+        const uint32_t R = max_edt2 - down[i];
+        if (R < kFloorR2) continue;
+        int x, y, z;
+        g.coords(cand[i], x, y, z);
+        const int r = static_cast<int>(isqrt_u32(R));
+        const unsigned long long key = ball_key(g, x, y, z, R);
+        // per axis: tiles whose far voxel is within r
+        const int ax = (max(x - r, 0) + kTile - 1) / kTile, bx = min(x + r, g.SX - 1) == g.SX - 1 ? t.TX - 1 : (x + r + 1) / kTile - 1;
+        const int ay = (max(y - r, 0) + kTile - 1) / kTile, by = min(y + r, g.SY - 1) == g.SY - 1 ? t.TY - 1 : (y + r + 1) / kTile - 1;
+        const int az = (max(z - r, 0) + kTile - 1) / kTile, bz = min(z + r, g.SZ - 1) == g.SZ - 1 ? t.TZ - 1 : (z + r + 1) / kTile - 1;
+        for (int tz = az; tz <= bz; ++tz) {
+            const int fz = max(abs(z - tz * kTile), abs(min(tz * kTile + kTile, g.SZ) - 1 - z));
+            for (int tx = ax; tx <= bx; ++tx) {
+                const int fx = max(abs(x - tx * kTile), abs(min(tx * kTile + kTile, g.SX) - 1 - x));
+                const uint32_t fxz = static_cast<uint32_t>(fx * fx + fz * fz);
+                if (fxz > R) continue;
+                for (int ty = ay; ty <= by; ++ty) {
+                    const int fy = max(abs(y - ty * kTile), abs(min(ty * kTile + kTile, g.SY) - 1 - y));
+                    if (fxz + static_cast<uint32_t>(fy * fy) > R) continue;
+                    const size_t tid = t.id(tx, ty, tz);
+                    // most lose to one recorded before: a plain read (possibly old: floors only grow) first
+                    if (key > *reinterpret_cast<volatile unsigned long long*>(floor + tid)) atomicMax(&floor[tid], key);
+                }
+            }
+        }
     }
-};
+}
 
 struct CountTile {
     const unsigned long long* floor;
     unsigned int* tcount;
     unsigned long long key;
-    __device__ void operator()(size_t tid, bool) const {
+    __device__ void operator()(size_t tid) const {
         if (key >= __ldg(floor + tid)) atomicAdd(&tcount[tid], 1u);
     }
 };
@@ -186,51 +245,33 @@ struct FillTile {
     unsigned int* tcursor;
     unsigned long long* entries;
     unsigned long long key;
-    __device__ void operator()(size_t tid, bool) const {
+    __device__ void operator()(size_t tid) const {
         if (key < __ldg(floor + tid)) return;
         const unsigned pos = atomicAdd(&tcursor[tid], 1u);
         entries[toff[tid] - base + pos] = key;
     }
 };
 
-__device__ __forceinline__ unsigned long long ball_key(Grid g, int x, int y, int z, uint32_t R) {
-    const uint32_t lex = (static_cast<uint32_t>(x) * g.SY + y) * static_cast<uint32_t>(g.SZ) + z;
-    return (static_cast<unsigned long long>(R) << 32) | (0xFFFFFFFFu - lex);
-}
-
-__global__ void balls_tile_floor(const uint32_t* __restrict__ edt2, const uint32_t* __restrict__ cand,
-                                 size_t nc, Grid g, Tiles t, unsigned long long* __restrict__ floor) {
-    PMA_GRID_STRIDE(i, nc) {
-        const uint32_t v = cand[i];
-        int x, y, z;
-        g.coords(v, x, y, z);
-        const uint32_t R = edt2[v];
-        for_each_tile(g, t, x, y, z, R, 0, t.TZ, FloorTile{floor, ball_key(g, x, y, z, R)});
-    }
-}
-
-__global__ void balls_tile_count(const uint32_t* __restrict__ edt2, const uint32_t* __restrict__ cand,
+__global__ void balls_tile_count(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
                                  size_t nc, Grid g, Tiles t, const unsigned long long* __restrict__ floor,
                                  unsigned int* __restrict__ tcount) {
     PMA_GRID_STRIDE(i, nc) {
-        const uint32_t v = cand[i];
         int x, y, z;
-        g.coords(v, x, y, z);
-        const uint32_t R = edt2[v];
+        g.coords(cand[i], x, y, z);
+        const uint32_t R = max_edt2 - down[i];
         for_each_tile(g, t, x, y, z, R, 0, t.TZ, CountTile{floor, tcount, ball_key(g, x, y, z, R)});
     }
 }
 
-__global__ void balls_tile_fill(const uint32_t* __restrict__ edt2, const uint32_t* __restrict__ cand,
+__global__ void balls_tile_fill(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
                                 size_t nc, Grid g, Tiles t, int tz0, int tz1,
                                 const unsigned long long* __restrict__ floor,
                                 const unsigned long long* __restrict__ toff, unsigned long long base,
                                 unsigned int* __restrict__ tcursor, unsigned long long* __restrict__ entries) {
     PMA_GRID_STRIDE(i, nc) {
-        const uint32_t v = cand[i];
         int x, y, z;
-        g.coords(v, x, y, z);
-        const uint32_t R = edt2[v];
+        g.coords(cand[i], x, y, z);
+        const uint32_t R = max_edt2 - down[i];
         for_each_tile(g, t, x, y, z, R, tz0, tz1,
                       FillTile{floor, toff, base, tcursor, entries, ball_key(g, x, y, z, R)});
     }
@@ -262,24 +303,28 @@ __device__ __forceinline__ unsigned long long pos_key(int4 c, Grid g) {
     return (static_cast<unsigned long long>(static_cast<uint32_t>(c.w)) << 32) | (0xFFFFFFFFu - lex);
 }
 
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        v = t < v ? t : v;
-    }
-    return v;
+// Lanes of a warp's box lie at y + 4 x + 16 z: the y (x) values present in a lane mask, as 4 bits.
+__device__ __forceinline__ unsigned int fold_y(unsigned int m) {
+    m |= m >> 16;
+    m |= m >> 8;
+    m |= m >> 4;
+    return m & 15u;
+}
+__device__ __forceinline__ unsigned int fold_x(unsigned int m) {
+    m |= m >> 16;
+    return ((m & 0xFu) ? 1u : 0u) | ((m & 0xF0u) ? 2u : 0u) | ((m & 0xF00u) ? 4u : 0u) | ((m & 0xF000u) ? 8u : 0u);
 }
 
 // One CTA per tile of the z-range starting at tz0: winner key of each voxel.
 //
 // The tile's list is taken in chunks of up to kListCap entries. Each chunk is decoded into
 // shared memory ordered by radius, largest first (a counting sort on r^2 when the chunk's r^2
-// span fits kSortBins, else left in list order). A warp covers a 1 x 4 x 8 box of voxels and
+// span fits kSortBins, else left in list order). A warp covers a 2 x 4 x 4 box of voxels and
 // keeps, per lane, the largest covering key so far (best). It reads the chunk 32 entries at a
-// time: an entry can matter only if its ball reaches the warp's box and its key exceeds the
-// smallest best of the warp's lanes; the lanes test every such entry against their own voxel.
-// In a chunk sorted by radius the warp stops once the next entry's r^2 is below the smallest
-// best's r^2 (every later entry's key is smaller). The result is the largest covering key over
+// time: an entry can matter only if its ball reaches the box of the lanes whose best is not above
+// the radii still to come; the lanes test every such entry against their own voxel.
+// In a chunk sorted by radius the warp stops once no lane is left whose best has an r^2 of at most
+// the next entry's (every later entry's key is smaller). The result is the largest covering key over
 // the whole list, i.e. the covering centre of largest key.
 constexpr int kSortBins = 2048;
 
@@ -297,15 +342,12 @@ __global__ void __launch_bounds__(kTileVox, 3) balls_tile_gather(
     const int tx = static_cast<int>(rest % t.TX);
     const int tz = static_cast<int>(rest / t.TX);
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // voxel of this thread: y fastest, then x, then z (a warp covers a 1 x 4 x 8 box)
-    const int vy = ty * kTile + (threadIdx.x & 7);
-    const int vx = tx * kTile + ((threadIdx.x >> 3) & 7);
-    const int vz = tz * kTile + (threadIdx.x >> 6);
+    // a warp covers a box of 2 x 4 x 4 voxels (z, x, y)
+    const int by0 = ty * kTile + (warp & 1) * 4, bx0 = tx * kTile + ((warp >> 1) & 1) * 4, bz0 = tz * kTile + (warp >> 2) * 2;
+    const int vy = by0 + (lane & 3), vx = bx0 + ((lane >> 2) & 3), vz = bz0 + (lane >> 4);
     const bool inside = vx < g.SX && vy < g.SY && vz < g.SZ;
     const size_t v = inside ? g.idx(vx, vy, vz) : 0;
     const bool void_voxel = inside && edt2[v] != 0;
-    // the warp's box
-    const int bx0 = tx * kTile + (warp & 1) * 4, by0 = ty * kTile, bz = vz;
     const unsigned int L = tcount[tile];
     const unsigned long long* list = entries + (toff[tile] - base);
     unsigned long long best = void_voxel ? 0ull : ~0ull;
@@ -338,6 +380,7 @@ __global__ void __launch_bounds__(kTileVox, 3) balls_tile_gather(
         }
         __syncthreads();
         const unsigned int r_hi = s_rmax;
+        if (!__syncthreads_or(static_cast<uint32_t>(best >> 32) <= r_hi)) continue;  // no voxel of the block can gain
         const bool sorted = r_hi - s_rmin < static_cast<unsigned int>(kSortBins);
         unsigned int rank[kPer];
         if (sorted) {  // counting sort, descending r^2: bin = r_hi - r^2
@@ -394,28 +437,40 @@ __global__ void __launch_bounds__(kTileVox, 3) balls_tile_gather(
             }
         }
         __syncthreads();
-        // the warp's pass over the chunk
+        // the warp's pass over the chunk; open: lanes whose best may still be beaten, in the box
+        // [lo, hi] of which a ball has to reach
+        unsigned int open = 0;
+        int lox = 0, loy = 0, loz = 0, hix = 0, hiy = 0, hiz = 0;
         for (unsigned int e0 = 0; e0 < m; e0 += 32) {
-            const unsigned long long mb = warp_min_u64(best);
-            if (mb == ~0ull) break;  // no void voxel left to improve
-            if (sorted && static_cast<uint32_t>(s_pos[e0].w) < static_cast<uint32_t>(mb >> 32)) break;
+            const uint32_t most = sorted ? static_cast<uint32_t>(s_pos[e0].w) : r_hi;  // r^2 from here on
+            const unsigned int now = __ballot_sync(0xFFFFFFFFu, static_cast<uint32_t>(best >> 32) <= most);
+            if (!now) break;
+            if (now != open) {
+                open = now;
+                const unsigned int y4 = fold_y(now), x4 = fold_x(now);
+                loy = by0 + __ffs(y4) - 1;
+                hiy = by0 + 31 - __clz(y4);
+                lox = bx0 + __ffs(x4) - 1;
+                hix = bx0 + 31 - __clz(x4);
+                loz = bz0 + ((now & 0xFFFFu) ? 0 : 1);
+                hiz = bz0 + ((now >> 16) ? 1 : 0);
+            }
             bool cand = false;
             if (e0 + lane < m) {
                 const int4 c = s_pos[e0 + lane];
-                if (pos_key(c, g) > mb) {  // can beat some lane; does the ball reach the box?
-                    const int dx = c.x < bx0 ? bx0 - c.x : (c.x > bx0 + 3 ? c.x - bx0 - 3 : 0);
-                    const int dy = c.y < by0 ? by0 - c.y : (c.y > by0 + 7 ? c.y - by0 - 7 : 0);
-                    const int dz = c.z < bz ? bz - c.z : (c.z > bz ? c.z - bz : 0);
-                    cand = covers(make_int4(dx, dy, dz, c.w), 0, 0, 0);
-                }
+                const int dx = max(max(lox - c.x, c.x - hix), 0), dy = max(max(loy - c.y, c.y - hiy), 0),
+                          dz = max(max(loz - c.z, c.z - hiz), 0);
+                cand = covers(make_int4(dx, dy, dz, c.w), 0, 0, 0);
             }
             unsigned int mask = __ballot_sync(0xFFFFFFFFu, cand);
             while (mask) {
                 const int b = __ffs(mask) - 1;
                 mask &= mask - 1;
                 const int4 c = s_pos[e0 + b];
-                const unsigned long long kc = pos_key(c, g);
-                if (kc > best && void_voxel && covers(c, vx, vy, vz)) best = kc;
+                if (covers(c, vx, vy, vz)) {
+                    const unsigned long long kc = pos_key(c, g);
+                    if (kc > best) best = kc;  // never where best is ~0: solid or outside
+                }
             }
         }
         if (c0 + kListCap < L) __syncthreads();  // before the next chunk replaces s_pos
@@ -521,7 +576,9 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
     int64_t nc = 0;
     {
         KernelTimer kt(ctx, "balls_candidates");
-        balls_candidate_flags<<<G, 256, 0, s>>>(edt2, g, n, mtab, ntab, nR, flags, err);
+        const unsigned BY = div_up(d.sy, kBrickY), BX = div_up(d.sx, kBrickX), BZ = div_up(d.sz, kBrickZ);
+        balls_candidate_flags<<<BY * BX * BZ, 32 * kBrickX, 0, s>>>(edt2, g, static_cast<int>(BY), static_cast<int>(BX), mtab,
+                                                                   ntab, nR, flags, err);
         ctx->check_launch("balls_candidate_flags");
         nc = select_flagged(ctx, thrust::counting_iterator<uint32_t>(0), flags, cand,
                             static_cast<int64_t>(n), reinterpret_cast<int64_t*>(misc + 2));
@@ -532,6 +589,26 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
     PMA_REQUIRE(!(h_err & 1u), PMA_ERR_ARGUMENT,
                 "pma_containing_balls: max_edt2 is smaller than the largest squared distance");
 
+    // Large volumes take the kept centres by descending radius: the lanes of a warp then visit equally
+    // many tiles, floors rise early, and the tile lists come out nearly ordered, so that a gather's
+    // later chunks hold smaller balls and are mostly skipped. Below kSortCentres the sort's launches cost
+    // more than it saves.
+    constexpr int64_t kSortCentres = 1 << 18;
+    uint32_t* down = buf<uint32_t>(ctx, "balls.down", nc);
+    if (nc) {
+        balls_radii<<<grid_for(ctx, nc), 256, 0, s>>>(edt2, cand, nc, max_edt2, down);
+        ctx->check_launch("balls_radii");
+        if (nc >= kSortCentres) {
+            KernelTimer kt(ctx, "balls_sort");
+            int bits = 1;
+            while (bits < 32 && (max_edt2 >> bits) != 0) ++bits;
+            uint32_t* down2 = buf<uint32_t>(ctx, "balls.down2", nc);
+            uint32_t* cand2 = buf<uint32_t>(ctx, "balls.cand2", nc);
+            sort_pairs(ctx, down, down2, cand, cand2, nc, bits);
+            down = down2;
+            cand = cand2;
+        }
+    }
     // Tile lists: counts, 64-bit offsets (host scan), then fill + gather by tile z-ranges
     // whose entries fit the memory budget.
     Tiles t{(d.sx + kTile - 1) / kTile, (d.sy + kTile - 1) / kTile, (d.sz + kTile - 1) / kTile};
@@ -546,9 +623,9 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
     PMA_CUDA(cudaMemsetAsync(floor, 0, ntiles * 8, s));
     if (nc) {
         KernelTimer kt(ctx, "balls_tile_count");
-        balls_tile_floor<<<grid_for(ctx, nc), 256, 0, s>>>(edt2, cand, nc, g, t, floor);
+        balls_tile_floor<<<grid_for(ctx, nc), 256, 0, s>>>(cand, down, max_edt2, nc, g, t, floor);
         ctx->check_launch("balls_tile_floor");
-        balls_tile_count<<<grid_for(ctx, nc), 256, 0, s>>>(edt2, cand, nc, g, t, floor, tcount);
+        balls_tile_count<<<grid_for(ctx, nc), 256, 0, s>>>(cand, down, max_edt2, nc, g, t, floor, tcount);
         ctx->check_launch("balls_tile_count");
     }
     // 64-bit list offsets by a device scan; the host reads back only the offsets at the tile
@@ -576,7 +653,7 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
         auto* entries = buf<unsigned long long>(ctx, "balls.entries", cnt);
         if (nc) {
             KernelTimer kt(ctx, "balls_tile_fill");
-            balls_tile_fill<<<grid_for(ctx, nc), 256, 0, s>>>(edt2, cand, nc, g, t, z0, z1, floor, toff,
+            balls_tile_fill<<<grid_for(ctx, nc), 256, 0, s>>>(cand, down, max_edt2, nc, g, t, z0, z1, floor, toff,
                                                               base, tcursor, entries);
             ctx->check_launch("balls_tile_fill");
         }
