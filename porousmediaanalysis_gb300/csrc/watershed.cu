@@ -56,7 +56,6 @@ constexpr int kSlots = 6;         // extending pores per record; a voxel chains 
 constexpr int kMaxExt = 26;       // extending pores of one voxel at most (26 neighbours touch it)
 constexpr int kMaxHops = (kMaxExt + kSlots - 1) / kSlots;  // records in one voxel's chain
 constexpr int kKeyMax = kMaxExt + 1;  // longest key: the claimer and every extending pore
-constexpr int kChunk = 1024;      // event slots per compaction block
 constexpr int kGensPerLaunch = 64;  // generations per cooperative launch (host checks between)
 constexpr unsigned long long kMaxGen = 1ull << 23;              // generations per call
 constexpr unsigned long long kSeqMask = (1ull << 40) - 1;       // touch time within a generation
@@ -84,10 +83,10 @@ struct WsState {
     unsigned int* err;
     int spin_limit;               // polls of one wait on another block before giving up
     unsigned long long* gen_hist; // NULL, or per log2 of the frontier size: [c] generations,
-                                  // [64 + c] ns in claim phases, [128 + c] ns in resolve phases;
-                                  // [192], [193]: block 0's ns resolving events, scan + look-back
+                                  // [64 + c] ns in claim phases, [128 + c] ns in resolve phases
     int time_shift;               // bucket entry time = (generation << time_shift) | event
-    uint8_t* ev_touch;            // per event slot: phase 0 touched an unclaimed voxel
+    uint32_t* touched;            // a bit per event: its claim phase touched an unclaimed voxel
+    uint32_t* won;                // a bit per event: it gives a node of the next generation
     unsigned long long* bpos;        // per depth: where its bucket's next entry goes
     unsigned long long* ent_time;
     unsigned long long* ent_val;
@@ -101,18 +100,6 @@ __host__ __device__ __forceinline__ unsigned long long ws_word(int packed, unsig
 __device__ __forceinline__ uint32_t ws_claimer(int packed, unsigned long long word) {
     const unsigned long long st = packed ? word >> 16 : word;
     return st < kTouched ? static_cast<uint32_t>(st) : 0u;
-}
-
-// The radius and claim state of voxel w (one load when packed).
-__device__ __forceinline__ void ws_load(const WsState& s, size_t w, uint32_t& r, unsigned long long& st) {
-    const unsigned long long word = __ldcg(s.state + w);
-    if (s.packed) {
-        r = static_cast<uint32_t>(word & 0xFFFFu);
-        st = word >> 16;
-    } else {
-        r = __ldg(s.crad + w);
-        st = word;
-    }
 }
 
 __global__ void ws_init(size_t n, const uint32_t* __restrict__ crad, int packed,
@@ -211,6 +198,14 @@ __device__ __forceinline__ uint32_t ws_follow(uint32_t* link, const WsState& s) 
     return rec;
 }
 
+// A touch that waits for a record number that nothing writes: the wait runs out after spin_limit polls
+// and sets bit 8, the path of a stalled allocation.
+__global__ void ws_wait_selftest(WsState s, uint32_t* link) {
+    if (threadIdx.x != 0) return;
+    *reinterpret_cast<volatile uint32_t*>(link) = kRecBusy;
+    ws_follow(link, s);
+}
+
 // Records that `pore` touched shared voxel w at time t (its first touch per pore is kept).
 // Out of line: it is the rare path of the touch kernel. Slots fill in order along the
 // voxel's record chain, so two touches by one pore meet at the same slot.
@@ -261,62 +256,11 @@ __global__ void ws_record_extensions(WsState s, uint32_t begin, uint32_t end) {
     }
 }
 
-// The neighbour of v at an offset that stays inside the volume (indices fit 32 bits).
-__device__ __forceinline__ uint32_t ws_neighbour(const WsState& s, uint32_t v, int dx, int dy, int dz) {
-    return v + (static_cast<uint32_t>(dz) * s.g.SX + dx) * s.g.SY + dy;  // modulo 2^32
-}
-
-// Touch events of the generation's nodes. Phase 0 claims: the smallest touch time of each
-// unclaimed voxel wins (atomicMin on its state word). A touch of a voxel claimed in an
-// earlier generation is final in phase 0 already: it is an extension when the toucher is not the owner (claims
-// never change, and extensions keep each pore's smallest time, so the order of recording
-// does not matter). Phase 0 flags, per event, a touch of an unclaimed voxel; phase 1 resolves
-// only those: the winner records its claim, and every other touch by a pore other than the
-// winner's is an extension.
-// One thread per event (node i, stencil position j): seq = i * 27 + j.
-// All generations of a launch run in one kernel (see ws_generations), so data written by
-// other blocks earlier in the launch is read with __ldcg (L2, not a possibly stale L1 line);
-// only the radii, which never change, go through the read-only path.
-__device__ __forceinline__ void ws_claim_event(const WsState& s, const uint32_t* gv, const uint32_t* gp,
-                                               unsigned long long seq, uint32_t depth, unsigned long long gen) {
-    const unsigned long long i = seq / 27;
-    const int j = static_cast<int>(seq - i * 27);
-    uint8_t touched = 0;
-    int dx, dy, dz;
-    if (stencil_offset(j, s.d3q7, dx, dy, dz)) {
-        const uint32_t v = __ldcg(gv + i);
-        const uint32_t node = __ldcg(gp + i), pore = node & ~kFace;
-        bool inside = true;
-        if (node & kFace) {
-            int x, y, z;
-            s.g.coords(v, x, y, z);
-            inside = s.g.inside(x + dx, y + dy, z + dz);
-        }
-        if (!inside) {  // WC.cpp:140-144
-            s.pbound[pore] = 1;
-        } else {
-            const uint32_t w = ws_neighbour(s, v, dx, dy, dz);
-            uint32_t r;
-            unsigned long long st;
-            ws_load(s, w, r, st);
-            if (r != 0 && r <= depth) {  // WC.cpp:152-156
-                if (st >= kTouched) {
-                    atomicMin(&s.state[w], ws_word(s.packed, kTouched | seq, r));
-                    touched = 1;
-                } else if (st - 1 != pore) {
-                    ws_note(s, w, pore, (gen << 40) | seq);
-                }
-            }
-        }
-    }
-    s.ev_touch[seq] = touched;
-}
-
-// Appends the claim of voxel w (radius r, below the running depth) to its depth's bucket. Lanes
-// appending to the same depth take their slots with one atomic: a generation's claims of
+// Appends a claim (entry time, pore << 32 | voxel of radius r, below the running depth) to its
+// depth's bucket. Lanes appending to the same depth take their slots with one atomic: a generation's claims of
 // shallower voxels mostly go to a few depths, and one counter per depth would serialise them.
-__device__ __forceinline__ void ws_append(const WsState& s, unsigned lanes, uint32_t w, uint32_t pore, uint32_t r,
-                                          unsigned long long seq, unsigned long long gen) {
+__device__ __forceinline__ void ws_append_entry(const WsState& s, unsigned lanes, uint32_t r, unsigned long long time,
+                                                unsigned long long val) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned peers = __match_any_sync(lanes, r);
     const int leader = __ffs(peers) - 1;
@@ -324,177 +268,8 @@ __device__ __forceinline__ void ws_append(const WsState& s, unsigned lanes, uint
     if (static_cast<int>(lane) == leader) first = atomicAdd(&s.bpos[r], static_cast<unsigned long long>(__popc(peers)));
     first = __shfl_sync(peers, first, leader);
     const unsigned long long at = first + __popc(peers & ((1u << lane) - 1u));
-    s.ent_time[at] = (gen << s.time_shift) | seq;
-    s.ent_val[at] = (static_cast<unsigned long long>(pore) << 32) | w;
-}
-
-// Resolves event seq if it touched an unclaimed voxel: the winner records its claim, every other
-// touch by a pore other than the winner's is an extension. Returns true when the event claims a
-// voxel of the same depth (a node of the next generation).
-__device__ __forceinline__ bool ws_resolve_event(const WsState& s, const uint32_t* gv, const uint32_t* gp,
-                                                 unsigned long long seq, uint32_t depth, unsigned long long gen) {
-    const unsigned long long i = seq / 27;
-    const int j = static_cast<int>(seq - i * 27);
-    // the node (shared by the event's warp neighbours) is loaded along with the flag
-    const uint8_t touched = __ldcg(s.ev_touch + seq);
-    const uint32_t v = __ldcg(gv + i);
-    const uint32_t pore = __ldcg(gp + i) & ~kFace;
-    if (!touched) return false;
-    int dx, dy, dz;
-    stencil_offset(j, s.d3q7, dx, dy, dz);
-    // the neighbour is inside the box (phase 0 touched it)
-    const uint32_t nw = ws_neighbour(s, v, dx, dy, dz);
-    uint32_t r;
-    unsigned long long st;
-    ws_load(s, nw, r, st);
-    if (st == (kTouched | seq)) {  // the winner
-        s.state[nw] = ws_word(s.packed, pore + 1, r);  // one 64-bit store: readers see either word
-        if (r == depth) return true;
-        ws_append(s, __activemask(), nw, pore, r, seq, gen);
-        return false;
-    }
-    // the winner's pore: already stored as the claimer, or that of the winning touch's node
-    const uint32_t owner = st < kTouched ? static_cast<uint32_t>(st - 1) : __ldcg(gp + (st & kSeqMask) / 27) & ~kFace;
-    if (owner != pore) ws_note(s, nw, pore, (gen << 40) | seq);
-    return false;
-}
-
-// Writes the node that event seq gave.
-__device__ __forceinline__ void ws_put_node(const WsState& s, const uint32_t* gv, const uint32_t* gp,
-                                            unsigned long long seq, uint32_t* v_out, uint32_t* p_out) {
-    const unsigned long long i = seq / 27;
-    int dx, dy, dz;
-    stencil_offset(static_cast<int>(seq - i * 27), s.d3q7, dx, dy, dz);
-    const uint32_t w = ws_neighbour(s, __ldcg(gv + i), dx, dy, dz);
-    *v_out = w;
-    *p_out = ws_node(s.g, w, __ldcg(gp + i) & ~kFace);
-}
-
-// Ordered compaction of a generation's same-depth claims into the next frontier, in event
-// order, inside the resolve phase: each chunk of kChunk events (one block, four per thread)
-// ranks its claims, and its offset comes from a decoupled look-back over the chunks before it,
-// read 256 descriptors at a time by one warp. A descriptor holds (generation << 40) | state << 38
-// | count, state 1 = the chunk's own count, 2 = the inclusive prefix; one of an older
-// generation is not yet published. Chunks publish their own count before looking back and
-// every block of the cooperative grid is resident, so the look-back always ends; it is bounded
-// all the same (err bit 16). A generation thus needs two grid-wide barriers (after the claims,
-// after the resolved frontier) instead of four for a separate count, scan and scatter.
-// (Measured at 1024^3: 894 ms per step, against 910-950 ms with the count / scan / scatter
-// form for generations of more than 256 chunks, and 1108 ms with a look-back that read one
-// descriptor at a time.)
-constexpr unsigned long long kDescOwn = 1ull << 38;
-constexpr unsigned long long kDescIncl = 2ull << 38;
-constexpr unsigned long long kDescVal = (1ull << 38) - 1;
-
-// Called by all 32 lanes of one warp; returns the exclusive prefix of chunk c, reading 32
-// descriptors a poll. Used where chunks are dealt round-robin: its light polling leaves the L2 to
-// the blocks still resolving (a 256-wide poll made single-round generations 10-40 % slower).
-__device__ unsigned long long ws_lookback32(unsigned long long* desc, unsigned long long c, unsigned long long gen,
-                                          unsigned long long own, unsigned int* err, int spin_limit,
-                                          unsigned lane) {
-    volatile unsigned long long* vd = desc;
-    const unsigned long long tg = gen << 40;
-    if (lane == 0) vd[c] = tg | (c == 0 ? kDescIncl : kDescOwn) | own;
-    if (c == 0) return 0;
-    __threadfence();
-    unsigned long long excl = 0;
-    long long top = static_cast<long long>(c) - 1;
-    int spins = 0;
-    while (true) {
-        const long long p = top - static_cast<long long>(lane);
-        const bool valid = p >= 0;
-        const unsigned long long d = valid ? vd[p] : 0ull;
-        const bool ready = !valid || (d >> 40) == gen;
-        if (!__all_sync(0xFFFFFFFFu, ready)) {  // a predecessor has not published yet
-            if (++spins > spin_limit) {
-                if (lane == 0) atomicOr(err, 16u);
-                break;
-            }
-            continue;
-        }
-        // the nearest inclusive prefix ends the walk; owns before it are added
-        const unsigned incl = __ballot_sync(0xFFFFFFFFu, valid && (d & kDescIncl) != 0);
-        const int stop = incl ? __ffs(incl) - 1 : 31;
-        unsigned long long v = (valid && static_cast<int>(lane) <= stop) ? (d & kDescVal) : 0ull;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        excl += v;
-        if (incl || top < 32) break;  // chunk 0 is always inclusive
-        top -= 32;
-    }
-    if (lane == 0) {
-        __threadfence();
-        vd[c] = tg | kDescIncl | (excl + own);
-    }
-    return excl;
-}
-
-// Called by all 32 lanes of one warp; returns the exclusive prefix of range c. Each poll reads
-// kLookbackPer descriptors per lane (256 ranges, nearest first) and needs them published only
-// up to the nearest inclusive prefix, so a range far from its last inclusive predecessor
-// reaches it in a few polls instead of one per 32. Used once per block and generation by the
-// contiguous-range compaction.
-constexpr int kLookbackPer = 8;
-__device__ unsigned long long ws_lookback(unsigned long long* desc, unsigned long long c, unsigned long long gen,
-                                          unsigned long long own, unsigned int* err, int spin_limit,
-                                          unsigned lane) {
-    volatile unsigned long long* vd = desc;
-    const unsigned long long tg = gen << 40;
-    if (lane == 0) vd[c] = tg | (c == 0 ? kDescIncl : kDescOwn) | own;
-    if (c == 0) return 0;
-    __threadfence();
-    unsigned long long excl = 0;
-    long long top = static_cast<long long>(c) - 1;
-    int spins = 0;
-    while (true) {
-        // lane l holds chunks top - l * kLookbackPer - j; before chunk 0 reads as an inclusive
-        // zero (chunk 0 is always inclusive, so the walk stops there anyway)
-        unsigned long long d[kLookbackPer];
-#pragma unroll
-        for (int j = 0; j < kLookbackPer; ++j) {
-            const long long p = top - static_cast<long long>(lane) * kLookbackPer - j;
-            d[j] = p >= 0 ? vd[p] : (tg | kDescIncl);
-        }
-        int fi = kLookbackPer, fn = kLookbackPer;  // this lane's first inclusive / first unpublished
-#pragma unroll
-        for (int j = kLookbackPer - 1; j >= 0; --j) {
-            if ((d[j] >> 40) != gen) fn = j;
-            else if (d[j] & kDescIncl) fi = j;
-        }
-        const unsigned incl = __ballot_sync(0xFFFFFFFFu, fi < fn);
-        const unsigned gap = __ballot_sync(0xFFFFFFFFu, fn < fi);
-        const unsigned any = incl | gap;
-        const int stop = any ? __ffs(any) - 1 : 32;  // the lane that decides this poll
-        if (stop < 32 && ((gap >> stop) & 1u)) {     // a predecessor before the inclusive is unpublished
-            if (++spins > spin_limit) {
-                if (lane == 0) atomicOr(err, 16u);
-                break;
-            }
-            continue;
-        }
-        const int upto = static_cast<int>(lane) < stop ? kLookbackPer : (static_cast<int>(lane) == stop ? fi + 1 : 0);
-        unsigned long long v = 0;
-#pragma unroll
-        for (int j = 0; j < kLookbackPer; ++j)
-            if (j < upto) v += d[j] & kDescVal;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        excl += v;
-        if (stop < 32) break;
-        top -= 32 * kLookbackPer;
-    }
-    if (lane == 0) {
-        __threadfence();
-        vd[c] = tg | kDescIncl | (excl + own);
-    }
-    return excl;
-}
-
-// A look-back at a chunk descriptor that nothing publishes (chunk 0 of generation 0 while
-// chunk 1 of generation 1 waits for it): each bounded wait of the frontier compaction (the
-// 32-wide one in err[0], the 256-wide one in err[1]) runs out after spin_limit polls and sets
-// bit 16, the path a stalled generation would take.
-__global__ void ws_wait_selftest(unsigned long long* desc, unsigned int* err, int spin_limit) {
-    ws_lookback32(desc, 1, 1, 0, err, spin_limit, threadIdx.x & 31);
-    ws_lookback(desc, 1, 1, 0, err + 1, spin_limit, threadIdx.x & 31);
+    s.ent_time[at] = time;
+    s.ent_val[at] = val;
 }
 
 __device__ __forceinline__ unsigned long long ws_clock() {  // ns
@@ -503,21 +278,285 @@ __device__ __forceinline__ unsigned long long ws_clock() {  // ns
     return t;
 }
 
-// Up to max_gens generations of one depth in a single cooperative launch, two grid-wide
+// Touch events of a generation's nodes, one per node i and stencil position j: seq = i * 27 + j. The
+// claim phase lets the smallest touch time of each unclaimed voxel win (atomicMin on its state
+// word) and sets the event's bit in `touched`. A touch of a voxel claimed in an earlier
+// generation is final there already: it is an extension when the toucher is not the owner (claims
+// never change, and extensions keep each pore's smallest time, so the order of recording does
+// not matter). The resolve phase takes the touched events only: the winner records its claim, every
+// other touch by a pore other than the winner's is an extension.
+//
+// A warp takes strips of events, kStrip a lane (one in generations that the grid covers at once): the
+// strip's nodes and touch bits are read one strip ahead, a lane's state words are loaded
+// together, and extensions and claims of shallower voxels gather in lists of the warp, which go to the log and
+// the buckets about a hundred at a time. No block barrier comes between strips. All generations of a launch run in
+// one kernel, so data written by other blocks earlier in the launch is read with __ldcg (L2, not a possibly
+// stale L1 line); only the radii, which never change, go through the read-only path.
+// What bounds a generation: below 2^14 nodes the three grid barriers (about 2 us each with 608 blocks)
+// and the chain of dependent loads between them, above it instructions and the latency of
+// the scattered state words (40 % of the issue slots, L2 at 11 %). Generations of 2^13 / 2^17 / 2^20 nodes, us:
+// one event a thread with a node load, a state load and an answered atomic one after the other
+// 17 / 147 / 780, now 18 / 94 / 580; stage of a 640 x 600 x 672 spinodal 315 -> 288 ms, of a 512^3
+// field 146 -> 123 ms. (Chunks of 1024 events a block with a block barrier each: the same within 2 %.)
+constexpr int kGenThreads = 256;
+constexpr int kGenWarps = kGenThreads / 32;
+constexpr int kStrip = 2;             // events a lane of a strip
+constexpr unsigned kGenList = 128;    // entries of a warp's lists
+
+struct WsGenShared {
+    uint32_t delta[27];                 // index step of a stencil position
+    unsigned int count[kGenWarps], base[kGenWarps];
+    ulonglong2 ext[kGenWarps][kGenList];                                            // as in the log
+    unsigned long long up_time[kGenWarps][kGenList], up_val[kGenWarps][kGenList];  // as in a bucket
+    uint32_t up_r[kGenWarps][kGenList];
+};
+
+struct WsLists {  // lengths of the warp's lists
+    unsigned ext, up;
+};
+
+__device__ __noinline__ void ws_flush_ext(const WsState& s, WsGenShared& sh, unsigned n) {
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(s.log_n, static_cast<unsigned long long>(n));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    __syncwarp();
+    for (unsigned i = lane; i < n; i += 32) {
+        const ulonglong2 e = sh.ext[warp][i];
+        if (base + i < s.log_cap) s.log[base + i] = e;
+        else ws_extend(s, static_cast<uint32_t>(e.y), static_cast<uint32_t>(e.y >> 32), e.x);  // log full
+    }
+    __syncwarp();
+}
+
+__device__ __noinline__ void ws_flush_up(const WsState& s, WsGenShared& sh, unsigned n) {
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncwarp();
+    for (unsigned i0 = 0; i0 < n; i0 += 32) {
+        const unsigned lanes = n - i0 >= 32 ? 0xFFFFFFFFu : (1u << (n - i0)) - 1u;
+        if (lane < n - i0) ws_append_entry(s, lanes, sh.up_r[warp][i0 + lane], sh.up_time[warp][i0 + lane], sh.up_val[warp][i0 + lane]);
+    }
+    __syncwarp();
+}
+
+// All 32 lanes call; ext = this lane has an extending touch.
+__device__ __forceinline__ void ws_list_ext(const WsState& s, WsGenShared& sh, WsLists& l, bool ext, uint32_t w, uint32_t pore,
+                                            unsigned long long t) {
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, ext);
+    if (!m) return;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (l.ext > kGenList - 32) {
+        ws_flush_ext(s, sh, l.ext);
+        l.ext = 0;
+    }
+    if (ext) sh.ext[warp][l.ext + __popc(m & ((1u << lane) - 1u))] = make_ulonglong2(t, (static_cast<unsigned long long>(pore) << 32) | w);
+    l.ext += __popc(m);
+}
+
+__device__ __forceinline__ void ws_list_up(const WsState& s, WsGenShared& sh, WsLists& l, bool up, uint32_t w, uint32_t pore,
+                                           uint32_t r, unsigned long long time) {
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, up);
+    if (!m) return;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (l.up > kGenList - 32) {
+        ws_flush_up(s, sh, l.up);
+        l.up = 0;
+    }
+    if (up) {
+        const unsigned at = l.up + __popc(m & ((1u << lane) - 1u));
+        sh.up_time[warp][at] = time;
+        sh.up_val[warp][at] = (static_cast<unsigned long long>(pore) << 32) | w;
+        sh.up_r[warp][at] = r;
+    }
+    l.up += __popc(m);
+}
+
+// A strip of PER * 32 events: its first event, that event's node and how many events of that node come before.
+struct WsStrip {
+    unsigned long long e0, first;
+    uint32_t skip, n;  // n: events of the strip
+};
+
+template <int PER>
+__device__ __forceinline__ WsStrip ws_strip(unsigned long long c, unsigned long long nev) {
+    WsStrip k;
+    k.e0 = c * (PER * 32);
+    k.first = k.e0 / 27;
+    k.skip = static_cast<uint32_t>(k.e0 - k.first * 27);
+    k.n = static_cast<uint32_t>(min(nev - k.e0, static_cast<unsigned long long>(PER * 32)));
+    return k;
+}
+
+// Lane i: the strip's i-th node (at most six); lane k: the touch bits of the strip's k-th 32 events.
+struct WsAhead {
+    uint32_t v, p, touched;
+};
+
+template <int PER>
+__device__ __forceinline__ WsAhead ws_fetch(const WsState& s, const WsStrip& k, const uint32_t* gv, const uint32_t* gp, bool touched) {
+    const unsigned lane = threadIdx.x & 31;
+    WsAhead a{0, 0, 0};
+    if (lane < (k.skip + k.n + 26) / 27) {
+        a.v = __ldcg(gv + k.first + lane);
+        a.p = __ldcg(gp + k.first + lane);
+    }
+    if (touched && lane < PER) a.touched = __ldcg(s.touched + (k.e0 >> 5) + lane);
+    return a;
+}
+
+template <int PER>
+__device__ __forceinline__ void ws_claim_strip(const WsState& s, WsGenShared& sh, WsLists& l, const WsStrip& ck, const WsAhead& a,
+                                               uint32_t depth, unsigned long long gen) {
+    const unsigned lane = threadIdx.x & 31;
+    unsigned long long word[PER];
+    uint32_t w[PER], pore[PER], rad[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const uint32_t e = k * 32 + lane, i = (ck.skip + e) / 27;
+        const int j = static_cast<int>(ck.skip + e - i * 27);
+        const uint32_t v = __shfl_sync(0xFFFFFFFFu, a.v, i), node = __shfl_sync(0xFFFFFFFFu, a.p, i);
+        bool live = e < ck.n && j != 13;
+        int dx, dy, dz;
+        if (s.d3q7) live = live && stencil_offset(j, 1, dx, dy, dz);
+        pore[k] = node & ~kFace;
+        w[k] = v + sh.delta[j];
+        if (live && (node & kFace)) {
+            int x, y, z;
+            s.g.coords(v, x, y, z);
+            stencil_offset(j, 0, dx, dy, dz);
+            if (!s.g.inside(x + dx, y + dy, z + dz)) {  // WC.cpp:140-144
+                s.pbound[pore[k]] = 1;
+                live = false;
+            }
+        }
+        word[k] = 0;  // radius 0
+        rad[k] = 0;
+        if (live) {
+            word[k] = __ldcg(s.state + w[k]);
+            if (!s.packed) rad[k] = __ldg(s.crad + w[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const unsigned long long seq = ck.e0 + k * 32 + lane;
+        const uint32_t r = s.packed ? static_cast<uint32_t>(word[k] & 0xFFFFu) : rad[k];
+        const unsigned long long st = s.packed ? word[k] >> 16 : word[k];
+        const bool in = r != 0 && r <= depth, open = in && st >= kTouched;  // WC.cpp:152-156
+        if (open) atomicMin(&s.state[w[k]], ws_word(s.packed, kTouched | seq, r));
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, open);
+        if (lane == 0) s.touched[(ck.e0 >> 5) + k] = m;
+        ws_list_ext(s, sh, l, in && !open && st - 1 != pore[k], w[k], pore[k], (gen << 40) | seq);
+    }
+}
+
+// Returns the strip's claims of this depth.
+template <int PER>
+__device__ __forceinline__ unsigned ws_resolve_strip(const WsState& s, WsGenShared& sh, WsLists& l, const WsStrip& ck, const WsAhead& a,
+                                                     const uint32_t* gp, uint32_t depth, unsigned long long gen) {
+    const unsigned lane = threadIdx.x & 31;
+    unsigned count = 0;
+    unsigned long long word[PER];
+    uint32_t w[PER], pore[PER], rad[PER], owner[PER], hits = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const uint32_t e = k * 32 + lane, i = (ck.skip + e) / 27;
+        hits |= (__shfl_sync(0xFFFFFFFFu, a.touched, k) >> lane & 1u) << k;
+        pore[k] = __shfl_sync(0xFFFFFFFFu, a.p, i) & ~kFace;
+        w[k] = __shfl_sync(0xFFFFFFFFu, a.v, i) + sh.delta[ck.skip + e - i * 27];
+        word[k] = 0;
+        rad[k] = 0;
+        if ((hits >> k) & 1u) {
+            word[k] = __ldcg(s.state + w[k]);
+            if (!s.packed) rad[k] = __ldg(s.crad + w[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const unsigned long long seq = ck.e0 + k * 32 + lane;
+        const uint32_t r = s.packed ? static_cast<uint32_t>(word[k] & 0xFFFFu) : rad[k];
+        const unsigned long long st = s.packed ? word[k] >> 16 : word[k];
+        const bool hit = (hits >> k) & 1u, win = hit && st == (kTouched | seq);
+        owner[k] = pore[k];
+        if (win) s.state[w[k]] = ws_word(s.packed, pore[k] + 1, r);  // one 64-bit store: readers see either word
+        else if (hit)  // the winner's pore: stored as the claimer already, or that of the winning touch's node
+            owner[k] = st < kTouched ? static_cast<uint32_t>(st - 1) : __ldcg(gp + (st & kSeqMask) / 27) & ~kFace;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, win && r == depth);
+        if (lane == 0) s.won[(ck.e0 >> 5) + k] = m;
+        count += __popc(m);
+        ws_list_up(s, sh, l, win && r != depth, w[k], pore[k], r, (gen << s.time_shift) | seq);
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) ws_list_ext(s, sh, l, owner[k] != pore[k], w[k], pore[k], (gen << 40) | (ck.e0 + k * 32 + lane));
+    return count;
+}
+
+// One generation's phases, PER events a lane and strip.
+template <int PER>
+__device__ __forceinline__ void ws_claims(const WsState& s, WsGenShared& sh, WsLists& l, const uint32_t* gv, const uint32_t* gp,
+                                          unsigned long long nev, uint32_t depth, unsigned long long gen) {
+    const unsigned long long strips = (nev + PER * 32 - 1) / (PER * 32), step = static_cast<unsigned long long>(gridDim.x) * kGenWarps;
+    // strips dealt to the blocks first, so that a generation of few strips spreads over the SMs
+    unsigned long long c = (threadIdx.x >> 5) * static_cast<unsigned long long>(gridDim.x) + blockIdx.x;
+    if (c >= strips) return;
+    WsStrip next = ws_strip<PER>(c, nev);
+    WsAhead ahead = ws_fetch<PER>(s, next, gv, gp, false);
+    for (; c < strips; c += step) {
+        const WsStrip ck = next;
+        const WsAhead a = ahead;
+        if (c + step < strips) {
+            next = ws_strip<PER>(c + step, nev);
+            ahead = ws_fetch<PER>(s, next, gv, gp, false);
+        }
+        ws_claim_strip<PER>(s, sh, l, ck, a, depth, gen);
+    }
+}
+
+template <int PER>
+__device__ __forceinline__ unsigned ws_resolves(const WsState& s, WsGenShared& sh, WsLists& l, const uint32_t* gv, const uint32_t* gp,
+                                                unsigned long long c, unsigned long long c1, unsigned long long nev, uint32_t depth,
+                                                unsigned long long gen) {
+    if (c >= c1) return 0;
+    unsigned count = 0;
+    WsStrip next = ws_strip<PER>(c, nev);
+    WsAhead ahead = ws_fetch<PER>(s, next, gv, gp, true);
+    for (; c < c1; ++c) {
+        const WsStrip ck = next;
+        const WsAhead a = ahead;
+        if (c + 1 < c1) {
+            next = ws_strip<PER>(c + 1, nev);
+            ahead = ws_fetch<PER>(s, next, gv, gp, true);
+        }
+        count += ws_resolve_strip<PER>(s, sh, l, ck, a, gp, depth, gen);
+    }
+    return count;
+}
+
+// The next frontier is written in event order: each warp resolves one contiguous range of strips and counts
+// its claims of this depth, and behind a grid-wide barrier each block adds up the counts of the blocks before
+// it. (A decoupled look-back in place of that barrier made the generations of 2^12 to 2^15 nodes 20 to 40 %
+// slower.)
+//
+// Up to max_gens generations of one depth in a single cooperative launch, three grid-wide
 // barriers per generation. ng[2] holds the two frontier sizes; the frontier starts on side
 // `cur`. The launch ends early when the frontier has at most small_nodes nodes. out[0] =
 // generations run, out[1] = the side holding the next frontier.
-__global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint32_t* gv0, uint32_t* gp0, uint32_t* gv1,
+__global__ void __launch_bounds__(kGenThreads, 4) ws_generations(WsState s, uint32_t* gv0, uint32_t* gp0, uint32_t* gv1,
                                                              uint32_t* gp1, unsigned int* ng,
-                                                             unsigned long long* desc, uint32_t depth,
+                                                             unsigned int* counts, uint32_t depth,
                                                              unsigned long long gen0, int max_gens, int cur,
                                                              unsigned small_nodes, unsigned long long* out) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    __shared__ unsigned int part[33];
-    const unsigned long long tid = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
-    const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    __shared__ WsGenShared sh;
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+    const bool first_thread = blockIdx.x == 0 && tid == 0;
+    if (tid < 27) {
+        int dx, dy, dz;
+        stencil_offset(static_cast<int>(tid), 0, dx, dy, dz);
+        sh.delta[tid] = (static_cast<uint32_t>(dz) * s.g.SX + dx) * s.g.SY + dy;  // modulo 2^32
+    }
+    WsLists lists{0, 0};
+    __syncthreads();
     unsigned long long gen = gen0;
     int it = 0;
     for (; it < max_gens; ++it) {
@@ -526,7 +565,7 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
         ++gen;
         const int hc = min(63, 63 - __clzll(nev / 27));
         unsigned long long t_start = 0;
-        if (s.gen_hist && tid == 0) {
+        if (s.gen_hist && first_thread) {
             atomicAdd(&s.gen_hist[hc], 1ull);
             t_start = ws_clock();
         }
@@ -534,130 +573,72 @@ __global__ void __launch_bounds__(kChunk / 4, 4) ws_generations(WsState s, uint3
         const uint32_t* gp = cur ? gp1 : gp0;
         uint32_t* nv = cur ? gv0 : gv1;
         uint32_t* np_ = cur ? gp0 : gp1;
-        for (unsigned long long seq = tid; seq < nev; seq += stride) ws_claim_event(s, gv, gp, seq, depth, gen);
+        // one event a lane while the grid covers the generation in two rounds, else kStrip
+        const bool one = nev <= 2ull * gridDim.x * kGenThreads;
+        if (one) ws_claims<1>(s, sh, lists, gv, gp, nev, depth, gen);
+        else ws_claims<kStrip>(s, sh, lists, gv, gp, nev, depth, gen);
         grid.sync();
-        if (s.gen_hist && tid == 0) {
+        if (s.gen_hist && first_thread) {
             const unsigned long long t = ws_clock();
             atomicAdd(&s.gen_hist[64 + hc], t - t_start);
             t_start = t;
         }
-        const unsigned long long nchunks = (nev + kChunk - 1) / kChunk;
-        if (nchunks > 8ull * gridDim.x) {
-            // More than eight rounds of chunks: each block resolves one contiguous range of
-            // events (each warp a contiguous part of it, 32 events a step) and counts its
-            // same-depth claims, marking them in ev_touch; one look-back per block gives its
-            // offset, and a second sweep over the range writes the marked claims in event order.
-            // (Chunks dealt round-robin wait, round after round, for the slowest of their
-            // predecessors in the previous round: at 1024^3, 720 against 837 us per generation
-            // of 2^20 nodes; with fewer rounds the extra sweep costs more than it saves. Issuing
-            // each thread's loads of several events together did not pay in either phase.)
-            const bool probe = s.gen_hist && blockIdx.x == 0 && threadIdx.x == 0;
-            const unsigned long long ta = probe ? ws_clock() : 0;
-            const unsigned nwarp = blockDim.x >> 5;
-            const unsigned long long steps = (nev + 31) / 32;
-            const unsigned long long per_block = (steps + gridDim.x - 1) / gridDim.x;
-            const unsigned long long used = (steps + per_block - 1) / per_block;  // blocks with events
-            const unsigned long long per_warp = (per_block + nwarp - 1) / nwarp;
-            const unsigned long long b0 = blockIdx.x * per_block;
-            const unsigned long long b1 = min(b0 + per_block, steps);
-            const unsigned long long w0 = min(b0 + warp * per_warp, b1);
-            const unsigned long long w1 = min(w0 + per_warp, b1);
-            if (blockIdx.x < used) {
-                unsigned cnt = 0;
-                for (unsigned long long st = w0; st < w1; ++st) {
-                    const unsigned long long seq = st * 32 + lane;
-                    const bool f = seq < nev && ws_resolve_event(s, gv, gp, seq, depth, gen);
-                    if (f) s.ev_touch[seq] = 2;
-                    cnt += __popc(__ballot_sync(0xFFFFFFFFu, f));
-                }
-                if (lane == 0) part[warp] = cnt;
-                __syncthreads();
-                const unsigned long long tb = probe ? ws_clock() : 0;
-                if (warp == 0) {
-                    const unsigned v = lane < nwarp ? part[lane] : 0u;
-                    unsigned incl = v;
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const unsigned t2 = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                        if (lane >= static_cast<unsigned>(o)) incl += t2;
-                    }
-                    const unsigned total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-                    if (lane < nwarp) part[lane] = incl - v;
-                    const unsigned long long base = ws_lookback(desc, blockIdx.x, gen, total, s.err, s.spin_limit, lane);
-                    if (lane == 0) {
-                        part[32] = static_cast<unsigned int>(base);
-                        if (blockIdx.x == used - 1) ng[cur ^ 1] = static_cast<unsigned int>(base + total);
-                    }
-                }
-                __syncthreads();
-                if (probe) {
-                    const unsigned long long tc = ws_clock();
-                    atomicAdd(&s.gen_hist[192], tb - ta);
-                    atomicAdd(&s.gen_hist[193], tc - tb);
-                }
-                unsigned long long pos = static_cast<unsigned long long>(part[32]) + part[warp];
-                for (unsigned long long st = w0; st < w1; ++st) {
-                    const unsigned long long seq = st * 32 + lane;
-                    const bool f = seq < nev && __ldcg(s.ev_touch + seq) == 2;  // L2: no stale L1 line
-                    const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
-                    if (f) ws_put_node(s, gv, gp, seq, nv + (pos + __popc(m & lt)), np_ + (pos + __popc(m & lt)));
-                    pos += __popc(m);
-                }
-            }
-        } else
-        // Resolve by chunks of kChunk events: event k * blockDim + t of a chunk is thread t's
-        // k-th, so event order is k-major, then thread.
-        for (unsigned long long c = blockIdx.x; c < nchunks; c += gridDim.x) {
-            const bool probe = s.gen_hist && blockIdx.x == 0 && threadIdx.x == 0;  // block 0's split
-            const unsigned long long ta = probe ? ws_clock() : 0;
-            unsigned won = 0;  // bit k: the thread's k-th event gives a node of the next generation
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const unsigned long long seq = c * kChunk + k * (kChunk / 4) + threadIdx.x;
-                const bool f = seq < nev && ws_resolve_event(s, gv, gp, seq, depth, gen);
-                if (f) won |= 1u << k;
-                const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
-                if (lane == 0) part[k * (kChunk / 128) + warp] = __popc(m);
-            }
-            __syncthreads();
-            const unsigned long long tb = probe ? ws_clock() : 0;
-            if (warp == 0) {  // 4 rounds x 8 warps = 32 counts in event order
-                const unsigned v = part[lane];
-                unsigned incl = v;
+        // warp w of block b resolves the strips [w0, w1)
+        const unsigned strip = one ? 32 : 32 * kStrip;
+        const unsigned long long strips = (nev + strip - 1) / strip, warps = static_cast<unsigned long long>(gridDim.x) * kGenWarps;
+        const unsigned long long per = (strips + warps - 1) / warps;
+        const unsigned long long w0 = min((static_cast<unsigned long long>(blockIdx.x) * kGenWarps + warp) * per, strips);
+        const unsigned long long w1 = min(w0 + per, strips);
+        unsigned count = one ? ws_resolves<1>(s, sh, lists, gv, gp, w0, w1, nev, depth, gen)
+                             : ws_resolves<kStrip>(s, sh, lists, gv, gp, w0, w1, nev, depth, gen);
+        if (lane == 0) sh.count[warp] = count;
+        __syncthreads();
+        unsigned before = 0, total = 0;  // the block's claims: of the warps before this one, of all
+        for (int i = 0; i < kGenWarps; ++i) {
+            if (i < static_cast<int>(warp)) before += sh.count[i];
+            total += sh.count[i];
+        }
+        if (tid == 0) counts[blockIdx.x] = total;
+        grid.sync();
+        // the claims of the blocks before this one
+        unsigned base = 0;
+        for (unsigned b = tid; b < blockIdx.x; b += kGenThreads) base += __ldcg(counts + b);
+        base = __reduce_add_sync(0xFFFFFFFFu, base);
+        if (lane == 0) sh.base[warp] = base;
+        __syncthreads();
+        base = 0;
+        for (int i = 0; i < kGenWarps; ++i) base += sh.base[i];
+        if (blockIdx.x == gridDim.x - 1 && tid == 0) ng[cur ^ 1] = base + total;
+        size_t pos = static_cast<size_t>(base) + before;
+        if (count) {
+            const unsigned long long b0 = w0 * (strip / 32), b1 = w1 * (strip / 32);  // the range's words of won bits
+            for (unsigned long long b = b0; b < b1; b += 32) {
+                const uint32_t bits = b + lane < b1 ? __ldcg(s.won + b + lane) : 0u;
+                uint32_t incl = __popc(bits);
                 for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned t2 = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                    if (lane >= static_cast<unsigned>(o)) incl += t2;
+                    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= static_cast<unsigned>(o)) incl += t;
                 }
-                const unsigned total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-                part[lane] = incl - v;
-                const unsigned long long base = ws_lookback32(desc, c, gen, total, s.err, s.spin_limit, lane);
-                if (lane == 0) {
-                    part[32] = static_cast<unsigned int>(base);
-                    if (c == nchunks - 1) ng[cur ^ 1] = static_cast<unsigned int>(base + total);
+                for (unsigned some = __ballot_sync(0xFFFFFFFFu, bits); some; some &= some - 1) {
+                    const int q = __ffs(some) - 1;
+                    const uint32_t m = __shfl_sync(0xFFFFFFFFu, bits, q), at = __shfl_sync(0xFFFFFFFFu, incl, q) - __popc(m);
+                    if ((m >> lane) & 1u) {
+                        const unsigned long long e = (b + q) * 32 + lane, i = e / 27;
+                        const uint32_t v = __ldcg(gv + i) + sh.delta[e - i * 27];
+                        nv[pos + at + __popc(m & lt)] = v;
+                        np_[pos + at + __popc(m & lt)] = ws_node(s.g, v, __ldcg(gp + i) & ~kFace);
+                    }
                 }
+                pos += __shfl_sync(0xFFFFFFFFu, incl, 31);
             }
-            __syncthreads();
-            if (probe) {
-                const unsigned long long tc = ws_clock();
-                atomicAdd(&s.gen_hist[192], tb - ta);  // events resolved
-                atomicAdd(&s.gen_hist[193], tc - tb);  // scan and look-back
-            }
-            const unsigned base = part[32];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const bool f = (won >> k) & 1u;
-                const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
-                if (f) {
-                    const unsigned pos = base + part[k * (kChunk / 128) + warp] + __popc(m & lt);
-                    ws_put_node(s, gv, gp, c * kChunk + k * (kChunk / 4) + threadIdx.x, nv + pos, np_ + pos);
-                }
-            }
-            __syncthreads();  // part is reused by the next chunk
         }
         grid.sync();
-        if (s.gen_hist && tid == 0) atomicAdd(&s.gen_hist[128 + hc], ws_clock() - t_start);
+        if (s.gen_hist && first_thread) atomicAdd(&s.gen_hist[128 + hc], ws_clock() - t_start);
         cur ^= 1;
     }
-    if (tid == 0) {
+    if (lists.ext) ws_flush_ext(s, sh, lists.ext);
+    if (lists.up) ws_flush_up(s, sh, lists.up);
+    if (first_thread) {
         out[0] = static_cast<unsigned long long>(it);
         out[1] = static_cast<unsigned long long>(cur);
     }
@@ -868,7 +849,8 @@ __device__ __noinline__ uint32_t ws_small_generation(const WsState& s, WsSmallSh
                             sh.up_val[at] = (static_cast<unsigned long long>(pore) << 32) | w[u];
                             sh.up_r[at] = r;
                         } else {
-                            ws_append(s, __activemask(), w[u], pore, r, seq, gen);
+                            ws_append_entry(s, __activemask(), r, (gen << s.time_shift) | seq,
+                                            (static_cast<unsigned long long>(pore) << 32) | w[u]);
                         }
                     }
                 } else if (st < kTouched) {
@@ -1434,8 +1416,8 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     ws.spin_limit = ctx->limits.spin_limit;
     ws.gen_hist = nullptr;
     if (ctx->timing) {  // frontier sizes of the generations, for the timing report
-        ws.gen_hist = buf<unsigned long long>(ctx, "ws.gen_hist", 194);
-        PMA_CUDA(cudaMemsetAsync(ws.gen_hist, 0, 194 * 8, s));
+        ws.gen_hist = buf<unsigned long long>(ctx, "ws.gen_hist", 192);
+        PMA_CUDA(cudaMemsetAsync(ws.gen_hist, 0, 192 * 8, s));
     }
     ws.pbound = buf<unsigned int>(ctx, "ws.pbound", npores);
     // Shared-voxel records: a first guess of n/32; the pool doubles (copying the records)
@@ -1541,11 +1523,10 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
         ws.time_shift = 1;
         while (ws.time_shift < 41 && (1ull << ws.time_shift) <= std::max<size_t>(max_events, npores)) ++ws.time_shift;
 
-        ws.ev_touch = buf<uint8_t>(ctx, "ws.ev_touch", max_events);  // written for every event by phase 0
-        // chunk descriptors of the frontier compaction; generations restart at 1 in this attempt
-        const size_t max_chunks = (max_events + kChunk - 1) / kChunk;
-        auto* desc = buf<unsigned long long>(ctx, "ws.desc", max_chunks);
-        PMA_CUDA(cudaMemsetAsync(desc, 0, max_chunks * 8, s));
+        // event bits, whole strips; every word of a generation's strips is written before it is read
+        const size_t max_strips = (max_events + kStrip * 32 - 1) / (kStrip * 32);
+        ws.touched = buf<uint32_t>(ctx, "ws.touched", max_strips * kStrip);
+        ws.won = buf<uint32_t>(ctx, "ws.won", max_strips * kStrip);
         PMA_CUDA(cudaMemcpyAsync(d_boff, boff.data(), (nb + 1) * 8ull, cudaMemcpyHostToDevice, s));
         std::vector<unsigned int> h_fill(nb, 0);
         if (npores) {
@@ -1576,15 +1557,14 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
         uint32_t* gpb[2] = {buf<uint32_t>(ctx, "ws.gp0", max_bucket), buf<uint32_t>(ctx, "ws.gp1", max_bucket)};
         // cooperative grid: every block resident at once (grid-wide barriers)
         int per_sm = 0;
-        PMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ws_generations, kChunk / 4, 0));
+        PMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ws_generations, kGenThreads, 0));
         PMA_REQUIRE(per_sm > 0, PMA_ERR_CUDA, "pma_watershed: generation kernel does not fit an SM");
-        // sized to the largest frontier (about 16 events per thread and phase), so that the
-        // launches of small volumes leave the rest of the GPU to other streams (batch lanes).
-        // (Sizing each launch to its starting frontier instead, at about 4 events per thread,
-        // made barriers cheaper but the step slower: 950 -> 971 ms at 1024^3.)
-        const size_t coop_need = (max_events + 16 * (kChunk / 4) - 1) / (16 * (kChunk / 4));
-        const unsigned coop_grid = static_cast<unsigned>(
-            std::max<size_t>(1, std::min<size_t>(coop_need, static_cast<size_t>(ctx->num_sms) * std::min(per_sm, 8))));
+        // sized to the largest frontier (four strips a warp), so that the launches of small volumes
+        // leave the rest of the GPU to other streams (batch lanes)
+        const unsigned coop_grid = static_cast<unsigned>(std::max<size_t>(
+            1, std::min<size_t>((max_strips + 4 * kGenWarps - 1) / (4 * kGenWarps),
+                                static_cast<size_t>(ctx->num_sms) * std::min(per_sm, 8))));
+        unsigned int* counts = buf<unsigned int>(ctx, "ws.counts", coop_grid);  // claims of each block's range
         // generations of this call at most: the context's bound, within the entry-time range
         const unsigned long long max_gen =
             std::min<unsigned long long>(ctx->limits.watershed_generations, kMaxGen - 1);
@@ -1644,10 +1624,10 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
                 PMA_REQUIRE(c.gen < max_gen, PMA_ERR_LIMIT, "pma_watershed: generation limit reached");
                 int gens = static_cast<int>(std::min<unsigned long long>(kGensPerLaunch, max_gen - c.gen));
                 unsigned small_nodes = kSmallNodes;
-                void* args[] = {&ws, &gvb[0], &gpb[0], &gvb[1], &gpb[1], &d_ng, &desc,
+                void* args[] = {&ws, &gvb[0], &gpb[0], &gvb[1], &gpb[1], &d_ng, &counts,
                                 const_cast<uint32_t*>(&dep), &c.gen, &gens, &cur, &small_nodes, &d_out};
                 PMA_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ws_generations), coop_grid,
-                                                     kChunk / 4, args, 0, s));
+                                                     kGenThreads, args, 0, s));
                 ctx->count_launch(1);
                 ctx->count("ws.cooperative_launches", 1);
                 ReadBack rb;
@@ -1671,9 +1651,8 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     }
     PMA_REQUIRE(!(h_err & 2u), PMA_ERR_INTERNAL, "pma_watershed: a shared voxel recorded more pores than touch it");
     PMA_REQUIRE(!(h_err & 8u), PMA_ERR_LIMIT, "pma_watershed: shared-voxel record allocation did not finish");
-    PMA_REQUIRE(!(h_err & 16u), PMA_ERR_LIMIT, "pma_watershed: frontier compaction look-back did not finish");
     if (ws.gen_hist) {
-        unsigned long long hh[194];
+        unsigned long long hh[192];
         PMA_CUDA(cudaMemcpyAsync(hh, ws.gen_hist, sizeof(hh), cudaMemcpyDeviceToHost, s));
         ctx->sync();
         for (int b = 0; b < 64; ++b)
@@ -1683,8 +1662,6 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
                 ctx->count(c + ".claim_ms", hh[64 + b] * 1e-6);
                 ctx->count(c + ".resolve_ms", hh[128 + b] * 1e-6);
             }
-        ctx->count("ws.block0.resolve_events_ms", hh[192] * 1e-6);
-        ctx->count("ws.block0.scan_lookback_ms", hh[193] * 1e-6);
     }
 
     KernelTimer kt_tables(ctx, "ws_tables");  // to the end of the stage
@@ -1829,16 +1806,18 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
 }
 
 void wait_selftest(pma_ctx* ctx, int* timed_out) {
-    unsigned long long* desc = buf<unsigned long long>(ctx, "ws.selftest", 3);
-    unsigned int* err = reinterpret_cast<unsigned int*>(desc + 2);
-    PMA_CUDA(cudaMemsetAsync(desc, 0, 3 * 8, ctx->stream));
-    ws_wait_selftest<<<1, 32, 0, ctx->stream>>>(desc, err, ctx->limits.spin_limit);
+    unsigned int* word = buf<unsigned int>(ctx, "ws.selftest", 2);
+    PMA_CUDA(cudaMemsetAsync(word, 0, 2 * 4, ctx->stream));
+    WsState ws{};
+    ws.err = word + 1;
+    ws.spin_limit = ctx->limits.spin_limit;
+    ws_wait_selftest<<<1, 32, 0, ctx->stream>>>(ws, word);
     ctx->count_launch();
     ctx->check_launch("ws_wait_selftest");
-    unsigned int h[2] = {0, 0};
-    PMA_CUDA(cudaMemcpyAsync(h, err, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    unsigned int h = 0;
+    PMA_CUDA(cudaMemcpyAsync(&h, word + 1, 4, cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
-    *timed_out = (h[0] & h[1] & 16u) ? 1 : 0;
+    *timed_out = (h & 8u) ? 1 : 0;
 }
 
 }  // namespace pma
