@@ -15,9 +15,9 @@
 //    with an edge into p.
 //  * Plateaus are found by a union-find over equal-crad neighbours (from 2^24 voxels:
 //    pointer jumping on the initial trees, then unions of the recorded parent pairs).
-//  * Both recurrences run plateau by plateau in decreasing crad, one launch per crad level. The ball order is std::sort's on the host (ordered_sort: libstdc++'s own
-//    introsort steps on several threads) applied to the same sequence (z, x, y scan order)
-//    with the same comparator, so equal radii tie-break exactly as in the reference.
+//  * Both recurrences run plateau by plateau in decreasing crad, one launch per crad level. The ball
+//    order is the permutation that std::sort gives the same sequence (z, x, y scan order) under the
+//    same comparator (ordered_sort_device), so equal radii tie-break exactly as in the reference.
 //  * A voxel's label is its seed's pore id when |S| = 1 and a shared type ("throat") when
 //    |S| >= 2. Pore volumes, boundary flags, type volumes and type pore lists are exact.
 //    The reference numbers types in its depth-first creation order, which also consumed ids
@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "devutil.cuh"
+#include "ordered_sort.cuh"
 #include "ordered_sort.h"
 
 namespace pma {
@@ -74,9 +75,13 @@ __global__ void pack_items(const uint32_t* __restrict__ r2, const uint32_t* __re
     PMA_GRID_STRIDE(i, n) items[i] = (static_cast<unsigned long long>(r2[i]) << 32) | idx[i];
 }
 
-__global__ void scatter_rank(const uint32_t* __restrict__ voxel_of_rank, size_t n,
-                             uint32_t* __restrict__ crank) {
-    PMA_GRID_STRIDE(r, n) crank[voxel_of_rank[r]] = static_cast<uint32_t>(r);
+__global__ void scatter_rank(const unsigned long long* __restrict__ items, size_t n, uint32_t* __restrict__ crank) {
+    PMA_GRID_STRIDE(r, n) crank[static_cast<uint32_t>(items[r])] = static_cast<uint32_t>(r);
+}
+
+__global__ void gather_items(const unsigned long long* __restrict__ items, const uint32_t* __restrict__ ranks, size_t n,
+                             unsigned long long* __restrict__ out) {
+    PMA_GRID_STRIDE(k, n) out[k] = items[ranks[k]];
 }
 
 // --- union-find over equal-crad neighbours (parents always point to smaller indices) ---
@@ -1225,61 +1230,37 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         gather_u32<<<grid_for(ctx, nb), 256, 0, s>>>(edt2, balls, nb, ball_r2);
         ctx->check_launch("gather_u32");
     }
-    // std::sort with the reference's comparator (PoreAndThroatComputer.cpp:121-122), run on
-    // host threads (ordered_sort: the same permutation) while the plateau kernels below run.
-    // The items are 8-byte (r2, voxel index) pairs compared on r2 alone: std::sort's moves
-    // depend only on comparison results, so the permutation equals the one the reference's
-    // 16-byte balls go through, and the sorted items carry each rank's voxel. They are packed
-    // on the device and sorted in a page-locked buffer of the context.
-    auto kt_balls_host = std::make_unique<KernelTimer>(ctx, "pores_balls_to_host");
-    auto* items = static_cast<unsigned long long*>(ctx->host_buffer("pores.items", nb * 8));
-    auto* voxel_of_rank = static_cast<uint32_t*>(ctx->host_buffer("pores.voxel_of_rank", nb * 4));
+    // std::sort with the reference's comparator (PoreAndThroatComputer.cpp:121-122): the items are
+    // 8-byte (r2, voxel index) pairs compared on r2 alone. std::sort's moves depend only on
+    // comparison results, so the permutation equals the one the reference's 16-byte balls go
+    // through, and the sorted items carry each rank's voxel.
+    auto* items = buf<unsigned long long>(ctx, "pores.d_items", nb);
+    uint32_t* pid = buf<uint32_t>(ctx, "pores.pid", n);      // root voxel, then plateau id
+    uint32_t* crank = buf<uint32_t>(ctx, "pores.crank", n);  // both are the sort's scratch first
     if (nb) {
-        auto* d_items = buf<unsigned long long>(ctx, "pores.d_items", nb);
-        pack_items<<<grid_for(ctx, nb), 256, 0, s>>>(ball_r2, balls, nb, d_items);
-        ctx->check_launch("pack_items");
-        copy_to_host(ctx, items, d_items, nb * 8);
-        ctx->sync();
-    }
-    kt_balls_host.reset();
-    struct Joiner {
-        std::thread t;
-        ~Joiner() {
-            if (t.joinable()) t.join();
-        }
-    } sorter;
-    // up to 16 leaf tasks (levels 4) where the host has the cores and each leaf gets at least
-    // 2^16 balls: the leaves' sorts are most of the time, the top partition steps run on one
-    // to eight threads; small volumes (the batched and serving forms run many at once) sort
-    // on this one thread
-    int sort_levels = 0;
-    while (sort_levels < 4 && (2u << sort_levels) <= std::thread::hardware_concurrency() &&
-           (static_cast<unsigned long long>(nb) >> (16 + sort_levels + 1)) > 0)
-        ++sort_levels;
-    // then the voxel of each rank, taken from the sorted items on host threads too
-    sorter.t = std::thread([items, voxel_of_rank, nb, sort_levels] {
-        ordered_sort(
-            items, items + nb,
-            [](unsigned long long a, unsigned long long b) { return (a >> 32) > (b >> 32); }, sort_levels);
-        const int64_t m = nb;
-        auto gather = [&](int64_t lo, int64_t hi) {
-            for (int64_t r = lo; r < hi; ++r) voxel_of_rank[r] = static_cast<uint32_t>(items[r]);
+        KernelTimer kt(ctx, "pores_sort");
+        auto pack = [&] {
+            pack_items<<<grid_for(ctx, nb), 256, 0, s>>>(ball_r2, balls, nb, items);
+            ctx->check_launch("pack_items");
         };
-        const int nt = m >= (1 << 20) ? (1 << sort_levels) : 1;
-        std::vector<std::thread> ts;
-        for (int t = 1; t < nt; ++t) {
-            try {
-                ts.emplace_back(gather, m * t / nt, m * (t + 1) / nt);
-            } catch (const std::system_error&) {
-                gather(m * t / nt, m * (t + 1) / nt);  // no thread to be had: in line
-            }
+        pack();
+        if (!ordered_sort_device(ctx, items, nb, pid, crank)) {
+            // a range reached std::sort's depth limit (an adversary's order; none is known from a volume):
+            // libstdc++'s own routines on the host, on up to 16 threads
+            pack();
+            std::vector<unsigned long long> h(nb);
+            PMA_CUDA(cudaMemcpyAsync(h.data(), items, nb * 8, cudaMemcpyDeviceToHost, s));
+            ctx->sync();
+            int levels = 0;
+            while (levels < 4 && (2u << levels) <= std::thread::hardware_concurrency()) ++levels;
+            ordered_sort(
+                h.data(), h.data() + nb, [](unsigned long long x, unsigned long long y) { return (x >> 32) > (y >> 32); }, levels);
+            PMA_CUDA(cudaMemcpyAsync(items, h.data(), nb * 8, cudaMemcpyHostToDevice, s));
+            ctx->sync();
         }
-        gather(0, m / nt);
-        for (auto& th : ts) th.join();
-    });
+    }
 
     // Plateaus: connected sets of equal crad under the stencil.
-    uint32_t* pid = buf<uint32_t>(ctx, "pores.pid", n);  // root voxel, then plateau id
     uf_init<<<G, 256, 0, s>>>(crad2, g, n, d3q7, pid);
     ctx->check_launch("uf_init");
     {
@@ -1389,16 +1370,11 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     ctx->check_launch("edge_offsets");
     kt_edges.reset();
 
-    auto kt_join = std::make_unique<KernelTimer>(ctx, "pores_sort_wait");
-    sorter.t.join();
-    kt_join.reset();
     auto kt_stats = std::make_unique<KernelTimer>(ctx, "plateau_stats");
-    uint32_t* crank = buf<uint32_t>(ctx, "pores.crank", n);
     fill_u32<<<G, 256, 0, s>>>(crank, n, kNone);
     ctx->check_launch("fill_u32");
     if (nb) {
-        copy_from_host(ctx, balls, voxel_of_rank, nb * 4);
-        scatter_rank<<<grid_for(ctx, nb), 256, 0, s>>>(balls, nb, crank);
+        scatter_rank<<<grid_for(ctx, nb), 256, 0, s>>>(items, nb, crank);
         ctx->check_launch("scatter_rank");
     }
     uint32_t* pcrad = buf<uint32_t>(ctx, "pores.pcrad", np);
@@ -1581,6 +1557,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     fill_u32<<<grid_for(ctx, nrank), 256, 0, s>>>(d_rank2pore, nrank, kNone);
     ctx->check_launch("fill_u32");
     PMA_CUDA(cudaMemsetAsync(d_rank2id, 0, nrank * 4, s));
+    auto* seed_items = buf<unsigned long long>(ctx, "pores.seed_items", npores);
     if (npores) {
         std::vector<uint32_t> up(2 * npores);
         std::copy(seed_ranks.begin(), seed_ranks.end(), up.begin());
@@ -1589,6 +1566,8 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         PMA_CUDA(cudaMemcpyAsync(d_up, up.data(), up.size() * 4, cudaMemcpyHostToDevice, s));
         scatter_seed_ids<<<grid_for(ctx, npores), 256, 0, s>>>(d_up, npores, d_rank2pore, d_rank2id);
         ctx->check_launch("scatter_seed_ids");
+        gather_items<<<grid_for(ctx, npores), 256, 0, s>>>(items, d_up, npores, seed_items);
+        ctx->check_launch("gather_items");
     }
     PoreAcc pa;
     pa.rank2pore = d_rank2pore;
@@ -1737,22 +1716,23 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     // Table (pores in id order, throats in id order).
     std::vector<unsigned long long> pvol(npores);
     std::vector<unsigned int> pbound(npores);
+    std::vector<unsigned long long> h_items(npores);
     if (npores) {
+        PMA_CUDA(cudaMemcpyAsync(h_items.data(), seed_items, npores * 8, cudaMemcpyDeviceToHost, s));
         PMA_CUDA(cudaMemcpyAsync(pvol.data(), pa.pvol, npores * 8, cudaMemcpyDeviceToHost, s));
         PMA_CUDA(cudaMemcpyAsync(pbound.data(), pa.pbound, npores * 4, cudaMemcpyDeviceToHost, s));
     }
     ctx->sync();
     for (size_t k = 0; k < npores; ++k) {
-        const uint32_t r = seed_ranks[k];
         int x, y, z;
-        g.coords(voxel_of_rank[r], x, y, z);
+        g.coords(static_cast<uint32_t>(h_items[k]), x, y, z);
         pma_pore p;
         std::memset(&p, 0, sizeof(p));
         p.id = ids[k];
         p.seed_x = x;
         p.seed_y = y;
         p.seed_z = z;
-        p.seed_r2 = static_cast<uint32_t>(items[r] >> 32);
+        p.seed_r2 = static_cast<uint32_t>(h_items[k] >> 32);
         p.is_boundary = pbound[k] ? 1 : 0;
         p.volume = pvol[k];
         t->pores.push_back(p);
