@@ -372,7 +372,7 @@ inline bool ordered_sort_device(pma_ctx* ctx, unsigned long long* items, int64_t
         sort_positions<<<nc, kPartThreads, 0, s>>>(items, d_ranges, d_chunks, d_left, d_right, lpos, rpos);
         sort_cuts<<<div_up(nr, 4), 128, 0, s>>>(d_ranges, nr, d_total, lpos, rpos, d_swaps, d_cut);
         sort_swap<<<nc, kPartThreads, 0, s>>>(items, d_ranges, d_chunks, d_swaps, lpos, rpos);
-        ctx->count_launch(6);
+        ctx->count_launch(5);
         ctx->check_launch("sort_partition");
         cuts.resize(nr);
         PMA_CUDA(cudaMemcpyAsync(cuts.data(), d_cut, nr * 4ull, cudaMemcpyDeviceToHost, s));
@@ -392,7 +392,6 @@ inline bool ordered_sort_device(pma_ctx* ctx, unsigned long long* items, int64_t
     PMA_CUDA(cudaMemcpyAsync(d_small, small.data(), small.size() * sizeof(SortRange), cudaMemcpyHostToDevice, s));
     if (!small.empty()) {
         sort_block<<<static_cast<unsigned>(small.size()), kBlockSortThreads, sizeof(BlockSortShared), s>>>(items, d_small, failed);
-        ctx->count_launch();
         ctx->check_launch("sort_block");
     }
     auto* h = static_cast<unsigned int*>(ctx->host_staging(64));

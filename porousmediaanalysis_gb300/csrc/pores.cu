@@ -38,6 +38,7 @@
 #include "devutil.cuh"
 #include "ordered_sort.cuh"
 #include "ordered_sort.h"
+#include "type_rows.cuh"
 
 namespace pma {
 namespace {
@@ -1094,7 +1095,6 @@ __global__ void group_starts(const uint32_t* __restrict__ sorted_p, const unsign
 }
 
 struct GroupOut {
-    uint32_t* group_of;             // per multi index (sorted order) -> group
     unsigned long long* gvol;       // per group
     unsigned long long* gfirst;     // per group: smallest root voxel index
     uint32_t* grep;                 // per group: representative plateau
@@ -1183,14 +1183,27 @@ __global__ void to_group_index(const uint32_t* __restrict__ excl, const uint32_t
     PMA_GRID_STRIDE(i, m) out[i] = excl[i] + start[i] - 1u;
 }
 
-// Pore ids of each group's seed list (ascending ranks give ascending ids).
-__global__ void gather_lists(const unsigned long long* __restrict__ soff, const uint32_t* __restrict__ slen,
-                             const uint32_t* __restrict__ pool, const uint32_t* __restrict__ rep,
-                             const unsigned long long* __restrict__ roff, size_t ng,
-                             const uint32_t* __restrict__ rank2id, uint32_t* __restrict__ out) {
-    PMA_GRID_STRIDE(gi, ng) {
-        const uint32_t p = rep[gi];
-        for (uint32_t k = 0; k < slen[p]; ++k) out[roff[gi] + k] = rank2id[pool[soff[p] + k]];
+// A type's pore ids in processing order, [second, first, third, ...] of its seed list in ascending ranks,
+// which are ascending ids (BasePoreAndThroatComputer.cpp:338-340, 370-371).
+struct SeedLists {
+    const uint32_t* grep;
+    const unsigned long long* soff;
+    const uint32_t* slen;
+    const uint32_t* pool;
+    const uint32_t* rank2id;
+    __device__ __forceinline__ uint32_t length(uint32_t g) const { return slen[grep[g]]; }
+    __device__ __forceinline__ uint32_t pore(uint32_t g, uint32_t j) const {
+        return rank2id[pool[soff[grep[g]] + (j < 2 ? 1 - j : j)]];
+    }
+};
+
+// Keys that order the types: (last pore, first voxel) (BasePoreAndThroatComputer.cpp:122-130). Both fit 32
+// bits, and the first voxels are distinct. In place of the first voxels.
+__global__ void type_keys(SeedLists lists, size_t ng, unsigned long long* __restrict__ first_voxel) {
+    PMA_GRID_STRIDE(g, ng) {
+        const uint32_t p = lists.grep[g];  // lists of at least two: the last seed is the last pore
+        const uint32_t last = lists.rank2id[lists.pool[lists.soff[p] + lists.slen[p] - 1]];
+        first_voxel[g] = (static_cast<unsigned long long>(last) << 32) | (first_voxel[g] & 0xFFFFFFFFull);
     }
 }
 
@@ -1591,15 +1604,10 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     const int64_t nm = np ? select_flagged(ctx, thrust::counting_iterator<uint32_t>(0), flags, multi,
                                            np, d_count)
                           : 0;
-    std::vector<uint32_t> group_tid_h;
     uint32_t* plateau_group = buf<uint32_t>(ctx, "pores.pgroup", np);
-    uint32_t* group_tid = nullptr;
     pma_table* t = new pma_table;
-    std::vector<unsigned long long> h_gvol, h_gfirst;
-    std::vector<uint32_t> h_grep;
-    std::vector<uint32_t> flat;                // pore ids of each group's list, concatenated
-    std::vector<unsigned long long> roff(1, 0);  // list offsets into flat
     int64_t ngroups = 0;
+    GroupOut go{};
     if (nm) {
         auto* h1 = buf<unsigned long long>(ctx, "pores.h1", nm);
         auto* h2 = buf<unsigned long long>(ctx, "pores.h2", nm);
@@ -1645,61 +1653,29 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         ngroups = static_cast<int64_t>(last_off) + last_start;
         to_group_index<<<grid_for(ctx, nm), 256, 0, s>>>(gid, gstart, nm, gstart);
         ctx->check_launch("to_group_index");
-        GroupOut go;
         go.gvol = buf<unsigned long long>(ctx, "pores.gvol", ngroups);
         go.gfirst = buf<unsigned long long>(ctx, "pores.gfirst", ngroups);
         go.grep = buf<uint32_t>(ctx, "pores.grep", ngroups);
-        go.group_of = nullptr;
         PMA_CUDA(cudaMemsetAsync(go.gvol, 0, ngroups * 8, s));
         PMA_CUDA(cudaMemsetAsync(go.gfirst, 0xFF, ngroups * 8, s));
         group_reduce<<<grid_for(ctx, nm), 256, 0, s>>>(v2, gstart, nm, psize, roots, go, plateau_group);
         ctx->check_launch("group_reduce");
-        h_gvol.resize(ngroups);
-        h_gfirst.resize(ngroups);
-        h_grep.resize(ngroups);
-        PMA_CUDA(cudaMemcpyAsync(h_gvol.data(), go.gvol, ngroups * 8, cudaMemcpyDeviceToHost, s));
-        PMA_CUDA(cudaMemcpyAsync(h_gfirst.data(), go.gfirst, ngroups * 8, cudaMemcpyDeviceToHost, s));
-        PMA_CUDA(cudaMemcpyAsync(h_grep.data(), go.grep, ngroups * 4, cudaMemcpyDeviceToHost, s));
         unsigned int h_err = 0;
         PMA_CUDA(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s));
         ctx->sync();
         PMA_REQUIRE(!(h_err & 4u), PMA_ERR_INTERNAL, "pma_pores: seed-set hash collision");
-        // Representative seed lists, gathered into one buffer.
-        std::vector<uint32_t> rlen(ngroups);
-        uint32_t* d_rep_len = buf<uint32_t>(ctx, "pores.rlen", ngroups);
-        gather_u32<<<grid_for(ctx, ngroups), 256, 0, s>>>(slen, go.grep, ngroups, d_rep_len);
-        ctx->check_launch("gather_u32");
-        PMA_CUDA(cudaMemcpyAsync(rlen.data(), d_rep_len, ngroups * 4, cudaMemcpyDeviceToHost, s));
-        ctx->sync();
-        roff.assign(ngroups + 1, 0);
-        for (int64_t gi = 0; gi < ngroups; ++gi) roff[gi + 1] = roff[gi] + rlen[gi];
-        auto* d_roff = buf<unsigned long long>(ctx, "pores.roff", ngroups + 1);
-        uint32_t* d_rlist = buf<uint32_t>(ctx, "pores.rlist", roff[ngroups]);
-        PMA_CUDA(cudaMemcpyAsync(d_roff, roff.data(), (ngroups + 1) * 8, cudaMemcpyHostToDevice, s));
-        gather_lists<<<grid_for(ctx, ngroups), 256, 0, s>>>(soff, slen, ps.pool, go.grep, d_roff,
-                                                            ngroups, d_rank2id, d_rlist);
-        ctx->check_launch("gather_lists");
-        flat.resize(roff[ngroups]);
-        PMA_CUDA(cudaMemcpyAsync(flat.data(), d_rlist, flat.size() * 4, cudaMemcpyDeviceToHost, s));
-        ctx->sync();
     }
     kt_groups.reset();
-    auto kt_host = std::make_unique<KernelTimer>(ctx, "tables_ids");
-    // Throat ids: order by (last pore of the type, first voxel), counting down from
-    // UINT32_MAX - 1 (BasePoreAndThroatComputer.cpp:122-130).
-    // key = (last pore id << 32) | first voxel; both fit 32 bits and first voxels are distinct
-    std::vector<std::pair<unsigned long long, int64_t>> gkey(ngroups);
-    for (int64_t i = 0; i < ngroups; ++i)
-        gkey[i] = {(static_cast<unsigned long long>(flat[roff[i + 1] - 1]) << 32) | (h_gfirst[i] & 0xFFFFFFFFull), i};
-    std::sort(gkey.begin(), gkey.end());
-    std::vector<int64_t> gorder(ngroups);
-    for (int64_t k = 0; k < ngroups; ++k) gorder[k] = gkey[k].second;
-    group_tid_h.assign(std::max<int64_t>(ngroups, 1), 0);
-    for (int64_t k = 0; k < ngroups; ++k) group_tid_h[gorder[k]] = 0xFFFFFFFFu - 1u - static_cast<uint32_t>(k);
-    group_tid = buf<uint32_t>(ctx, "pores.gtid", group_tid_h.size());
-    PMA_CUDA(cudaMemcpyAsync(group_tid, group_tid_h.data(), group_tid_h.size() * 4, cudaMemcpyHostToDevice, s));
+    auto kt_types = std::make_unique<KernelTimer>(ctx, "tables_ids");
+    uint32_t* group_tid = buf<uint32_t>(ctx, "pores.gtid", ngroups);
+    if (ngroups) {
+        const SeedLists lists{go.grep, soff, slen, ps.pool, d_rank2id};
+        type_keys<<<grid_for(ctx, ngroups), 256, 0, s>>>(lists, ngroups, go.gfirst);
+        ctx->check_launch("type_keys");
+        type_rows(ctx, go.gfirst, ngroups, lists, go.gvol, group_tid, t);
+    }
 
-    kt_host.reset();
+    kt_types.reset();
     auto kt_labels = std::make_unique<KernelTimer>(ctx, "tables_labels");
     // Labels.
     uint32_t* plabel = buf<uint32_t>(ctx, "pores.plabel", np);
@@ -1713,7 +1689,7 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
 
     kt_labels.reset();
     KernelTimer kt_rows(ctx, "tables_rows");
-    // Table (pores in id order, throats in id order).
+    // The pores' rows, in id order.
     std::vector<unsigned long long> pvol(npores);
     std::vector<unsigned int> pbound(npores);
     std::vector<unsigned long long> h_items(npores);
@@ -1736,24 +1712,6 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         p.is_boundary = pbound[k] ? 1 : 0;
         p.volume = pvol[k];
         t->pores.push_back(p);
-    }
-    // Throat rows: pore list in processing order [second, first, third, ...]
-    // (BasePoreAndThroatComputer.cpp:338-340, 370-371), sorted by id.
-    t->throats.resize(ngroups);
-    t->pool.resize(roff[ngroups]);
-    size_t at = 0;
-    for (int64_t k = 0; k < ngroups; ++k) {
-        const int64_t gi = gorder[ngroups - 1 - k];
-        pma_throat& th = t->throats[k];
-        th.id = group_tid_h[gi];
-        th.volume = h_gvol[gi];
-        th.pool_offset = at;
-        const uint32_t* L = flat.data() + roff[gi];
-        const size_t nl = roff[gi + 1] - roff[gi];
-        th.n_pores = static_cast<uint32_t>(nl);
-        t->pool[at++] = L[1];
-        t->pool[at++] = L[0];
-        for (size_t j = 2; j < nl; ++j) t->pool[at++] = L[j];
     }
     if (ctx->reference_throat_ids && ngroups) {
         KernelTimer kt_exact(ctx, "exact_type_ids");

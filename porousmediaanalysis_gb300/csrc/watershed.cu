@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "devutil.cuh"
+#include "type_rows.cuh"
 
 namespace pma {
 namespace {
@@ -1257,10 +1258,6 @@ __global__ void ws_keys(const uint32_t* __restrict__ sv, size_t ns, const unsign
     }
 }
 
-__global__ void ws_iota(uint32_t* __restrict__ a, size_t n) {
-    PMA_GRID_STRIDE(i, n) a[i] = static_cast<uint32_t>(i);
-}
-
 __global__ void ws_gather_h(const unsigned long long* __restrict__ h, const uint32_t* __restrict__ idx,
                             size_t n, unsigned long long* __restrict__ out) {
     PMA_GRID_STRIDE(i, n) out[i] = h[idx[i]];
@@ -1339,14 +1336,18 @@ __global__ void ws_shared_labels(const uint32_t* __restrict__ sv, const uint32_t
     PMA_GRID_STRIDE(i, ns) labels[sv[i]] = gid[final_group[i]];
 }
 
-__global__ void ws_group_rows(const uint32_t* __restrict__ grep, size_t ngr, const uint32_t* __restrict__ kseq,
-                              const unsigned long long* __restrict__ koff, const uint32_t* __restrict__ rvox,
-                              uint32_t* __restrict__ out) {
-    PMA_GRID_STRIDE(g, ngr) {
-        const RecRef a = ws_rec(grep[g], rvox, koff);
-        for (uint32_t k = 0; k < kKeyMax; ++k) out[g * kKeyMax + k] = k < a.L ? kseq[a.kbase + k] : kNone;
+// A type's pore ids in the order of its list: the prefix that its representative record stands for.
+struct PrefixLists {
+    const uint32_t* grep;
+    const uint32_t* kseq;
+    const unsigned long long* koff;
+    const uint32_t* rvox;
+    const uint32_t* pore_id;
+    __device__ __forceinline__ uint32_t length(uint32_t g) const { return ws_rec(grep[g], rvox, koff).L; }
+    __device__ __forceinline__ uint32_t pore(uint32_t g, uint32_t j) const {
+        return pore_id[kseq[ws_rec(grep[g], rvox, koff).kbase + j]];
     }
-}
+};
 
 // The dynamic shared-memory limit is a process-wide attribute of the kernel: set once per device.
 void small_smem_attribute() {
@@ -1723,8 +1724,8 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     ctx->check_launch("ws_keys");
     uint32_t* rec = buf<uint32_t>(ctx, "ws.rec", nr);
     uint32_t* rec2 = buf<uint32_t>(ctx, "ws.rec2", nr);
-    ws_iota<<<grid_for(ctx, nr), 256, 0, s>>>(rec, nr);
-    ctx->check_launch("ws_iota");
+    type_iota<<<grid_for(ctx, nr), 256, 0, s>>>(rec, nr);
+    ctx->check_launch("type_iota");
     // Equal prefixes become adjacent: a radix sort by the first hash (values: record ids),
     // unless two different prefixes share it (about n^2 / 2^65 likely), which ws_group_starts
     // flags; then stable sorts by the second hash and then the first.
@@ -1765,43 +1766,12 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     ws_group_reduce<<<grid_for(ctx, nr), 256, 0, s>>>(rec, gexcl, gstart, nr, rtime, klen, koff, rvox, gtime,
                                                       gvol, grep, final_group);
     ctx->check_launch("ws_group_reduce");
-    uint32_t* rows = buf<uint32_t>(ctx, "ws.rows", static_cast<size_t>(ngr) * kKeyMax);
-    ws_group_rows<<<grid_for(ctx, ngr), 256, 0, s>>>(grep, ngr, kseq, koff, rvox, rows);
-    ctx->check_launch("ws_group_rows");
-    std::vector<unsigned long long> h_gtime(ngr), h_gvol(ngr);
-    std::vector<uint32_t> h_rows(static_cast<size_t>(ngr) * kKeyMax);
-    PMA_CUDA(cudaMemcpyAsync(h_gtime.data(), gtime, ngr * 8, cudaMemcpyDeviceToHost, s));
-    PMA_CUDA(cudaMemcpyAsync(h_gvol.data(), gvol, ngr * 8, cudaMemcpyDeviceToHost, s));
-    PMA_CUDA(cudaMemcpyAsync(h_rows.data(), rows, h_rows.size() * 4, cudaMemcpyDeviceToHost, s));
-    ctx->sync();
-    // ids in creation order
-    std::vector<std::pair<unsigned long long, uint32_t>> by_time(ngr);  // creation times are distinct
-    for (int64_t i = 0; i < ngr; ++i) by_time[i] = {h_gtime[i], static_cast<uint32_t>(i)};
-    std::sort(by_time.begin(), by_time.end());
-    std::vector<uint32_t> order(ngr);
-    for (int64_t k = 0; k < ngr; ++k) order[k] = by_time[k].second;
-    std::vector<uint32_t> gid(ngr);
-    for (int64_t k = 0; k < ngr; ++k) gid[order[k]] = 0xFFFFFFFFu - 1u - static_cast<uint32_t>(k);
+    // ids in creation order (creation times are distinct), rows by ascending id
     uint32_t* d_gid = buf<uint32_t>(ctx, "ws.gid", ngr);
-    PMA_CUDA(cudaMemcpyAsync(d_gid, gid.data(), ngr * 4, cudaMemcpyHostToDevice, s));
+    type_rows(ctx, gtime, ngr, PrefixLists{grep, kseq, koff, rvox, d_pid}, gvol, d_gid, t);
     ws_shared_labels<<<grid_for(ctx, nsh), 256, 0, s>>>(sv, final_group, d_gid, nsh, labels);
     ctx->check_launch("ws_shared_labels");
     ctx->sync();
-    // rows in id order (ascending id = reverse creation order)
-    t->throats.reserve(ngr);
-    t->pool.reserve(static_cast<size_t>(ngr) * 3);
-    for (int64_t k = ngr - 1; k >= 0; --k) {
-        const uint32_t gi = order[k];
-        pma_throat th;
-        th.id = gid[gi];
-        th.volume = h_gvol[gi];
-        th.pool_offset = t->pool.size();
-        uint32_t L = 0;
-        for (int j = 0; j < kKeyMax && h_rows[static_cast<size_t>(gi) * kKeyMax + j] != kNone; ++j, ++L)
-            t->pool.push_back(pore_id[h_rows[static_cast<size_t>(gi) * kKeyMax + j]]);
-        th.n_pores = L;
-        t->throats.push_back(th);
-    }
     return t;
 }
 
