@@ -15,20 +15,24 @@
 // exactly for R < kExactTable and replaced above it by the continuous sufficient condition
 // (sqrt(R) + sqrt(k))^2 <= R'.
 //
-// Gather: the volume is cut into 8^3 tiles; every kept centre is listed in each tile its
-// ball reaches, unless its key is below the tile's floor (the largest key of a ball covering
-// the whole tile, which every voxel of the tile is covered by). One CTA per tile orders its
-// list by radius in shared memory, and each warp of voxels takes, per voxel, the largest key
-// among the entries whose ball covers it: the reference's winner. A warp only tests entries
-// that reach its 2 x 4 x 4 box and beat its lanes' smallest key so far, and stops where the
-// radius order shows that no later entry can, so the work is close to the winners' ranks in
-// the list rather than the ball volumes a scatter would touch.
+// Gather: the volume is cut into 8^3 tiles, in groups of 2 x 2 x 2; every kept centre is listed in each
+// group its ball reaches, and from there in each of the group's tiles that it reaches, unless its
+// key is below the tile's floor (the largest key found of a ball covering the whole tile, which every
+// voxel of the tile is covered by). One CTA per tile orders its list by radius in shared memory, and
+// each warp of voxels takes, per voxel, the largest key among the entries whose ball covers it: the
+// reference's winner. A warp only tests entries that reach the box of its voxels that may still gain
+// and stops where the radius order shows that no later entry can, so the work is close to the
+// winners' ranks in the list rather than the ball volumes a scatter would touch.
 //
-// What bounds it: instructions in the gather (half the issue slots), atomics in the count and the fill (1.3
-// entries per voxel of a spinodal). 704 x 768 x 811 spinodal, before and after these forms, ms: kept
-// centres 13 -> 2.9, floors and counts 23 -> 19.9, fill 19 -> 18.2, gather 117 -> 44 (least key by
-// 32-bit reductions and 2 x 4 x 4 boxes 82, centres by descending radius 73, the box of the lanes still
-// open 44); stage 170 -> 91.
+// What bounds it: instructions and barriers in the gather, a chunk after the other; atomics and scattered
+// stores in the fill. Atomics go at 60 G/s, whatever they add: one for each entry of a tile (1.1 G in
+// a 704 x 768 x 811 spinodal) took 18 ms in the count and again in the fill; the groups' lists have a
+// quarter of the entries, and the split reads them in order. That spinodal, ms: kept centres 13 -> 2.9 (bricks),
+// floors and counts 23 -> 4.6 (groups; a quarter of the centres for the floors, 9 -> 2.5), fill 19 -> 7.0
+// and split 7.9, gather 117 -> 38 (least key by 32-bit reductions and 2 x 4 x 4 boxes 82, centres by
+// descending radius 73, the box of the lanes still open 44, lists in the order of the radii 41, four CTAs
+// an SM 38); stage 170 -> 66. A gather that filters its group's list itself took 68 ms, one that keeps the
+// lists' own order 45, lists in chunks of 1024 44.
 #include <thrust/iterator/counting_iterator.h>
 
 #include <vector>
@@ -41,6 +45,7 @@ namespace {
 constexpr uint32_t kExactTable = 1u << 16;
 constexpr int kTile = 8;          // tile edge
 constexpr int kTileVox = 512;     // voxels (and threads) per tile
+constexpr int kGroup = 2;         // tiles along the edge of a group, which shares one list
 constexpr int kListCap = 2048;    // entries ordered in shared memory at a time; longer lists go in chunks
 
 __device__ __forceinline__ uint32_t isqrt_u32(uint32_t n) {
@@ -148,31 +153,32 @@ __global__ void __launch_bounds__(32 * kBrickX) balls_candidate_flags(const uint
 }
 
 struct Tiles {
-    int TX, TY, TZ;  // tiles per axis
+    int TX, TY, TZ;  // tiles (or groups of them) per axis
     __device__ __forceinline__ size_t id(int tx, int ty, int tz) const {
         return (static_cast<size_t>(tz) * TX + tx) * TY + ty;
     }
 };
 
-// Visits the tiles whose box is within sqrt(R) of centre (x, y, z), restricted to tile
+// Visits the groups whose box is within sqrt(R) of centre (x, y, z), restricted to group
 // z-range [tz0, tz1).
 template <class F>
-__device__ __forceinline__ void for_each_tile(Grid g, Tiles t, int x, int y, int z, uint32_t R,
-                                              int tz0, int tz1, F f) {
+__device__ __forceinline__ void for_each_group(Grid g, Tiles t, int x, int y, int z, uint32_t R,
+                                               int tz0, int tz1, F f) {
+    constexpr int kEdge = kTile * kGroup;
     const int r = static_cast<int>(isqrt_u32(R));
-    const int ax = max(x - r, 0) / kTile, bx = min(x + r, g.SX - 1) / kTile;
-    const int ay = max(y - r, 0) / kTile, by = min(y + r, g.SY - 1) / kTile;
-    const int az = max(max(z - r, 0) / kTile, tz0), bz = min(min(z + r, g.SZ - 1) / kTile, tz1 - 1);
+    const int ax = max(x - r, 0) / kEdge, bx = min(x + r, g.SX - 1) / kEdge;
+    const int ay = max(y - r, 0) / kEdge, by = min(y + r, g.SY - 1) / kEdge;
+    const int az = max(max(z - r, 0) / kEdge, tz0), bz = min(min(z + r, g.SZ - 1) / kEdge, tz1 - 1);
     for (int tz = az; tz <= bz; ++tz) {
-        const int lz = tz * kTile, hz = min(lz + kTile - 1, g.SZ - 1);
+        const int lz = tz * kEdge, hz = min(lz + kEdge - 1, g.SZ - 1);
         const int dz = z < lz ? lz - z : (z > hz ? z - hz : 0);
         for (int tx = ax; tx <= bx; ++tx) {
-            const int lx = tx * kTile, hx = min(lx + kTile - 1, g.SX - 1);
+            const int lx = tx * kEdge, hx = min(lx + kEdge - 1, g.SX - 1);
             const int dx = x < lx ? lx - x : (x > hx ? x - hx : 0);
             const int dxz = dx * dx + dz * dz;
             if (static_cast<uint32_t>(dxz) > R) continue;
             for (int ty = ay; ty <= by; ++ty) {
-                const int ly = ty * kTile, hy = min(ly + kTile - 1, g.SY - 1);
+                const int ly = ty * kEdge, hy = min(ly + kEdge - 1, g.SY - 1);
                 const int dy = y < ly ? ly - y : (y > hy ? y - hy : 0);
                 if (static_cast<uint32_t>(dxz + dy * dy) > R) continue;
                 f(t.id(tx, ty, tz));
@@ -199,8 +205,9 @@ __global__ void balls_radii(const uint32_t* __restrict__ edt2, const uint32_t* _
 constexpr uint32_t kFloorR2 = 37;  // half the diagonal between a tile's corner voxels: 3 * 3.5^2 = 36.75
 
 __global__ void balls_tile_floor(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
-                                 size_t nc, Grid g, Tiles t, unsigned long long* __restrict__ floor) {
-    PMA_GRID_STRIDE(i, nc) {
+                                 size_t nc, size_t step, Grid g, Tiles t, unsigned long long* __restrict__ floor) {
+    PMA_GRID_STRIDE(k, (nc + step - 1) / step) {
+        const size_t i = k * step;
         const uint32_t R = max_edt2 - down[i];
         if (R < kFloorR2) continue;
         int x, y, z;
@@ -229,60 +236,90 @@ __global__ void balls_tile_floor(const uint32_t* __restrict__ cand, const uint32
     }
 }
 
-struct CountTile {
-    const unsigned long long* floor;
-    unsigned int* tcount;
+// Floor of a group: the least of its tiles' floors, what every voxel of the group's winner's key is at least.
+__global__ void balls_group_floor(const unsigned long long* __restrict__ floor, Tiles t, Tiles gt, size_t ngroups,
+                                  unsigned long long* __restrict__ gfloor) {
+    PMA_GRID_STRIDE(i, ngroups) {
+        const int gy = static_cast<int>(i % gt.TY);
+        const size_t rest = i / gt.TY;
+        const int gx = static_cast<int>(rest % gt.TX), gz = static_cast<int>(rest / gt.TX);
+        unsigned long long least = ~0ull;
+        for (int tz = gz * kGroup; tz < min(gz * kGroup + kGroup, t.TZ); ++tz)
+            for (int tx = gx * kGroup; tx < min(gx * kGroup + kGroup, t.TX); ++tx)
+                for (int ty = gy * kGroup; ty < min(gy * kGroup + kGroup, t.TY); ++ty) least = min(least, floor[t.id(tx, ty, tz)]);
+        gfloor[i] = least;
+    }
+}
+
+// Adds one to *counter and returns what it held. Where the lanes' centres are neighbours (kNear) most
+// of them are at the same counter, and one lane adds for all.
+template <bool kNear>
+__device__ __forceinline__ unsigned int add_one(unsigned int* counter, size_t id) {
+    if (!kNear) return atomicAdd(counter, 1u);
+    const unsigned lane = threadIdx.x & 31, peers = __match_any_sync(__activemask(), static_cast<unsigned int>(id));
+    const int leader = __ffs(peers) - 1;
+    unsigned int at = 0;
+    if (static_cast<int>(lane) == leader) at = atomicAdd(counter, __popc(peers));
+    return __shfl_sync(peers, at, leader) + __popc(peers & ((1u << lane) - 1u));
+}
+
+template <bool kNear>
+struct CountGroup {
+    const unsigned long long* gfloor;
+    unsigned int* gcount;
     unsigned long long key;
-    __device__ void operator()(size_t tid) const {
-        if (key >= __ldg(floor + tid)) atomicAdd(&tcount[tid], 1u);
+    __device__ void operator()(size_t id) const {
+        if (key >= __ldg(gfloor + id)) add_one<kNear>(&gcount[id], id);
     }
 };
 
-struct FillTile {
-    const unsigned long long* floor;
-    const unsigned long long* toff;
+template <bool kNear>
+struct FillGroup {
+    const unsigned long long* gfloor;
+    const unsigned long long* goff;
     unsigned long long base;
-    unsigned int* tcursor;
-    unsigned long long* entries;
+    unsigned int* gcursor;
+    unsigned long long* groups;
     unsigned long long key;
-    __device__ void operator()(size_t tid) const {
-        if (key < __ldg(floor + tid)) return;
-        const unsigned pos = atomicAdd(&tcursor[tid], 1u);
-        entries[toff[tid] - base + pos] = key;
+    __device__ void operator()(size_t id) const {
+        if (key < __ldg(gfloor + id)) return;
+        const unsigned int at = add_one<kNear>(&gcursor[id], id);
+        groups[goff[id] - base + at] = key;
     }
 };
 
-__global__ void balls_tile_count(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
-                                 size_t nc, Grid g, Tiles t, const unsigned long long* __restrict__ floor,
-                                 unsigned int* __restrict__ tcount) {
+template <bool kNear>
+__global__ void balls_group_count(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
+                                  size_t nc, Grid g, Tiles gt, const unsigned long long* __restrict__ gfloor,
+                                  unsigned int* __restrict__ gcount) {
     PMA_GRID_STRIDE(i, nc) {
         int x, y, z;
         g.coords(cand[i], x, y, z);
         const uint32_t R = max_edt2 - down[i];
-        for_each_tile(g, t, x, y, z, R, 0, t.TZ, CountTile{floor, tcount, ball_key(g, x, y, z, R)});
+        for_each_group(g, gt, x, y, z, R, 0, gt.TZ, CountGroup<kNear>{gfloor, gcount, ball_key(g, x, y, z, R)});
     }
 }
 
-__global__ void balls_tile_fill(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
-                                size_t nc, Grid g, Tiles t, int tz0, int tz1,
-                                const unsigned long long* __restrict__ floor,
-                                const unsigned long long* __restrict__ toff, unsigned long long base,
-                                unsigned int* __restrict__ tcursor, unsigned long long* __restrict__ entries) {
+template <bool kNear>
+__global__ void balls_group_fill(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
+                                 size_t nc, Grid g, Tiles gt, int gz0, int gz1,
+                                 const unsigned long long* __restrict__ gfloor,
+                                 const unsigned long long* __restrict__ goff, unsigned long long base,
+                                 unsigned int* __restrict__ gcursor, unsigned long long* __restrict__ groups) {
     PMA_GRID_STRIDE(i, nc) {
         int x, y, z;
         g.coords(cand[i], x, y, z);
         const uint32_t R = max_edt2 - down[i];
-        for_each_tile(g, t, x, y, z, R, tz0, tz1,
-                      FillTile{floor, toff, base, tcursor, entries, ball_key(g, x, y, z, R)});
+        for_each_group(g, gt, x, y, z, R, gz0, gz1,
+                       FillGroup<kNear>{gfloor, goff, base, gcursor, groups, ball_key(g, x, y, z, R)});
     }
 }
 
-__device__ __forceinline__ int4 decode_key(unsigned long long key, Grid g) {
+__device__ __forceinline__ int4 decode_key(unsigned long long key, Grid g, FastDiv fsz) {
     const uint32_t lex = 0xFFFFFFFFu - static_cast<uint32_t>(key);
-    const uint32_t syz = static_cast<uint32_t>(g.SY) * g.SZ;
-    const uint32_t x = lex / syz, rem = lex % syz;
-    return make_int4(static_cast<int>(x), static_cast<int>(rem / g.SZ), static_cast<int>(rem % g.SZ),
-                     static_cast<int>(key >> 32));
+    const uint32_t xy = fsz.div(lex), x = g.fy.div(xy);
+    return make_int4(static_cast<int>(x), static_cast<int>(xy - x * static_cast<uint32_t>(g.SY)),
+                     static_cast<int>(lex - xy * static_cast<uint32_t>(g.SZ)), static_cast<int>(key >> 32));
 }
 
 // 32-bit arithmetic while every offset is below 2^15 (the squared sum then fits), 64-bit
@@ -315,7 +352,90 @@ __device__ __forceinline__ unsigned int fold_x(unsigned int m) {
     return ((m & 0xFu) ? 1u : 0u) | ((m & 0xF0u) ? 2u : 0u) | ((m & 0xF00u) ? 4u : 0u) | ((m & 0xF000u) ? 8u : 0u);
 }
 
-// One CTA per tile of the z-range starting at tz0: winner key of each voxel.
+constexpr int kSub = kGroup * kGroup * kGroup;  // tiles of a group
+
+// Tile `sub` of a group, which may lie outside the volume.
+__device__ __forceinline__ void tile_of(Tiles gt, size_t group, int sub, int& tx, int& ty, int& tz) {
+    const size_t rest = group / gt.TY;
+    ty = static_cast<int>(group % gt.TY) * kGroup + sub % kGroup;
+    tx = static_cast<int>(rest % gt.TX) * kGroup + sub / kGroup % kGroup;
+    tz = static_cast<int>(rest / gt.TX) * kGroup + sub / (kGroup * kGroup);
+}
+
+// Where a tile's list starts: each tile of a group has room for the whole group's list.
+__device__ __forceinline__ unsigned long long tile_list(unsigned long long group_at, unsigned int group_count, int sub) {
+    return group_at * kSub + static_cast<unsigned long long>(group_count) * sub;
+}
+
+// Splits each group's list into its tiles' lists: the entries that reach the tile and are not below
+// its floor. One CTA per group; an entry is decoded once and tested against the eight tiles, a
+// warp takes its places in all eight lists with one atomic instruction in shared memory.
+constexpr int kSplitThreads = 256;
+
+__global__ void __launch_bounds__(kSplitThreads) balls_split(Grid g, FastDiv fsz, Tiles t, Tiles gt, int gz0,
+                                                             const unsigned long long* __restrict__ floor,
+                                                             const unsigned int* __restrict__ gcount,
+                                                             const unsigned long long* __restrict__ goff, unsigned long long base,
+                                                             unsigned long long tile_base,
+                                                             const unsigned long long* __restrict__ groups,
+                                                             unsigned long long* __restrict__ entries,
+                                                             unsigned int* __restrict__ tcount) {
+    static_assert(kGroup == 2, "two tiles an axis");
+    __shared__ unsigned int s_n[kSub];
+    __shared__ unsigned long long s_floor[kSub];
+    const size_t group = static_cast<size_t>(gz0) * gt.TX * gt.TY + blockIdx.x;
+    const unsigned lane = threadIdx.x & 31;
+    int tx, ty, tz;
+    if (threadIdx.x < kSub) {
+        tile_of(gt, group, threadIdx.x, tx, ty, tz);
+        s_n[threadIdx.x] = 0;
+        s_floor[threadIdx.x] = ty < t.TY && tx < t.TX && tz < t.TZ ? floor[t.id(tx, ty, tz)] : ~0ull;  // no tile: nothing
+    }
+    tile_of(gt, group, 0, tx, ty, tz);
+    __syncthreads();
+    const unsigned int L = gcount[group];
+    const unsigned long long* list = groups + (goff[group] - base);
+    unsigned long long* out = entries + tile_list(goff[group] - tile_base, L, 0);
+    // voxels a ball must reach along an axis, from the tile's first to its last
+    auto reach = [](int c, int tile, int size) {
+        const int lo = tile * kTile, hi = min(lo + kTile, size) - 1;
+        return max(max(lo - c, c - hi), 0);
+    };
+    for (unsigned int i0 = 0; i0 < L; i0 += kSplitThreads) {
+        const unsigned int i = i0 + threadIdx.x;
+        const unsigned long long key = i < L ? list[i] : 0ull;
+        unsigned int to = 0;  // tiles that take the entry
+        if (i < L) {
+            const int4 c = decode_key(key, g, fsz);
+            int dx[kGroup], dy[kGroup], dz[kGroup];
+#pragma unroll
+            for (int k = 0; k < kGroup; ++k) {
+                dx[k] = reach(c.x, tx + k, g.SX);
+                dy[k] = reach(c.y, ty + k, g.SY);
+                dz[k] = reach(c.z, tz + k, g.SZ);
+            }
+#pragma unroll
+            for (int sub = 0; sub < kSub; ++sub)
+                if (key >= s_floor[sub] && covers(make_int4(dx[sub / 2 % 2], dy[sub % 2], dz[sub / 4], c.w), 0, 0, 0)) to |= 1u << sub;
+        }
+        unsigned int mine = 0, n = 0;  // the lanes that go to tile `lane`
+#pragma unroll
+        for (int sub = 0; sub < kSub; ++sub) {
+            const unsigned int m = __ballot_sync(0xFFFFFFFFu, (to >> sub) & 1u);
+            if (lane == static_cast<unsigned>(sub)) mine = m;
+        }
+        if (lane < kSub && mine) n = atomicAdd(&s_n[lane], __popc(mine));
+#pragma unroll
+        for (int sub = 0; sub < kSub; ++sub) {
+            const unsigned int m = __shfl_sync(0xFFFFFFFFu, mine, sub), from = __shfl_sync(0xFFFFFFFFu, n, sub);
+            if ((to >> sub) & 1u) out[static_cast<unsigned long long>(L) * sub + from + __popc(m & ((1u << lane) - 1u))] = key;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kSub) tcount[static_cast<size_t>(blockIdx.x) * kSub + threadIdx.x] = s_n[threadIdx.x];
+}
+
+// One CTA per tile of the groups of the z-range starting at gz0: winner key of each voxel.
 //
 // The tile's list is taken in chunks of up to kListCap entries. Each chunk is decoded into
 // shared memory ordered by radius, largest first (a counting sort on r^2 when the chunk's r^2
@@ -328,19 +448,18 @@ __device__ __forceinline__ unsigned int fold_x(unsigned int m) {
 // the whole list, i.e. the covering centre of largest key.
 constexpr int kSortBins = 2048;
 
-__global__ void __launch_bounds__(kTileVox, 3) balls_tile_gather(
-    const uint32_t* __restrict__ edt2, Grid g, Tiles t, int tz0,
-    const unsigned int* __restrict__ tcount, const unsigned long long* __restrict__ toff,
-    unsigned long long base, const unsigned long long* __restrict__ entries,
+__global__ void __launch_bounds__(kTileVox, 4) balls_tile_gather(
+    const uint32_t* __restrict__ edt2, Grid g, FastDiv fsz, Tiles t, Tiles gt, int gz0,
+    const unsigned int* __restrict__ tcount, const unsigned int* __restrict__ gcount,
+    const unsigned long long* __restrict__ goff, unsigned long long tile_base, const unsigned long long* __restrict__ entries,
     unsigned long long* __restrict__ keys, unsigned int* __restrict__ err) {
     __shared__ int4 s_pos[kListCap];
     __shared__ unsigned int s_bin[kSortBins];
     __shared__ unsigned int s_rmin, s_rmax, s_wsum[kTileVox / 32];
-    const size_t tile = static_cast<size_t>(tz0) * t.TX * t.TY + blockIdx.x;
-    const int ty = static_cast<int>(tile % t.TY);
-    const size_t rest = tile / t.TY;
-    const int tx = static_cast<int>(rest % t.TX);
-    const int tz = static_cast<int>(rest / t.TX);
+    const size_t group = static_cast<size_t>(gz0) * gt.TX * gt.TY + blockIdx.x / kSub;
+    int tx, ty, tz;
+    tile_of(gt, group, blockIdx.x % kSub, tx, ty, tz);
+    if (ty >= t.TY || tx >= t.TX || tz >= t.TZ) return;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // a warp covers a box of 2 x 4 x 4 voxels (z, x, y)
     const int by0 = ty * kTile + (warp & 1) * 4, bx0 = tx * kTile + ((warp >> 1) & 1) * 4, bz0 = tz * kTile + (warp >> 2) * 2;
@@ -348,12 +467,12 @@ __global__ void __launch_bounds__(kTileVox, 3) balls_tile_gather(
     const bool inside = vx < g.SX && vy < g.SY && vz < g.SZ;
     const size_t v = inside ? g.idx(vx, vy, vz) : 0;
     const bool void_voxel = inside && edt2[v] != 0;
-    const unsigned int L = tcount[tile];
-    const unsigned long long* list = entries + (toff[tile] - base);
+    const unsigned int L = tcount[blockIdx.x];
+    const unsigned long long* list = entries + tile_list(goff[group] - tile_base, gcount[group], blockIdx.x % kSub);
     unsigned long long best = void_voxel ? 0ull : ~0ull;
     for (unsigned int c0 = 0; c0 < L; c0 += kListCap) {
         const unsigned int m = min(static_cast<unsigned int>(kListCap), L - c0);
-        // radius span of the chunk; up to four entries per thread stay in registers
+        // radius span of the chunk; the entries stay in registers
         constexpr int kPer = kListCap / kTileVox;
         unsigned long long k[kPer];
         if (threadIdx.x == 0) {
@@ -433,7 +552,7 @@ __global__ void __launch_bounds__(kTileVox, 3) balls_tile_gather(
             const unsigned int i = threadIdx.x + q * kTileVox;
             if (i < m) {
                 const unsigned int at = sorted ? s_bin[r_hi - static_cast<unsigned int>(k[q] >> 32)] + rank[q] : i;
-                s_pos[at] = decode_key(k[q], g);
+                s_pos[at] = decode_key(k[q], g, fsz);
             }
         }
         __syncthreads();
@@ -534,12 +653,12 @@ T* buf(pma_ctx* ctx, const char* tag, size_t count) {
     return static_cast<T*>(ctx->scratch(tag, std::max<size_t>(count, 1) * sizeof(T)));
 }
 
-// Tile counts as 64-bit values, with a zero past the end (the scan then gives the total).
+// Group counts as 64-bit values, with a zero past the end (the scan then gives the total).
 __global__ void widen_counts(const unsigned int* __restrict__ c, size_t n, unsigned long long* __restrict__ out) {
     PMA_GRID_STRIDE(i, n + 1) out[i] = i < n ? c[i] : 0ull;
 }
 
-// Offsets of the first tile of each z-slab (and the total at tz).
+// Offsets of the first group of each z-slab (and the total at tz).
 __global__ void slab_offsets(const unsigned long long* __restrict__ toff, size_t per_z, int tz,
                              unsigned long long* __restrict__ zoff) {
     const int z = blockIdx.x * blockDim.x + threadIdx.x;
@@ -594,11 +713,14 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
     // later chunks hold smaller balls and are mostly skipped. Below kSortCentres the sort's launches cost
     // more than it saves.
     constexpr int64_t kSortCentres = 1 << 18;
+    // of centres in that order every fourth serves for the floors, which are near those of all
+    constexpr size_t kFloorStep = 4;
+    const bool sorted = nc >= kSortCentres;
     uint32_t* down = buf<uint32_t>(ctx, "balls.down", nc);
     if (nc) {
         balls_radii<<<grid_for(ctx, nc), 256, 0, s>>>(edt2, cand, nc, max_edt2, down);
         ctx->check_launch("balls_radii");
-        if (nc >= kSortCentres) {
+        if (sorted) {
             KernelTimer kt(ctx, "balls_sort");
             int bits = 1;
             while (bits < 32 && (max_edt2 >> bits) != 0) ++bits;
@@ -609,61 +731,87 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
             cand = cand2;
         }
     }
-    // Tile lists: counts, 64-bit offsets (host scan), then fill + gather by tile z-ranges
-    // whose entries fit the memory budget.
+    // Lists: counts, 64-bit offsets, then fill, split and gather by z-ranges whose entries fit the
+    // memory budget. One centre a thread and no strides: the lists keep the order of the centres roughly.
     Tiles t{(d.sx + kTile - 1) / kTile, (d.sy + kTile - 1) / kTile, (d.sz + kTile - 1) / kTile};
-    const size_t per_z = static_cast<size_t>(t.TX) * t.TY;
-    const size_t ntiles = per_z * t.TZ;
-    unsigned int* tcount = buf<unsigned int>(ctx, "balls.tcount", ntiles);
-    unsigned int* tcursor = buf<unsigned int>(ctx, "balls.tcursor", ntiles);
-    auto* toff = buf<unsigned long long>(ctx, "balls.toff", ntiles + 1);
+    const size_t ntiles = static_cast<size_t>(t.TX) * t.TY * t.TZ;
+    const Tiles gt{(t.TX + kGroup - 1) / kGroup, (t.TY + kGroup - 1) / kGroup, (t.TZ + kGroup - 1) / kGroup};
+    const size_t per_z = static_cast<size_t>(gt.TX) * gt.TY;
+    const size_t ngroups = per_z * gt.TZ;
+    // Few groups: dozens of the threads in flight are at one counter. Fill of a 128^3 union (512 groups) 0.26 ms
+    // without add_one's grouping, 0.11 with it; of 32 thousand groups (512^3) 0.84 and 0.99.
+    const bool near = ngroups < 8192;
+    unsigned int* gcount = buf<unsigned int>(ctx, "balls.gcount", ngroups);
+    unsigned int* gcursor = buf<unsigned int>(ctx, "balls.gcursor", ngroups);
+    auto* goff = buf<unsigned long long>(ctx, "balls.goff", ngroups + 1);
     auto* floor = buf<unsigned long long>(ctx, "balls.floor", ntiles);
-    PMA_CUDA(cudaMemsetAsync(tcount, 0, ntiles * 4, s));
-    PMA_CUDA(cudaMemsetAsync(tcursor, 0, ntiles * 4, s));
+    auto* gfloor = buf<unsigned long long>(ctx, "balls.gfloor", ngroups);
+    PMA_CUDA(cudaMemsetAsync(gcount, 0, ngroups * 4, s));
+    PMA_CUDA(cudaMemsetAsync(gcursor, 0, ngroups * 4, s));
     PMA_CUDA(cudaMemsetAsync(floor, 0, ntiles * 8, s));
     if (nc) {
         KernelTimer kt(ctx, "balls_tile_count");
-        balls_tile_floor<<<grid_for(ctx, nc), 256, 0, s>>>(cand, down, max_edt2, nc, g, t, floor);
+        const size_t step = sorted ? kFloorStep : 1;
+        balls_tile_floor<<<div_up((nc + step - 1) / step, 256), 256, 0, s>>>(cand, down, max_edt2, nc, step, g, t, floor);
         ctx->check_launch("balls_tile_floor");
-        balls_tile_count<<<grid_for(ctx, nc), 256, 0, s>>>(cand, down, max_edt2, nc, g, t, floor, tcount);
-        ctx->check_launch("balls_tile_count");
+        balls_group_floor<<<grid_for(ctx, ngroups), 256, 0, s>>>(floor, t, gt, ngroups, gfloor);
+        ctx->check_launch("balls_group_floor");
+        (near ? balls_group_count<true> : balls_group_count<false>)<<<div_up(nc, 256), 256, 0, s>>>(cand, down, max_edt2, nc, g, gt, gfloor, gcount);
+        ctx->check_launch("balls_group_count");
     }
-    // 64-bit list offsets by a device scan; the host reads back only the offsets at the tile
-    // z-slab boundaries, which choose the slabs that fit the memory budget
-    auto* tc64 = buf<unsigned long long>(ctx, "balls.tc64", ntiles + 1);
-    widen_counts<<<grid_for(ctx, ntiles + 1), 256, 0, s>>>(tcount, ntiles, tc64);
+    // 64-bit list offsets by a device scan; the host reads back only the offsets at the z-slab
+    // boundaries, which choose the slabs that fit the memory budget
+    auto* tc64 = buf<unsigned long long>(ctx, "balls.tc64", ngroups + 1);
+    widen_counts<<<grid_for(ctx, ngroups + 1), 256, 0, s>>>(gcount, ngroups, tc64);
     ctx->check_launch("widen_counts");
-    exclusive_sum(ctx, tc64, toff, static_cast<int64_t>(ntiles + 1));
-    auto* zoff = buf<unsigned long long>(ctx, "balls.zoff", t.TZ + 1);
-    slab_offsets<<<div_up(t.TZ + 1, 256), 256, 0, s>>>(toff, per_z, t.TZ, zoff);
+    exclusive_sum(ctx, tc64, goff, static_cast<int64_t>(ngroups + 1));
+    auto* zoff = buf<unsigned long long>(ctx, "balls.zoff", gt.TZ + 1);
+    slab_offsets<<<div_up(gt.TZ + 1, 256), 256, 0, s>>>(goff, per_z, gt.TZ, zoff);
     ctx->check_launch("slab_offsets");
-    std::vector<unsigned long long> hz(t.TZ + 1);
-    PMA_CUDA(cudaMemcpyAsync(hz.data(), zoff, (t.TZ + 1) * 8ull, cudaMemcpyDeviceToHost, s));
+    std::vector<unsigned long long> hz(gt.TZ + 1);
+    PMA_CUDA(cudaMemcpyAsync(hz.data(), zoff, (gt.TZ + 1) * 8ull, cudaMemcpyDeviceToHost, s));
     ctx->sync();
-    auto ho_at = [&](int z) { return hz[z]; };  // offset of the first tile of slab z
+    auto ho_at = [&](int z) { return hz[z]; };  // offset of the first group of slab z
     size_t free_b = 0, total_b = 0;
     PMA_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const unsigned long long budget = std::max<unsigned long long>(
-        1ull << 20, std::min<unsigned long long>(free_b / 3, 32ull << 30) / 8);
-    for (int z0 = 0; z0 < t.TZ;) {
+    // group lists by z-ranges that fit the memory budget, and of these the tiles' lists (with room for
+    // every entry of the group in each of its tiles) by z-ranges that fit theirs
+    auto upto = [&](int z0, int end, unsigned long long budget) {
         int z1 = z0 + 1;
-        while (z1 < t.TZ && ho_at(z1 + 1) - ho_at(z0) <= budget) ++z1;
+        while (z1 < end && ho_at(z1 + 1) - ho_at(z0) <= budget) ++z1;
+        return z1;
+    };
+    const unsigned long long budget = std::max<unsigned long long>(1ull << 20, std::min<unsigned long long>(free_b / 6, 32ull << 30) / 8);
+    const unsigned long long tile_budget =
+        std::max<unsigned long long>(1ull << 17, std::min<unsigned long long>(free_b / 6, 8ull << 30) / (8 * kSub));
+    const FastDiv fsz(static_cast<uint32_t>(d.sz));
+    for (int z0 = 0, z1 = 0; z0 < gt.TZ; z0 = z1) {
+        z1 = upto(z0, gt.TZ, budget);
         const unsigned long long base = ho_at(z0);
-        const unsigned long long cnt = ho_at(z1) - base;
-        auto* entries = buf<unsigned long long>(ctx, "balls.entries", cnt);
+        auto* groups = buf<unsigned long long>(ctx, "balls.groups", ho_at(z1) - base);
         if (nc) {
             KernelTimer kt(ctx, "balls_tile_fill");
-            balls_tile_fill<<<grid_for(ctx, nc), 256, 0, s>>>(cand, down, max_edt2, nc, g, t, z0, z1, floor, toff,
-                                                              base, tcursor, entries);
-            ctx->check_launch("balls_tile_fill");
+            (near ? balls_group_fill<true> : balls_group_fill<false>)<<<div_up(nc, 256), 256, 0, s>>>(
+                cand, down, max_edt2, nc, g, gt, z0, z1, gfloor, goff, base, gcursor, groups);
+            ctx->check_launch("balls_group_fill");
         }
-        {
+        for (int y0 = z0, y1 = z0; y0 < z1; y0 = y1) {
+            y1 = upto(y0, z1, tile_budget);
+            const unsigned long long tile_base = ho_at(y0);
+            const unsigned slab = static_cast<unsigned>((y1 - y0) * per_z);
+            auto* entries = buf<unsigned long long>(ctx, "balls.entries", (ho_at(y1) - tile_base) * kSub);
+            auto* tcount = buf<unsigned int>(ctx, "balls.tcount", static_cast<size_t>(slab) * kSub);
+            {
+                KernelTimer kt(ctx, "balls_split");
+                balls_split<<<slab, kSplitThreads, 0, s>>>(g, fsz, t, gt, y0, floor, gcount, goff, base, tile_base, groups, entries,
+                                                           tcount);
+                ctx->check_launch("balls_split");
+            }
             KernelTimer kt(ctx, "balls_tile_gather");
-            balls_tile_gather<<<static_cast<unsigned>((z1 - z0) * per_z), kTileVox, 0, s>>>(
-                edt2, g, t, z0, tcount, toff, base, entries, keys, err);
+            balls_tile_gather<<<slab * kSub, kTileVox, 0, s>>>(edt2, g, fsz, t, gt, y0, tcount, gcount, goff, tile_base, entries,
+                                                               keys, err);
             ctx->check_launch("balls_tile_gather");
         }
-        z0 = z1;
     }
     balls_unpack<<<G, 256, 0, s>>>(keys, g, n, crad2, cx, cy, cz, mask);
     ctx->check_launch("balls_unpack");
