@@ -215,85 +215,171 @@ __global__ void uf_hook(const uint32_t* __restrict__ crad, Grid g, size_t n, int
     }
 }
 
-// Large volumes, after the pointer jumps: almost every voxel points at its initial tree's
-// root, so a neighbour pair of equal crad whose parents differ is the rare case. uf_pairs
-// records those parent pairs (de-duplicated within the block's voxels) instead of walking to
-// the roots in line, and uf_union_pairs unions them, one thread per pair, so that the root
-// walks (into arrays far larger than L2) run in parallel rather than one neighbour after
-// another. The partition and its roots are the same: each plateau's root is its smallest
-// voxel index, whatever the union order.
-constexpr int kPairTable = 2048;
+// Pairs of neighbouring voxels' ids, each pair of ids once per tile, as 64-bit keys; count receives how many,
+// also those beyond cap (not written). Each unordered pair of voxels is looked at from the voxel of smaller index
+// (13 forward offsets, in 5 rows along y). A row is read once, coalesced, by a warp of 32 voxels along y: the
+// voxel's neighbours at y - 1 and y + 1 come from the lanes beside it, and a slice's rows serve the next slice.
+//
+// kUnion: id is the union-find's parent. After the pointer jumps almost every voxel points at its initial tree's
+// root, so that a pair of equal crad with different parents is the rare case; uf_union_pairs then unions them, one
+// thread a pair, instead of one walk to the roots after the other. The partition and its roots are the same:
+// each plateau's root is its smallest voxel index, whatever the order of the unions.
+// Else id is the plateau: edges (lower-radius plateau, higher-radius one), where crad differs.
+//
+// Neighbouring voxels mostly report the same pairs, and plateaus are 3-D blobs. A voxel of the same id as the one
+// before it along y leaves out what that one has seen of a row (all but the neighbour at y + 1), and any voxel the
+// neighbours of its own that follow an equal one. What is left is queued by warp and put, 32 at a time, into
+// a set in shared memory over the tile of 4 (z) x 8 (x) x 32 (y) voxels; the set is written out at the tile's end
+// with one atomic. A key that finds no slot in eight probes is written at once: the sort and unique (the unions)
+// that follow take copies.
+//
+// What bounds it: instructions. 512^3 random field: edges 8.25 -> 4.3 ms, pairs and unions 5.8 -> 2.5; one thread
+// a voxel with 13 look-ups of its own took 1425 instructions a warp for the edges alone, and an atomic on one
+// counter per warp and slice. (Reading a slot before the compare-and-swap: 9.7 ms.)
+constexpr int kTileY = 32, kTileX = 8, kTileZ = 4;  // a warp covers a row of the tile, one slice after another
+constexpr int kPairThreads = 32 * kTileX;
 
-__global__ void uf_pairs(const uint32_t* __restrict__ crad, Grid g, size_t n, int d3q7,
-                         const uint32_t* __restrict__ parent, unsigned long long* __restrict__ pairs,
-                         unsigned long long cap, unsigned long long* __restrict__ count) {
-    __shared__ unsigned long long table[kPairTable];
+struct PairRow {  // crad (0: solid or outside) and id at y - 1, y and y + 1 of a lane
+    uint32_t c[3], i[3];
+};
+
+__device__ __forceinline__ PairRow pair_row(const uint32_t* __restrict__ id, const uint32_t* __restrict__ crad, const Grid& g, int x, int y,
+                                            int z) {
     const unsigned lane = threadIdx.x & 31;
-    // block-uniform trip count: whole blocks reach the barriers and warps the placement below
-    for (size_t base = static_cast<size_t>(blockIdx.x) * blockDim.x; base < n;
-         base += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t v = base + threadIdx.x;
-        const uint32_t r = v < n ? crad[v] : 0u;
-        // shared-memory set of the block's pairs: keep the first copy of each
-        for (int i = threadIdx.x; i < kPairTable; i += blockDim.x) table[i] = ~0ull;
-        __syncthreads();
-        unsigned long long keys[13];
-        int kept = 0;
-        if (r) {
-            int x, y, z;
-            g.coords(v, x, y, z);
-            const uint32_t rv = parent[v];
-            uint32_t seen[13];
-            int ns = 0;
-            for (int k = 0; k < 13; ++k) {  // the 13 forward offsets, as in uf_hook
-                int dx, dy, dz;
-                if (k < 4) {
-                    dz = 0;
-                    dx = (k == 0) ? 0 : 1;
-                    dy = (k == 0) ? 1 : k - 2;
-                } else {
-                    dz = 1;
-                    dx = (k - 4) / 3 - 1;
-                    dy = (k - 4) % 3 - 1;
-                }
-                if (d3q7 && (dx != 0) + (dy != 0) + (dz != 0) > 1) continue;
-                const int nx = x + dx, ny = y + dy, nz = z + dz;
-                if (!g.inside(nx, ny, nz)) continue;
-                const size_t w = g.idx(nx, ny, nz);
-                if (crad[w] != r) continue;
-                const uint32_t pw = parent[w];
-                if (pw == rv) continue;  // already in one tree
-                bool dup = false;
-                for (int i = 0; i < ns; ++i) dup |= seen[i] == pw;
-                if (dup) continue;
-                seen[ns++] = pw;
-                const uint32_t lo = min(rv, pw), hi = max(rv, pw);
-                const unsigned long long key = (static_cast<unsigned long long>(lo) << 32) | hi;
-                unsigned h = static_cast<unsigned>((key * 0x9E3779B97F4A7C15ull) >> 40) & (kPairTable - 1);
-                bool fresh = true;
-                for (int probe = 0; probe < 8; ++probe, h = (h + 1) & (kPairTable - 1)) {
-                    const unsigned long long prev = atomicCAS(&table[h], ~0ull, key);
-                    if (prev == ~0ull) break;
-                    if (prev == key) {
-                        fresh = false;
-                        break;
+    PairRow r;
+    r.c[1] = 0;
+    r.i[1] = kNone;
+    uint32_t ce = 0, ie = kNone;  // past the warp's row, at lanes 0 and 31
+    if (x >= 0 && x < g.SX && z < g.SZ) {  // the same for the warp
+        const size_t at = g.idx(x, y, z);
+        if (y < g.SY) {
+            r.c[1] = crad[at];
+            r.i[1] = id[at];
+        }
+        if ((lane == 0 && y > 0) || (lane == 31 && y + 1 < g.SY)) {
+            const size_t e = lane == 0 ? at - 1 : at + 1;
+            ce = crad[e];
+            ie = id[e];
+        }
+    }
+    r.c[0] = __shfl_up_sync(0xFFFFFFFFu, r.c[1], 1);
+    r.i[0] = __shfl_up_sync(0xFFFFFFFFu, r.i[1], 1);
+    r.c[2] = __shfl_down_sync(0xFFFFFFFFu, r.c[1], 1);
+    r.i[2] = __shfl_down_sync(0xFFFFFFFFu, r.i[1], 1);
+    if (lane == 0) {
+        r.c[0] = ce;
+        r.i[0] = ie;
+    }
+    if (lane == 31) {
+        r.c[2] = ce;
+        r.i[2] = ie;
+    }
+    return r;
+}
+
+template <bool kUnion>
+__global__ void __launch_bounds__(kPairThreads, 5) voxel_pairs(const uint32_t* __restrict__ id, const uint32_t* __restrict__ crad, Grid g,
+                                                               int d3q7, int sb, unsigned long long* __restrict__ count,
+                                                               unsigned long long* __restrict__ out, unsigned long long cap) {
+    constexpr int kTable = kUnion ? 1024 : 2048, kPer = kTable / kPairThreads;
+    __shared__ unsigned long long table[kTable], s_queue[kTileX][64], s_base;
+    __shared__ unsigned s_sum[kTileX];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    const unsigned nty = (g.SY + kTileY - 1) / kTileY, ntx = (g.SX + kTileX - 1) / kTileX;
+    const size_t ntiles = static_cast<size_t>(nty) * ntx * ((g.SZ + kTileZ - 1) / kTileZ);
+    unsigned long long* queue = s_queue[warp];
+    auto insert = [&](unsigned long long key) {
+        unsigned h = static_cast<unsigned>((key * 0x9E3779B97F4A7C15ull) >> 40) & (kTable - 1);
+        for (int probe = 0; probe < 8; ++probe, h = (h + 1) & (kTable - 1)) {
+            const unsigned long long prev = atomicCAS(&table[h], ~0ull, key);
+            if (prev == ~0ull || prev == key) return;
+        }
+        const unsigned long long pos = atomicAdd(count, 1ull);
+        if (pos < cap) out[pos] = key;
+    };
+    for (int k = 0; k < kPer; ++k) table[threadIdx.x + k * kPairThreads] = ~0ull;
+    __syncthreads();
+    for (size_t t = blockIdx.x; t < ntiles; t += gridDim.x) {  // block-uniform
+        const int y = static_cast<int>(t % nty) * kTileY + static_cast<int>(lane);
+        const size_t rest = t / nty;
+        const int x = static_cast<int>(rest % ntx) * kTileX + static_cast<int>(warp), z0 = static_cast<int>(rest / ntx) * kTileZ;
+        unsigned head = 0, queued = 0;  // of the warp's queue, a ring of 64
+        if (x < g.SX) {
+            PairRow here = pair_row(id, crad, g, x, y, z0), next = pair_row(id, crad, g, x + 1, y, z0);
+            for (int z = z0; z < min(z0 + kTileZ, g.SZ); ++z) {
+                const uint32_t p = here.i[1], r = here.c[1];
+                const bool as_before = lane > 0 && here.i[0] == p;
+                auto consider = [&](bool see, uint32_t q, uint32_t rq) {
+                    const bool pair = see && r != 0 && (kUnion ? rq == r && q != p : rq != 0 && rq != r);
+                    const unsigned m = __ballot_sync(0xFFFFFFFFu, pair);
+                    if (!m) return;
+                    if (pair) {
+                        unsigned long long key;
+                        if (kUnion) key = (static_cast<unsigned long long>(min(p, q)) << 32) | max(p, q);
+                        else key = rq < r ? (static_cast<unsigned long long>(q) << sb) | p : (static_cast<unsigned long long>(p) << sb) | q;
+                        queue[(head + queued + __popc(m & lt)) & 63] = key;
                     }
-                }
-                if (fresh) keys[kept++] = key;
+                    queued += __popc(m);
+                    if (queued >= 32) {
+                        __syncwarp();
+                        insert(queue[(head + lane) & 63]);
+                        head += 32;
+                        queued -= 32;
+                        __syncwarp();
+                    }
+                };
+                auto row = [&](const PairRow& w) {
+                    if (d3q7) {
+                        consider(!(as_before && w.i[1] == w.i[0]), w.i[1], w.c[1]);
+                    } else {
+                        consider(!as_before, w.i[0], w.c[0]);
+                        consider(!as_before && w.i[1] != w.i[0], w.i[1], w.c[1]);
+                        consider(w.i[2] != w.i[1], w.i[2], w.c[2]);
+                    }
+                };
+                consider(true, here.i[2], here.c[2]);
+                row(next);
+                if (!d3q7) row(pair_row(id, crad, g, x - 1, y, z + 1));
+                here = pair_row(id, crad, g, x, y, z + 1);
+                row(here);
+                next = pair_row(id, crad, g, x + 1, y, z + 1);
+                if (!d3q7) row(next);
             }
+            __syncwarp();
+            if (lane < queued) insert(queue[(head + lane) & 63]);
         }
         __syncthreads();
-        // one atomic per warp; lanes place their pairs by a warp prefix sum
-        unsigned incl = static_cast<unsigned>(kept);
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= static_cast<unsigned>(o)) incl += t;
+        // the set, emptied for the next tile
+        unsigned long long keys[kPer];
+        unsigned kept = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            keys[k] = table[threadIdx.x + k * kPairThreads];
+            table[threadIdx.x + k * kPairThreads] = ~0ull;
+            kept += keys[k] != ~0ull ? 1u : 0u;
         }
-        unsigned long long pos = 0;
-        if (lane == 31 && incl) pos = atomicAdd(count, static_cast<unsigned long long>(incl));
-        pos = __shfl_sync(0xFFFFFFFFu, pos, 31) + (incl - static_cast<unsigned>(kept));
-        for (int i = 0; i < kept; ++i)
-            if (pos + i < cap) pairs[pos + i] = keys[i];
+        unsigned incl = kept;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t2 = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= static_cast<unsigned>(o)) incl += t2;
+        }
+        if (lane == 31) s_sum[warp] = incl;
+        __syncthreads();
+        unsigned before = 0, total = 0;
+#pragma unroll
+        for (unsigned w = 0; w < kTileX; ++w) {
+            before += w < warp ? s_sum[w] : 0u;
+            total += s_sum[w];
+        }
+        if (threadIdx.x == 0 && total) s_base = atomicAdd(count, static_cast<unsigned long long>(total));
+        __syncthreads();
+        unsigned long long pos = s_base + before + incl - kept;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k)
+            if (keys[k] != ~0ull) {
+                if (pos < cap) out[pos] = keys[k];
+                ++pos;
+            }
     }
 }
 
@@ -380,105 +466,6 @@ __global__ void plateau_stats(const uint32_t* __restrict__ pid, const uint32_t* 
         atomicAdd(&psize[p], static_cast<unsigned>(__popc(peers)));
         if (any_face) pface[p] = 1;
         if (min_rank != kNone) atomicMin(&pminrank[p], min_rank);
-    }
-}
-
-// Plateau edges q -> p (crad strictly decreasing), deduplicated per tile; count receives the
-// number of edges, also those beyond cap (not written). Each unordered voxel pair is visited
-// once, from the voxel of smaller index (the 13 forward offsets), and gives the edge from the
-// pair's higher-radius plateau to the lower one; the keys stay in registers.
-//
-// A block takes tiles of 4 (z) x 8 (x) x 32 (y) voxels: warp w covers row x = w of the tile,
-// lane l the voxel y = l (coalesced), one z slice after another. Neighbouring voxels mostly
-// report the same plateau pairs, and plateaus are 3-D blobs: the first copy of each pair is
-// kept per tile (a shared-memory hash set over the tile's four slices; a pair that finds no free
-// slot is kept too - the sort and unique that follow are exact). At 1024^3 a set over 256
-// consecutive voxels of one row wrote 1.36 G edges for 0.50 G distinct ones.
-constexpr int kEdgeTable = 2048;  // shared-memory pair set of plateau_edges (power of two)
-constexpr int kEdgeTileY = 32, kEdgeTileX = 8, kEdgeTileZ = 4;
-
-__global__ void __launch_bounds__(256, 4) plateau_edges(const uint32_t* __restrict__ pid, const uint32_t* __restrict__ crad,
-                              Grid g, int d3q7, int sb, unsigned long long* __restrict__ count,
-                              unsigned long long* __restrict__ edges, unsigned long long cap) {
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __shared__ unsigned long long table[kEdgeTable];
-    const unsigned nty = (g.SY + kEdgeTileY - 1) / kEdgeTileY, ntx = (g.SX + kEdgeTileX - 1) / kEdgeTileX;
-    const unsigned ntz = (g.SZ + kEdgeTileZ - 1) / kEdgeTileZ;
-    const size_t ntiles = static_cast<size_t>(nty) * ntx * ntz;
-    // block-uniform trip counts, so whole warps reach the warp-wide placement below
-    for (size_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const unsigned ty = static_cast<unsigned>(t % nty);
-        const size_t rest = t / nty;
-        const unsigned tx = static_cast<unsigned>(rest % ntx), tz = static_cast<unsigned>(rest / ntx);
-        for (int i = threadIdx.x; i < kEdgeTable; i += blockDim.x) table[i] = ~0ull;
-        __syncthreads();
-        const int x = static_cast<int>(tx) * kEdgeTileX + static_cast<int>(warp);
-        const int y = static_cast<int>(ty) * kEdgeTileY + static_cast<int>(lane);
-        for (int zs = 0; zs < kEdgeTileZ; ++zs) {
-            const int z = static_cast<int>(tz) * kEdgeTileZ + zs;
-            const bool in = x < g.SX && y < g.SY && z < g.SZ;
-            const size_t v = in ? g.idx(x, y, z) : 0;
-            unsigned long long key[13];
-            bool has[13];
-            const uint32_t p = in ? pid[v] : kNone;
-            const uint32_t r = p != kNone ? crad[v] : 0u;
-#pragma unroll
-            for (int k = 0; k < 13; ++k) {  // the forward offsets, as in uf_hook
-                int dx, dy, dz;
-                if (k < 4) {
-                    dz = 0;
-                    dx = (k == 0) ? 0 : 1;
-                    dy = (k == 0) ? 1 : k - 2;
-                } else {
-                    dz = 1;
-                    dx = (k - 4) / 3 - 1;
-                    dy = (k - 4) % 3 - 1;
-                }
-                has[k] = false;
-                key[k] = 0;
-                if (p == kNone || (d3q7 && (dx != 0) + (dy != 0) + (dz != 0) > 1)) continue;
-                const int nx = x + dx, ny = y + dy, nz = z + dz;
-                if (!g.inside(nx, ny, nz)) continue;
-                const size_t w = g.idx(nx, ny, nz);
-                const uint32_t rw = crad[w];
-                if (rw == 0 || rw == r) continue;
-                const uint32_t q = pid[w];
-                key[k] = rw < r ? (static_cast<unsigned long long>(q) << sb) | p
-                                : (static_cast<unsigned long long>(p) << sb) | q;
-                has[k] = true;
-            }
-            unsigned ns = 0;
-#pragma unroll
-            for (int k = 0; k < 13; ++k) {
-                if (!has[k]) continue;
-                unsigned h = static_cast<unsigned>((key[k] * 0x9E3779B97F4A7C15ull) >> 40) & (kEdgeTable - 1);
-                for (int probe = 0; probe < 8; ++probe, h = (h + 1) & (kEdgeTable - 1)) {
-                    const unsigned long long prev = atomicCAS(&table[h], ~0ull, key[k]);
-                    if (prev == ~0ull) break;
-                    if (prev == key[k]) {
-                        has[k] = false;
-                        break;
-                    }
-                }
-                ns += has[k] ? 1u : 0u;
-            }
-            // one atomic per warp; lanes place their edges by a warp prefix sum
-            unsigned incl = ns;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned t2 = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= static_cast<unsigned>(o)) incl += t2;
-            }
-            unsigned long long pos = 0;
-            if (lane == 31 && incl) pos = atomicAdd(count, static_cast<unsigned long long>(incl));
-            pos = __shfl_sync(0xFFFFFFFFu, pos, 31) + (incl - ns);
-#pragma unroll
-            for (int k = 0; k < 13; ++k)
-                if (has[k]) {
-                    if (pos < cap) edges[pos] = key[k];
-                    ++pos;
-                }
-        }
-        __syncthreads();  // before the next tile resets the table
     }
 }
 
@@ -1274,6 +1261,8 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
     }
 
     // Plateaus: connected sets of equal crad under the stencil.
+    const unsigned pair_grid = static_cast<unsigned>(std::min<size_t>(
+        static_cast<size_t>(div_up(d.sy, kTileY)) * div_up(d.sx, kTileX) * div_up(d.sz, kTileZ), ctx->num_sms * 32ull));
     uf_init<<<G, 256, 0, s>>>(crad2, g, n, d3q7, pid);
     ctx->check_launch("uf_init");
     {
@@ -1299,8 +1288,8 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
             for (int attempt = 0;; ++attempt) {
                 pairs = buf<unsigned long long>(ctx, "pores.uf_pairs", pcap);
                 PMA_CUDA(cudaMemsetAsync(pcount, 0, 8, s));
-                uf_pairs<<<G, 256, 0, s>>>(crad2, g, n, d3q7, pid, pairs, pcap, pcount);
-                ctx->check_launch("uf_pairs");
+                voxel_pairs<true><<<pair_grid, kPairThreads, 0, s>>>(pid, crad2, g, d3q7, 0, pcount, pairs, pcap);
+                ctx->check_launch("voxel_pairs");
                 PMA_CUDA(cudaMemcpyAsync(&npairs, pcount, 8, cudaMemcpyDeviceToHost, s));
                 ctx->sync();
                 if (npairs <= pcap) break;
@@ -1357,9 +1346,9 @@ pma_table* pores(pma_ctx* ctx, const uint8_t* mask, const uint32_t* edt2, const 
         PMA_CUDA(cudaMemsetAsync(ecount, 0, 8, s));
         {
             KernelTimer kt(ctx, "edges_write");
-            plateau_edges<<<G, 256, 0, s>>>(pid, crad2, g, d3q7, sb, ecount, edges_raw, ecap);
+            voxel_pairs<false><<<pair_grid, kPairThreads, 0, s>>>(pid, crad2, g, d3q7, sb, ecount, edges_raw, ecap);
         }
-        ctx->check_launch("plateau_edges");
+        ctx->check_launch("voxel_pairs");
         PMA_CUDA(cudaMemcpyAsync(&ne_kept, ecount, 8, cudaMemcpyDeviceToHost, s));
         ctx->sync();
         if (ne_kept <= ecap) break;
