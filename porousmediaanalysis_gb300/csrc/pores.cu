@@ -1795,120 +1795,96 @@ void remove_empty_pores(pma_ctx* ctx, pma_table* t, uint32_t* labels, pma_dims d
     for (size_t i = 0; i < nt; ++i) by_id[i] = static_cast<uint32_t>(i);
     auto id_less = [&](uint32_t a, uint32_t b) { return t->throats[a].id < t->throats[b].id; };
     if (!std::is_sorted(by_id.begin(), by_id.end(), id_less)) std::sort(by_id.begin(), by_id.end(), id_less);
-    // On host threads when there are many types: a count pass, then the lists written in place.
-    std::vector<uint32_t> lists;
+    // One pass, on host threads when there are many types: each list filtered and sorted in the place
+    // that its whole length would take, and hashed.
     std::vector<size_t> loff(nt + 1, 0);
-    auto filter = [&](size_t lo, size_t hi, bool write) {
-        std::vector<uint32_t> tmp;
+    for (size_t k = 0; k < nt; ++k) loff[k + 1] = loff[k] + t->throats[by_id[k]].n_pores;
+    std::vector<uint32_t> lists(loff[nt]), len(nt);
+    std::vector<unsigned long long> lhash(nt);
+    auto filter = [&](size_t lo, size_t hi) {
         for (size_t k = lo; k < hi; ++k) {
             const pma_throat& th = t->throats[by_id[k]];
-            tmp.assign(t->pool.begin() + th.pool_offset, t->pool.begin() + th.pool_offset + th.n_pores);
-            if (!std::is_sorted(tmp.begin(), tmp.end())) std::sort(tmp.begin(), tmp.end());
-            size_t at = write ? loff[k] : 0;
-            for (uint32_t pid : tmp)
-                if (pid > max_pore || !is_empty[pid]) {
-                    if (write) lists[at] = pid;
-                    ++at;
-                }
-            if (!write) loff[k + 1] = at;
+            const uint32_t* from = t->pool.data() + th.pool_offset;
+            uint32_t* list = lists.data() + loff[k];
+            uint32_t m = 0;
+            for (uint32_t i = 0; i < th.n_pores; ++i) {
+                const uint32_t pid = from[i];
+                if (pid > max_pore || !is_empty[pid]) list[m++] = pid;
+            }
+            if (m > 1 && !std::is_sorted(list, list + m)) std::sort(list, list + m);
+            unsigned long long h = 1469598103934665603ull ^ m;
+            for (uint32_t i = 0; i < m; ++i) h = (h ^ list[i]) * 1099511628211ull;
+            len[k] = m;
+            lhash[k] = h;
         }
     };
     const unsigned nth = nt >= (1u << 15) ? std::max(1u, std::min(8u, std::thread::hardware_concurrency())) : 1u;
-    auto parallel = [&](bool write) {
+    {
         std::vector<std::thread> ts;
         for (unsigned i = 1; i < nth; ++i) {
             try {
-                ts.emplace_back(filter, nt * i / nth, nt * (i + 1) / nth, write);
+                ts.emplace_back(filter, nt * i / nth, nt * (i + 1) / nth);
             } catch (const std::system_error&) {
-                filter(nt * i / nth, nt * (i + 1) / nth, write);  // no thread to be had: in line
+                filter(nt * i / nth, nt * (i + 1) / nth);  // no thread to be had: in line
             }
         }
-        filter(0, nt / nth, write);
+        filter(0, nt / nth);
         for (auto& th : ts) th.join();
-    };
-    parallel(false);  // loff[k + 1] = kept length of type k
-    for (size_t k = 0; k < nt; ++k) loff[k + 1] += loff[k];
-    lists.resize(loff[nt]);
-    parallel(true);
-    auto len = [&](size_t k) { return loff[k + 1] - loff[k]; };
+    }
     phase("removal.filter_ms");
     ctx->count("removal.types", static_cast<double>(nt));
     std::vector<char> alive(nt, 1);
     std::vector<std::pair<uint32_t, uint32_t>> remap;  // (old id, new id)
     // EPR.cpp:167-191: types with fewer than two pores.
     for (size_t k = 0; k < nt; ++k)
-        if (len(k) < 2) {
-            if (len(k) == 1) remap.emplace_back(t->throats[by_id[k]].id, lists[loff[k]]);
+        if (len[k] < 2) {
+            if (len[k] == 1) remap.emplace_back(t->throats[by_id[k]].id, lists[loff[k]]);
             alive[k] = 0;
         }
-    // EPR.cpp:126-165: merge types with equal pore lists into the largest id. Lists are put
-    // side by side through a hash of their contents and grouped by comparing them element by
-    // element within a hash (the groups, not their order, decide the result).
-    auto same_list = [&](uint32_t a, uint32_t b) {
-        return len(a) == len(b) && std::equal(lists.begin() + loff[a], lists.begin() + loff[a + 1],
-                                              lists.begin() + loff[b]);
-    };
-    std::vector<unsigned long long> lhash(nt);  // hashes of the lists, on the filter's threads
-    auto hash_range = [&](size_t lo, size_t hi) {
-        for (size_t k = lo; k < hi; ++k) {
-            unsigned long long h = 1469598103934665603ull ^ len(k);
-            for (size_t i = loff[k]; i < loff[k + 1]; ++i) h = (h ^ lists[i]) * 1099511628211ull;
-            lhash[k] = h;
+    // EPR.cpp:126-165: merge types with equal pore lists into the largest id. A hash table holds the first
+    // type of each list; equal hashes are settled by comparing the lists. (Sorting the hashes of 82
+    // thousand types took 4.2 ms; the whole removal took 8.1 ms before this form and the one-pass filter, 3.0 after.)
+    size_t slots = 16;
+    while (slots < 2 * nt) slots *= 2;
+    std::vector<uint32_t> first(slots, kNone), like(nt, kNone), keep(nt, 0);  // like: the first type of k's list
+    bool merged = false;
+    for (size_t k = 0; k < nt; ++k) {
+        if (!alive[k]) continue;
+        const uint32_t* list = lists.data() + loff[k];
+        for (size_t h = static_cast<size_t>((lhash[k] * 0x9E3779B97F4A7C15ull) >> 32) & (slots - 1);; h = (h + 1) & (slots - 1)) {
+            const uint32_t f = first[h];
+            if (f == kNone) first[h] = like[k] = static_cast<uint32_t>(k);
+            else if (lhash[f] == lhash[k] && len[f] == len[k] && std::equal(list, list + len[k], lists.data() + loff[f])) like[k] = f;
+            else continue;
+            break;
         }
-    };
-    {
-        std::vector<std::thread> ts;
-        for (unsigned i = 1; i < nth; ++i) {
-            try {
-                ts.emplace_back(hash_range, nt * i / nth, nt * (i + 1) / nth);
-            } catch (const std::system_error&) {
-                hash_range(nt * i / nth, nt * (i + 1) / nth);  // no thread to be had: in line
-            }
-        }
-        hash_range(0, nt / nth);
-        for (auto& th : ts) th.join();
+        merged |= like[k] != k;
+        keep[like[k]] = std::max(keep[like[k]], t->throats[by_id[k]].id);
     }
-    std::vector<std::pair<unsigned long long, uint32_t>> live;  // (hash of the list, type)
-    for (size_t k = 0; k < nt; ++k)
-        if (alive[k]) live.emplace_back(lhash[k], static_cast<uint32_t>(k));
-    std::sort(live.begin(), live.end());
-    std::vector<uint32_t> members;
-    for (size_t i = 0; i < live.size();) {
-        size_t j = i + 1;
-        while (j < live.size() && live[j].first == live[i].first) ++j;
-        for (size_t a = i; a < j && j - i > 1; ++a) {  // equal hashes: exact groups among them
-            if (!alive[live[a].second]) continue;
-            members.assign(1, live[a].second);
-            for (size_t b = a + 1; b < j; ++b)
-                if (alive[live[b].second] && same_list(live[a].second, live[b].second))
-                    members.push_back(live[b].second);
-            if (members.size() < 2) continue;
-            uint32_t keep = 0;
-            for (uint32_t m : members) keep = std::max(keep, t->throats[by_id[m]].id);
-            for (uint32_t m : members) {
-                const uint32_t id = t->throats[by_id[m]].id;
-                if (id != keep) {
-                    alive[m] = 0;
-                    remap.emplace_back(id, keep);
-                }
-            }
+    for (size_t k = 0; k < nt && merged; ++k) {
+        if (!alive[k]) continue;
+        const uint32_t id = t->throats[by_id[k]].id;
+        if (id != keep[like[k]]) {
+            alive[k] = 0;
+            remap.emplace_back(id, keep[like[k]]);
         }
-        i = j;
     }
     phase("removal.merge_ms");
     std::vector<pma_throat> throats;
     std::vector<uint32_t> pool;
+    throats.reserve(nt);
+    pool.reserve(lists.size());
     for (size_t k = 0; k < nt; ++k) {
         if (!alive[k]) continue;
         pma_throat th;
         th.id = t->throats[by_id[k]].id;
         th.volume = t->throats[by_id[k]].volume;
-        th.n_pores = static_cast<uint32_t>(len(k));
+        th.n_pores = len[k];
         th.pool_offset = pool.size();
-        pool.insert(pool.end(), lists.begin() + loff[k], lists.begin() + loff[k + 1]);
+        pool.insert(pool.end(), lists.begin() + loff[k], lists.begin() + loff[k] + len[k]);
         throats.push_back(th);
     }
-    t->pores = kept;
+    t->pores.swap(kept);
     t->throats.swap(throats);
     t->pool.swap(pool);
     std::sort(remap.begin(), remap.end());
