@@ -7,7 +7,7 @@
 //   pass X: columns packed into bitmasks in shared memory; the nearest solid on both sides is
 //           read off the bits, and the distance (not its square) goes out in 16 bits, into the
 //           first half of the voxel's row of the result. HBM: 1 B read + 2 B written per voxel.
-//   pass Y: one warp per row; reads the row's distances, writes squares over them. 2 B + 4 B.
+//   pass Y: a block per eight rows; reads their distances, writes squares over them. 2 B + 4 B.
 //   pass Z: tiles of 16 consecutive y by all z staged in shared memory, fused with the running
 //           maximum and the histogram of balls that do not cross the image boundary
 //           (EDC.cpp:310-327). 4 B + 4 B.
@@ -17,8 +17,8 @@
 // last one: it then counts with a distance larger than its own, which never lowers a minimum.
 // What bounds them: instructions, about two per output and step, as many steps as the largest
 // distance of the warp's outputs. 1024^3 spinodal, before (32-bit squares throughout, one output
-// a thread, both inputs read again for each) and after, ms: X 2.3 -> 1.2, Y 8.0 -> 5.9,
-// Z 10.9 -> 4.7 (1.8 TB/s).
+// a thread, both inputs read again for each) and after, ms: X 2.3 -> 1.2, Y 8.0 -> 5.1,
+// Z 10.9 -> 4.6 (1.9 TB/s).
 // Extents for which a square or a sum could pass 2^32 go through the general kernels.
 #include <algorithm>
 #include <mutex>
@@ -317,40 +317,47 @@ __device__ __forceinline__ void walk_line(F f, int n, int i0, int live, uint32_t
 }
 
 // ---------------------------------------------------------------------------------------
-// Pass Y: one warp per row. The row's distances lie in shared memory with two elements skipped
-// after every eight, so that the lanes' inputs (eight apart) fall on different banks.
+// Pass Y: a block takes as many rows as it has warps (eight, fewer where the rows are long), a warp a
+// stretch of all of them: 32 y of eight rows, not 256 y of one, because the longest walk of the warp
+// counts for all its lanes, and near outputs are alike (spinodal of wavelength 48: 16.3 steps on average,
+// not 24.5; 5.9 -> 5.1 ms). The rows' distances lie in shared memory with two elements skipped after every
+// eight and rows 4 (mod 8) words apart, so that the lanes' inputs fall on different banks.
+// Walks on 16-bit pairs (6.2 ms) and on floats with three-input minima (4.8, but pass Z 4.9) gave nothing.
 // ---------------------------------------------------------------------------------------
 constexpr int kYPad = kOut + 1;  // outputs of a lane, staged for coalesced stores
 
 __global__ void edt_pass_y(uint32_t* __restrict__ g, int SY, size_t nrows, int row_words) {
-    extern __shared__ uint32_t smem[];  // per warp: row_words words of distances, 32 * kYPad outputs
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    uint32_t* dist = smem + static_cast<size_t>(warp) * (row_words + 32 * kYPad);
-    uint32_t* stage = dist + row_words;
-    const uint16_t* d16 = reinterpret_cast<const uint16_t*>(dist);
+    extern __shared__ uint32_t smem[];  // per warp: row_words words of distances; then 32 * kYPad outputs
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, wb = __ffs(warps) - 1;
+    const int per_row = 32 >> wb, span = per_row * kOut;  // lanes and outputs of a row in a warp's stretch
+    const int mine = lane >> (5 - wb);
+    uint32_t* dist = smem + static_cast<size_t>(warp) * row_words;
+    uint32_t* stage = smem + static_cast<size_t>(warps) * row_words + warp * (32 * kYPad);
+    const uint16_t* d16 = reinterpret_cast<const uint16_t*>(smem + static_cast<size_t>(mine) * row_words);
     auto f = [&](int j) {
         const uint32_t d = d16[j + 2 * (j / kOut)];
         return d * d;
     };
-    for (size_t r = static_cast<size_t>(blockIdx.x) * warps + warp; r < nrows;
-         r += static_cast<size_t>(gridDim.x) * warps) {
-        uint32_t* row = g + r * SY;
-        for (int i = lane; i < (SY + 1) / 2; i += 32) dist[i + 2 * i / kOut] = row[i];
-        __syncwarp();
-        for (int y0 = 0; y0 < SY; y0 += 32 * kOut) {
-            const int i0 = y0 + lane * kOut;
+    for (size_t r0 = static_cast<size_t>(blockIdx.x) * warps; r0 < nrows; r0 += static_cast<size_t>(gridDim.x) * warps) {
+        uint32_t* rows = g + r0 * SY;
+        if (r0 + warp < nrows)
+            for (int i = lane; i < (SY + 1) / 2; i += 32) dist[i + 2 * i / kOut] = rows[static_cast<size_t>(warp) * SY + i];
+        __syncthreads();
+        for (int y0 = warp * span; y0 < SY; y0 += warps * span) {
+            const int i0 = y0 + (lane - mine * per_row) * kOut;
             uint32_t best[kOut];
-            walk_line(f, SY, min(i0, SY - 1), min(max(SY - i0, 0), kOut), best);
+            walk_line(f, SY, min(i0, SY - 1), r0 + mine < nrows ? min(max(SY - i0, 0), kOut) : 0, best);
 #pragma unroll
             for (int k = 0; k < kOut; ++k) stage[lane * kYPad + k] = best[k];
             __syncwarp();
 #pragma unroll
             for (int k = 0; k < kOut; ++k) {
-                const int i = k * 32 + lane;
-                if (y0 + i < SY) row[y0 + i] = stage[i + i / kOut];
+                const int i = k * 32 + lane, row = i >> (8 - wb), y = y0 + i - row * span;
+                if (y < SY && r0 + row < nrows) rows[static_cast<size_t>(row) * SY + y] = stage[i + i / kOut];
             }
             __syncwarp();
         }
+        __syncthreads();  // before the next rows are staged
     }
 }
 
@@ -399,7 +406,7 @@ __global__ void __launch_bounds__(kZThreads) edt_pass_z(uint32_t* __restrict__ g
             local_max = max(local_max, e);
             const int m = min(mxy, min(z, SZ - 1 - z));
             // e <= m^2 <=> the ball of radius sqrt(e) stays inside the image (EDC.cpp:316-327).
-            if (static_cast<unsigned long long>(e) <= static_cast<unsigned long long>(m) * m) {
+            if (e <= static_cast<uint32_t>(m) * static_cast<uint32_t>(m)) {  // m < 2^15 here
                 if (e < kHistSmall) atomicAdd(&h_small[e], 1u);
                 else if (e < hist_len) atomicAdd(&hist[e], 1ull);
             }
@@ -486,7 +493,8 @@ void edt_passes(const char* who, const uint8_t* solid, pma_dims d, uint32_t* edt
         else edt_pass_x<1><<<div_up(cols, kXThreads), kXThreads, x1, s>>>(solid, edt2, SX, SY, SZ, words, hist, nclear);
     });
     timed("edt_pass_y", [&] {
-        const size_t row_words = static_cast<size_t>(SY) / 2 + SY / kOut + 2;  // below the general pass's 4 SY bytes
+        // below the general pass's 4 SY bytes; 4 (mod 8)
+        const size_t row_words = (static_cast<size_t>(SY) / 2 + SY / kOut + 2 + 3) / 8 * 8 + 4;
         int warps = 8;
         while (warps > 1 && warps * (row_words + 32 * kYPad) * 4 > 96 * 1024) warps >>= 1;
         const size_t smem = warps * (row_words + 32 * kYPad) * 4;
