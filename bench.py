@@ -47,14 +47,14 @@ WORKLOADS = {
 # DRAM bytes per voxel measured by ncu over all launches of a kernel in one step of a 320^3
 # GRF, used as the roofline's `traffic` when that kernel dominates.
 TRAFFIC_PER_VOXEL = {
-    "ws_generations": (156.2, "ncu dram__bytes_read+write of the 107 ws_generations launches of one "
-                              "320^3 GRF step (4683 MB read, 436 MB written), scaled by voxels"),
+    "ws_generations": (125.4, "ncu dram__bytes_read+write of the 91 ws_generations launches of one "
+                              "320^3 GRF chain (3707 MB read, 403 MB written), scaled by voxels"),
 }
 
 # Algorithmic HBM bytes per voxel of the timed kernels (reads + writes each kernel must do).
 ALGO_BYTES = {
-    "edt_pass_x": 5.0,          # 1 B mask read + 4 B write
-    "edt_pass_y": 8.0,          # 4 B read + 4 B write
+    "edt_pass_x": 3.0,          # 1 B mask read + 2 B distance written
+    "edt_pass_y": 6.0,          # 2 B read + 4 B write
     "edt_pass_z": 8.0,          # 4 B read + 4 B write
     "balls_candidates": 16.0,   # 2 x (4 B EDT read) + 8 B key init write
     "balls_tile_gather": 20.0,  # 4 B EDT read + 16 B (radius, centre x, y, z) written

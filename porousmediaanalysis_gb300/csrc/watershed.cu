@@ -648,8 +648,8 @@ __global__ void __launch_bounds__(kGenThreads, 4) ws_generations(WsState s, uint
 // --- small generations --------------------------------------------------------------------
 //
 // Most generations are small (a few to a few thousand nodes) and their time is latency: in
-// ws_generations a generation of 2^6 to 2^10 nodes takes 10 to 14 us (two barriers over the whole
-// grid, the look-back, one launch and one host round trip per depth). ws_small runs them in one
+// ws_generations a generation of 2^6 to 2^10 nodes takes 10 to 14 us (three barriers over the whole
+// grid, one launch and one host round trip per depth). ws_small runs them in one
 // thread-block cluster, and goes from depth to depth by itself: it sorts a depth's bucket in
 // shared memory, runs its generations and takes the next depth, until a bucket or a frontier is
 // too large for it (the host then sorts that bucket and runs ws_generations until the frontier
