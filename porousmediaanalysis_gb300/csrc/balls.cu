@@ -782,8 +782,9 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
         return z1;
     };
     const unsigned long long budget = std::max<unsigned long long>(1ull << 20, std::min<unsigned long long>(free_b / 6, 32ull << 30) / 8);
-    const unsigned long long tile_budget =
-        std::max<unsigned long long>(1ull << 17, std::min<unsigned long long>(free_b / 6, 8ull << 30) / (8 * kSub));
+    // 16 bytes a voxel: with the groups' lists what lists of the tiles alone would take, four to seven slabs
+    const unsigned long long tile_bytes = std::min<unsigned long long>({free_b / 6, 8ull << 30, std::max<unsigned long long>(64ull << 20, 16ull * n)});
+    const unsigned long long tile_budget = std::max<unsigned long long>(1ull << 17, tile_bytes / (8 * kSub));
     const FastDiv fsz(static_cast<uint32_t>(d.sz));
     for (int z0 = 0, z1 = 0; z0 < gt.TZ; z0 = z1) {
         z1 = upto(z0, gt.TZ, budget);
