@@ -659,7 +659,9 @@ __global__ void __launch_bounds__(kGenThreads, 4) ws_generations(WsState s, uint
 // What bounds a generation: latency (a block barrier 50 cycles, a cluster barrier 400 and with it
 // the wait for the atomics in flight, an L2 load 300 to 700), and one sector a clock and SM for the
 // scattered state words; hence 16 blocks, and 64 nodes as the most for one block alone. From about
-// 2000 nodes the whole grid is faster (2^11 nodes: 20 us here, 16 there; 2^10: 13.5 against 15.7).
+// 2000 nodes the whole grid is faster (2^11 nodes: 20 us here, 12 there). At 2^10 it is too, 11.3 against 14.5, but each
+// change between the two costs a launch and a host round trip: with 1024 as the limit a 640 x 600 x 672
+// spinodal took 277 ms, not 279, a 128^3 union 42.2, not 40.6.
 // Whole stage, before and after (ms): 40 x 48 x 44 union 15.6 -> 5.2, 128^3 union 48.5 -> 30.7,
 // 300 x 341 x 277 spinodal 135 -> 119.
 constexpr int kSmallThreads = 512;
