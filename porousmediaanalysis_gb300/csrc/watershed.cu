@@ -704,6 +704,7 @@ struct WsSmallShared {
     uint32_t total[kSmallCluster];
     uint32_t delta[27];      // index step of a stencil position
     uint32_t log_base, log_used;  // the block's slab of the extension log
+    uint32_t found_di, found_n;   // the next depth with entries and how many
     WsCtl ctl;
 };
 
@@ -1042,7 +1043,7 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallTh
     __shared__ WsSmallShared sh;
     extern __shared__ __align__(16) unsigned char dynamic[];
     WsSortShared& so = *reinterpret_cast<WsSortShared*>(dynamic);
-    const unsigned tid = threadIdx.x, lane = tid & 31, rank = cl.block_rank();
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = cl.block_rank();
     if (tid < 27) {
         int dx, dy, dz;
         stencil_offset(static_cast<int>(tid), 0, dx, dy, dz);
@@ -1066,27 +1067,38 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallTh
         if (rank == 0) {  // solo generations, bucket sorts and the way from depth to depth
             c.mode = kWsDone;
             for (;;) {
-                // the host empties the log (and adds records) before it fills up
-                if ((c.n == 0 || (c.gen & 15) == 0) && 2ull * __ldcg(s.log_n) > s.log_cap) {
+                // The host empties the log (and adds records) before it fills up. One thread looks for the
+                // block: the other blocks may still be adding their first slabs to the counter, and
+                // threads that read it for themselves could part ways here, at barriers that do not match.
+                if ((c.n == 0 || (c.gen & 15) == 0) && __syncthreads_or(tid == 0 && 2ull * __ldcg(s.log_n) > s.log_cap)) {
                     c.mode = kWsGrow;
                     break;
                 }
-                if (c.n == 0) {  // the deepest depth with entries: 32 at a time
-                    uint32_t n0 = 0;
-                    for (; c.di < a.ndepths; c.di += 32) {
-                        uint32_t f = 0;
-                        if (c.di + lane < a.ndepths) {
-                            const uint32_t d = a.depths[c.di + lane];
-                            f = static_cast<uint32_t>(__ldcg(s.bpos + d) - __ldg(a.boff + d));
+                if (c.n == 0) {  // the deepest depth with entries: the first warp looks at 32 at a time, for the block
+                    if (warp == 0) {
+                        uint32_t di = c.di, n0 = 0;
+                        for (; di < a.ndepths; di += 32) {
+                            uint32_t f = 0;
+                            if (di + lane < a.ndepths) {
+                                const uint32_t d = a.depths[di + lane];
+                                f = static_cast<uint32_t>(__ldcg(s.bpos + d) - __ldg(a.boff + d));
+                            }
+                            const unsigned m = __ballot_sync(0xFFFFFFFFu, f != 0);
+                            if (m) {
+                                const int l = __ffs(m) - 1;
+                                n0 = __shfl_sync(0xFFFFFFFFu, f, l);
+                                di += l;
+                                break;
+                            }
                         }
-                        const unsigned m = __ballot_sync(0xFFFFFFFFu, f != 0);
-                        if (m) {
-                            const int l = __ffs(m) - 1;
-                            n0 = __shfl_sync(0xFFFFFFFFu, f, l);
-                            c.di += l;
-                            break;
+                        if (lane == 0) {
+                            sh.found_di = di;
+                            sh.found_n = n0;
                         }
                     }
+                    __syncthreads();
+                    c.di = sh.found_di;
+                    const uint32_t n0 = sh.found_n;
                     if (n0 == 0) break;  // done
                     c.n = n0;
                     if (n0 > kSmallSort) {
@@ -1462,6 +1474,8 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
     size_t used = 0;  // records in use when the log was last emptied
     auto record_extensions = [&](unsigned long long reserved) {
         const size_t noted = static_cast<size_t>(std::min<unsigned long long>(reserved, log_cap));
+        ctx->count("ws.log_entries", static_cast<double>(noted));
+        if (reserved > log_cap) ctx->count("ws.log_overflow", static_cast<double>(reserved - log_cap));
         unsigned int* h_used = static_cast<unsigned int*>(ctx->host_staging(128)) + 28;
         size_t at = 0;
         // each entry takes at most one new record: as many entries as records are free at a time
@@ -1606,7 +1620,10 @@ pma_table* watershed(pma_ctx* ctx, const pma_table* pt, const uint32_t* crad2, p
             if (c.mode == kWsDone || 2 * *h_log_n > ws.log_cap) record_extensions(*h_log_n);
             if (c.mode == kWsDone) break;
             PMA_REQUIRE(c.mode != kWsLimit, PMA_ERR_LIMIT, "pma_watershed: generation limit reached");
-            if (c.mode == kWsGrow) continue;
+            if (c.mode == kWsGrow) {
+                ctx->count("ws.log_stops", 1);
+                continue;
+            }
             const uint32_t dep = depths[c.di];
             int cur = static_cast<int>(c.cur);
             if (c.mode == kWsSort) {
