@@ -767,7 +767,8 @@ __device__ void sweep_block(const PlateauSets& st, SweepShared<W>& sh, uint32_t 
         uint32_t len = set_len(s);
         mp = min(mp, static_cast<uint32_t>(s.y));
         sum += len;
-        if (spread || *reinterpret_cast<volatile unsigned int*>(&sh.bover)) continue;  // sizes only
+        // sizes only; other warps set the flag meanwhile, so the warp decides by a vote
+        if (spread || __any_sync(0xFFFFFFFFu, *reinterpret_cast<volatile unsigned int*>(&sh.bover))) continue;
         const unsigned peers = __match_any_sync(0xFFFFFFFFu, len ? s.x : ~0ull);
         if (len && static_cast<int>(lane) != __ffs(peers) - 1) len = 0;
         if (len) {  // sets the block has seen already
