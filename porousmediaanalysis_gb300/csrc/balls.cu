@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "devutil.cuh"
+#include "group_runs.h"
 
 namespace pma {
 namespace {
@@ -278,11 +279,12 @@ struct FillGroup {
     const unsigned long long* gfloor;
     const unsigned long long* goff;
     unsigned long long base;
+    size_t g0, g1;  // the groups being filled
     unsigned int* gcursor;
     unsigned long long* groups;
     unsigned long long key;
     __device__ void operator()(size_t id) const {
-        if (key < __ldg(gfloor + id)) return;
+        if (id < g0 || id >= g1 || key < __ldg(gfloor + id)) return;
         const unsigned int at = add_one<kNear>(&gcursor[id], id);
         groups[goff[id] - base + at] = key;
     }
@@ -302,16 +304,18 @@ __global__ void balls_group_count(const uint32_t* __restrict__ cand, const uint3
 
 template <bool kNear>
 __global__ void balls_group_fill(const uint32_t* __restrict__ cand, const uint32_t* __restrict__ down, uint32_t max_edt2,
-                                 size_t nc, Grid g, Tiles gt, int gz0, int gz1,
+                                 size_t nc, Grid g, Tiles gt, size_t g0, size_t g1,
                                  const unsigned long long* __restrict__ gfloor,
                                  const unsigned long long* __restrict__ goff, unsigned long long base,
                                  unsigned int* __restrict__ gcursor, unsigned long long* __restrict__ groups) {
+    const size_t per_z = static_cast<size_t>(gt.TX) * gt.TY;
+    const int gz0 = static_cast<int>(g0 / per_z), gz1 = static_cast<int>((g1 - 1) / per_z) + 1;
     PMA_GRID_STRIDE(i, nc) {
         int x, y, z;
         g.coords(cand[i], x, y, z);
         const uint32_t R = max_edt2 - down[i];
         for_each_group(g, gt, x, y, z, R, gz0, gz1,
-                       FillGroup<kNear>{gfloor, goff, base, gcursor, groups, ball_key(g, x, y, z, R)});
+                       FillGroup<kNear>{gfloor, goff, base, g0, g1, gcursor, groups, ball_key(g, x, y, z, R)});
     }
 }
 
@@ -372,7 +376,7 @@ __device__ __forceinline__ unsigned long long tile_list(unsigned long long group
 // warp takes its places in all eight lists with one atomic instruction in shared memory.
 constexpr int kSplitThreads = 256;
 
-__global__ void __launch_bounds__(kSplitThreads) balls_split(Grid g, FastDiv fsz, Tiles t, Tiles gt, int gz0,
+__global__ void __launch_bounds__(kSplitThreads) balls_split(Grid g, FastDiv fsz, Tiles t, Tiles gt, size_t g0,
                                                              const unsigned long long* __restrict__ floor,
                                                              const unsigned int* __restrict__ gcount,
                                                              const unsigned long long* __restrict__ goff, unsigned long long base,
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(kSplitThreads) balls_split(Grid g, FastDiv fsz
     static_assert(kGroup == 2, "two tiles an axis");
     __shared__ unsigned int s_n[kSub];
     __shared__ unsigned long long s_floor[kSub];
-    const size_t group = static_cast<size_t>(gz0) * gt.TX * gt.TY + blockIdx.x;
+    const size_t group = g0 + blockIdx.x;
     const unsigned lane = threadIdx.x & 31;
     int tx, ty, tz;
     if (threadIdx.x < kSub) {
@@ -435,7 +439,7 @@ __global__ void __launch_bounds__(kSplitThreads) balls_split(Grid g, FastDiv fsz
     if (threadIdx.x < kSub) tcount[static_cast<size_t>(blockIdx.x) * kSub + threadIdx.x] = s_n[threadIdx.x];
 }
 
-// One CTA per tile of the groups of the z-range starting at gz0: winner key of each voxel.
+// One CTA per tile of the groups from g0 on: winner key of each voxel.
 //
 // The tile's list is taken in chunks of up to kListCap entries. Each chunk is decoded into
 // shared memory ordered by radius, largest first (a counting sort on r^2 when the chunk's r^2
@@ -449,14 +453,14 @@ __global__ void __launch_bounds__(kSplitThreads) balls_split(Grid g, FastDiv fsz
 constexpr int kSortBins = 2048;
 
 __global__ void __launch_bounds__(kTileVox, 4) balls_tile_gather(
-    const uint32_t* __restrict__ edt2, Grid g, FastDiv fsz, Tiles t, Tiles gt, int gz0,
+    const uint32_t* __restrict__ edt2, Grid g, FastDiv fsz, Tiles t, Tiles gt, size_t g0,
     const unsigned int* __restrict__ tcount, const unsigned int* __restrict__ gcount,
     const unsigned long long* __restrict__ goff, unsigned long long tile_base, const unsigned long long* __restrict__ entries,
     unsigned long long* __restrict__ keys, unsigned int* __restrict__ err) {
     __shared__ int4 s_pos[kListCap];
     __shared__ unsigned int s_bin[kSortBins];
     __shared__ unsigned int s_rmin, s_rmax, s_wsum[kTileVox / 32];
-    const size_t group = static_cast<size_t>(gz0) * gt.TX * gt.TY + blockIdx.x / kSub;
+    const size_t group = g0 + blockIdx.x / kSub;
     int tx, ty, tz;
     tile_of(gt, group, blockIdx.x % kSub, tx, ty, tz);
     if (ty >= t.TY || tx >= t.TX || tz >= t.TZ) return;
@@ -731,7 +735,7 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
             cand = cand2;
         }
     }
-    // Lists: counts, 64-bit offsets, then fill, split and gather by z-ranges whose entries fit the
+    // Lists: counts, 64-bit offsets, then fill, split and gather by runs of groups whose entries fit the
     // memory budget. One centre a thread and no strides: the lists keep the order of the centres roughly.
     Tiles t{(d.sx + kTile - 1) / kTile, (d.sy + kTile - 1) / kTile, (d.sz + kTile - 1) / kTile};
     const size_t ntiles = static_cast<size_t>(t.TX) * t.TY * t.TZ;
@@ -759,8 +763,8 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
         (near ? balls_group_count<true> : balls_group_count<false>)<<<div_up(nc, 256), 256, 0, s>>>(cand, down, max_edt2, nc, g, gt, gfloor, gcount);
         ctx->check_launch("balls_group_count");
     }
-    // 64-bit list offsets by a device scan; the host reads back only the offsets at the z-slab
-    // boundaries, which choose the slabs that fit the memory budget
+    // 64-bit list offsets by a device scan; the host reads back the offsets at the layers of groups (and
+    // those within a layer that does not fit), which choose the runs that fit the memory budget
     auto* tc64 = buf<unsigned long long>(ctx, "balls.tc64", ngroups + 1);
     widen_counts<<<grid_for(ctx, ngroups + 1), 256, 0, s>>>(gcount, ngroups, tc64);
     ctx->check_launch("widen_counts");
@@ -771,46 +775,72 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
     std::vector<unsigned long long> hz(gt.TZ + 1);
     PMA_CUDA(cudaMemcpyAsync(hz.data(), zoff, (gt.TZ + 1) * 8ull, cudaMemcpyDeviceToHost, s));
     ctx->sync();
-    auto ho_at = [&](int z) { return hz[z]; };  // offset of the first group of slab z
+    std::vector<unsigned long long> layer;  // offsets of layer layer_z's groups and of the next one's first
+    size_t layer_z = ~size_t(0);
+    auto layer_at = [&](size_t z) -> const unsigned long long* {
+        if (layer_z != z) {
+            layer.resize(per_z + 1);
+            PMA_CUDA(cudaMemcpyAsync(layer.data(), goff + z * per_z, (per_z + 1) * 8, cudaMemcpyDeviceToHost, s));
+            ctx->sync();
+            layer_z = z;
+        }
+        return layer.data();
+    };
+    auto offset_of = [&](size_t group) {
+        const size_t z = group / per_z;
+        return group == z * per_z ? hz[z] : layer_at(z)[group - z * per_z];
+    };
     size_t free_b = 0, total_b = 0;
     PMA_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    // group lists by z-ranges that fit the memory budget, and of these the tiles' lists (with room for
-    // every entry of the group in each of its tiles) by z-ranges that fit theirs
-    auto upto = [&](int z0, int end, unsigned long long budget) {
-        int z1 = z0 + 1;
-        while (z1 < end && ho_at(z1 + 1) - ho_at(z0) <= budget) ++z1;
-        return z1;
-    };
+    // Group lists by runs of groups that fit the memory budget, and of these the tiles' lists (with room for
+    // every entry of the group in each of its tiles) by runs that fit theirs: whole layers of groups, or a
+    // part of one where a layer alone takes more (wide and thin volumes; at least one group).
     const unsigned long long budget = std::max<unsigned long long>(1ull << 20, std::min<unsigned long long>(free_b / 6, 32ull << 30) / 8);
     // 16 bytes a voxel: with the groups' lists what lists of the tiles alone would take, four to seven slabs
     const unsigned long long tile_bytes = std::min<unsigned long long>({free_b / 6, 8ull << 30, std::max<unsigned long long>(64ull << 20, 16ull * n)});
     const unsigned long long tile_budget = std::max<unsigned long long>(1ull << 17, tile_bytes / (8 * kSub));
     const FastDiv fsz(static_cast<uint32_t>(d.sz));
-    for (int z0 = 0, z1 = 0; z0 < gt.TZ; z0 = z1) {
-        z1 = upto(z0, gt.TZ, budget);
-        const unsigned long long base = ho_at(z0);
-        auto* groups = buf<unsigned long long>(ctx, "balls.groups", ho_at(z1) - base);
+    struct Run {  // groups [g0, g1), entries [e0, e1)
+        size_t g0, g1;
+        unsigned long long e0, e1;
+    };
+    auto runs = [&](size_t g0, size_t end, unsigned long long most, unsigned long long& longest) {
+        std::vector<Run> v;
+        for (size_t g1; g0 < end; g0 = g1) {
+            g1 = group_run_end(hz.data(), per_z, g0, end, most, layer_at);
+            v.push_back({g0, g1, offset_of(g0), offset_of(g1)});
+            longest = std::max(longest, v.back().e1 - v.back().e0);
+        }
+        return v;
+    };
+    unsigned long long fill_room = 0, split_room = 0;
+    const std::vector<Run> fills = runs(0, ngroups, budget, fill_room);
+    std::vector<std::vector<Run>> splits;
+    for (const Run& f : fills) splits.push_back(runs(f.g0, f.g1, tile_budget, split_room));
+    size_t most_groups = 0;
+    for (const auto& v : splits)
+        for (const Run& r : v) most_groups = std::max(most_groups, r.g1 - r.g0);
+    auto* groups = buf<unsigned long long>(ctx, "balls.groups", fill_room);
+    auto* entries = buf<unsigned long long>(ctx, "balls.entries", split_room * kSub);
+    auto* tcount = buf<unsigned int>(ctx, "balls.tcount", most_groups * kSub);
+    for (size_t k = 0; k < fills.size(); ++k) {
+        const Run& f = fills[k];
         if (nc) {
             KernelTimer kt(ctx, "balls_tile_fill");
             (near ? balls_group_fill<true> : balls_group_fill<false>)<<<div_up(nc, 256), 256, 0, s>>>(
-                cand, down, max_edt2, nc, g, gt, z0, z1, gfloor, goff, base, gcursor, groups);
+                cand, down, max_edt2, nc, g, gt, f.g0, f.g1, gfloor, goff, f.e0, gcursor, groups);
             ctx->check_launch("balls_group_fill");
         }
-        for (int y0 = z0, y1 = z0; y0 < z1; y0 = y1) {
-            y1 = upto(y0, z1, tile_budget);
-            const unsigned long long tile_base = ho_at(y0);
-            const unsigned slab = static_cast<unsigned>((y1 - y0) * per_z);
-            auto* entries = buf<unsigned long long>(ctx, "balls.entries", (ho_at(y1) - tile_base) * kSub);
-            auto* tcount = buf<unsigned int>(ctx, "balls.tcount", static_cast<size_t>(slab) * kSub);
+        for (const Run& r : splits[k]) {
+            const unsigned run = static_cast<unsigned>(r.g1 - r.g0);
+            ctx->count("balls.runs", static_cast<double>(r.e1 - r.e0));
             {
                 KernelTimer kt(ctx, "balls_split");
-                balls_split<<<slab, kSplitThreads, 0, s>>>(g, fsz, t, gt, y0, floor, gcount, goff, base, tile_base, groups, entries,
-                                                           tcount);
+                balls_split<<<run, kSplitThreads, 0, s>>>(g, fsz, t, gt, r.g0, floor, gcount, goff, f.e0, r.e0, groups, entries, tcount);
                 ctx->check_launch("balls_split");
             }
             KernelTimer kt(ctx, "balls_tile_gather");
-            balls_tile_gather<<<slab * kSub, kTileVox, 0, s>>>(edt2, g, fsz, t, gt, y0, tcount, gcount, goff, tile_base, entries,
-                                                               keys, err);
+            balls_tile_gather<<<run * kSub, kTileVox, 0, s>>>(edt2, g, fsz, t, gt, r.g0, tcount, gcount, goff, r.e0, entries, keys, err);
             ctx->check_launch("balls_tile_gather");
         }
     }
