@@ -468,11 +468,13 @@ std::vector<pma_cavity> geodesic(pma_ctx* ctx, const uint8_t* solid, pma_dims d,
         int k = 1;
         while (true) {
             KernelTimer kt(ctx, "geo_bucket");
-            for (int i = 0; i < max_steps_per_sync; ++i, ++k) {
+            // up to the next multiple of max_steps_per_sync: the bucket limit is looked at there (step 0 was geo_start's)
+            const int from = k, to = (k / max_steps_per_sync + 1) * max_steps_per_sync;
+            for (; k < to; ++k) {
                 if (d3q7) geo_step<T, true><<<step_grid, kBrickThreads, 0, s>>>(g, w1, w2, w3, dist, cavity, br, k, cavity_id, epoch0);
                 else geo_step<T, false><<<step_grid, kBrickThreads, 0, s>>>(g, w1, w2, w3, dist, cavity, br, k, cavity_id, epoch0);
             }
-            ctx->count_launch(max_steps_per_sync - 1);
+            ctx->count_launch(to - from - 1);
             ctx->check_launch("geo_step");
             ReadBack rb;
             rb.add(h, misc, 5 * 8);
