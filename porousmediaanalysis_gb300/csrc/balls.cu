@@ -796,8 +796,11 @@ void containing_balls(pma_ctx* ctx, const uint32_t* edt2, pma_dims d, uint32_t m
     // every entry of the group in each of its tiles) by runs that fit theirs: whole layers of groups, or a
     // part of one where a layer alone takes more (wide and thin volumes; at least one group).
     const unsigned long long budget = std::max<unsigned long long>(1ull << 20, std::min<unsigned long long>(free_b / 6, 32ull << 30) / 8);
-    // 16 bytes a voxel: with the groups' lists what lists of the tiles alone would take, four to seven slabs
-    const unsigned long long tile_bytes = std::min<unsigned long long>({free_b / 6, 8ull << 30, std::max<unsigned long long>(64ull << 20, 16ull * n)});
+    // 16 bytes a voxel: with the groups' lists what lists of the tiles alone would take, four to seven slabs. At least
+    // 512 MB: runs too short to fill the GPU last as long as their longest lists. With 64 MB a volume with few
+    // large pores, whose lists are long, went layer by layer: random field of sigma 14, 160^3 36.9 ms, 256^3 31.8;
+    // with 256 MB 13.8 and 32.0, with 512 MB 9.0 and 18.8 (tiles' own lists, without groups, 11.6 and 23.6).
+    const unsigned long long tile_bytes = std::min<unsigned long long>({free_b / 6, 8ull << 30, std::max<unsigned long long>(512ull << 20, 16ull * n)});
     const unsigned long long tile_budget = std::max<unsigned long long>(1ull << 17, tile_bytes / (8 * kSub));
     const FastDiv fsz(static_cast<uint32_t>(d.sz));
     struct Run {  // groups [g0, g1), entries [e0, e1)
