@@ -364,15 +364,23 @@ __global__ void edt_pass_y(uint32_t* __restrict__ g, int SY, size_t nrows, int r
 // ---------------------------------------------------------------------------------------
 // Pass Z with maximum and histogram. pitch: 18 words a z-slice of the tile (the two halves of a
 // warp are eight slices apart: 144 words, other banks), 16 where that does not fit.
+// Up to kZShort slices 128 threads a block, which cover 64 slices at once (512 would mostly be idle), and
+// short_bins of the histogram in shared memory, as many as the extents allow (balls that do not cross
+// the boundary): clearing 2048 for 16 lines of a few voxels was as much again. 1000 x 1000 planes, solid
+// 1 %, ms with 512 threads / 128: 2 planes 0.33 / 0.08, 7 0.39 / 0.11, 64 0.53 / 0.30, 128 0.68 / 0.41 (one
+// output a thread: 0.12, 0.17, 0.40, 0.68). Longer lines take so much shared memory that few blocks fit
+// an SM: 700 x 700 spinodals of 300 planes 0.75 / 0.67, 512 1.03 / 1.16, 1024 2.17 / 3.98.
 // ---------------------------------------------------------------------------------------
-constexpr int kZThreads = 512;
+constexpr int kZShort = 128;
 
-__global__ void __launch_bounds__(kZThreads) edt_pass_z(uint32_t* __restrict__ g, int SX, int SY, int SZ, int pitch,
+template <int kZThreads>
+__global__ void __launch_bounds__(kZThreads) edt_pass_z(uint32_t* __restrict__ g, int SX, int SY, int SZ, int pitch, int short_bins,
                                                         unsigned long long* __restrict__ hist, size_t hist_len,
                                                         unsigned int* __restrict__ max_out) {
     extern __shared__ uint32_t smem[];
-    unsigned int* h_small = smem;         // [kHistSmall]
-    uint32_t* tile = smem + kHistSmall;   // [SZ][pitch]
+    const int bins = kZThreads == 512 ? kHistSmall : short_bins;
+    unsigned int* h_small = smem;   // [bins]
+    uint32_t* tile = smem + bins;   // [SZ][pitch]
     const int tiles_y = (SY + kTileY - 1) / kTileY;
     const int x = blockIdx.x / tiles_y;
     const int y0 = (blockIdx.x % tiles_y) * kTileY;
@@ -382,7 +390,7 @@ __global__ void __launch_bounds__(kZThreads) edt_pass_z(uint32_t* __restrict__ g
     const int yy = threadIdx.x % kTileY, z0 = threadIdx.x / kTileY;
     constexpr int kRows = kZThreads / kTileY;  // z-slices the block loads at a time
 
-    for (int i = threadIdx.x; i < kHistSmall; i += kZThreads) h_small[i] = 0;
+    for (int i = threadIdx.x; i < bins; i += kZThreads) h_small[i] = 0;
 #pragma unroll 8
     for (int z = z0; z < SZ; z += kRows) tile[z * pitch + yy] = yy < ny ? base[z * plane + yy] : 0u;
     __syncthreads();
@@ -407,7 +415,7 @@ __global__ void __launch_bounds__(kZThreads) edt_pass_z(uint32_t* __restrict__ g
             const int m = min(mxy, min(z, SZ - 1 - z));
             // e <= m^2 <=> the ball of radius sqrt(e) stays inside the image (EDC.cpp:316-327).
             if (e <= static_cast<uint32_t>(m) * static_cast<uint32_t>(m)) {  // m < 2^15 here
-                if (e < kHistSmall) atomicAdd(&h_small[e], 1u);
+                if (e < static_cast<uint32_t>(bins)) atomicAdd(&h_small[e], 1u);
                 else if (e < hist_len) atomicAdd(&hist[e], 1ull);
             }
         }
@@ -415,7 +423,7 @@ __global__ void __launch_bounds__(kZThreads) edt_pass_z(uint32_t* __restrict__ g
     local_max = __reduce_max_sync(0xFFFFFFFFu, local_max);
     if ((threadIdx.x & 31) == 0 && local_max) atomicMax(max_out, local_max);
     __syncthreads();
-    for (int i = threadIdx.x; i < kHistSmall && i < static_cast<int>(hist_len); i += kZThreads)
+    for (int i = threadIdx.x; i < bins && i < static_cast<int>(hist_len); i += kZThreads)
         if (h_small[i]) atomicAdd(&hist[i], static_cast<unsigned long long>(h_small[i]));
 }
 
@@ -438,7 +446,8 @@ void edt_smem_attributes(size_t optin) {
     PMA_CUDA(cudaFuncSetAttribute(edt_pass_x<1>, attr, bytes));
     PMA_CUDA(cudaFuncSetAttribute(edt_pass_x<4>, attr, bytes));
     PMA_CUDA(cudaFuncSetAttribute(edt_pass_y, attr, bytes));
-    PMA_CUDA(cudaFuncSetAttribute(edt_pass_z, attr, bytes));
+    PMA_CUDA(cudaFuncSetAttribute(edt_pass_z<128>, attr, bytes));
+    PMA_CUDA(cudaFuncSetAttribute(edt_pass_z<512>, attr, bytes));
     g_attr_devices.push_back(dev);
 }
 
@@ -502,9 +511,14 @@ void edt_passes(const char* who, const uint8_t* solid, pma_dims d, uint32_t* edt
         edt_pass_y<<<static_cast<unsigned>(blocks), warps * 32, smem, s>>>(edt2, SY, rows, static_cast<int>(row_words));
     });
     timed("edt_pass_z", [&] {
-        auto smem = [&](int pitch) { return static_cast<size_t>(SZ) * pitch * 4 + kHistSmall * 4; };
+        // balls inside the image have r^2 <= half^2; hist_len >= kHistSmall covers the rounding
+        const long long half = (std::min(SX, std::min(SY, SZ)) - 1) / 2;
+        const int bins = SZ > kZShort ? kHistSmall : static_cast<int>((std::min<long long>(kHistSmall, half * half + 1) + 3) / 4 * 4);
+        auto smem = [&](int pitch) { return (static_cast<size_t>(SZ) * pitch + bins) * 4; };
         const int pitch = smem(18) <= smem_optin ? 18 : 16;
-        edt_pass_z<<<static_cast<unsigned>(tiles), kZThreads, smem(pitch), s>>>(edt2, SX, SY, SZ, pitch, hist, hist_len, d_max);
+        const unsigned blocks = static_cast<unsigned>(tiles);
+        if (SZ <= kZShort) edt_pass_z<128><<<blocks, 128, smem(pitch), s>>>(edt2, SX, SY, SZ, pitch, bins, hist, hist_len, d_max);
+        else edt_pass_z<512><<<blocks, 512, smem(pitch), s>>>(edt2, SX, SY, SZ, pitch, bins, hist, hist_len, d_max);
     });
 }
 
