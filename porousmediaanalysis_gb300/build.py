@@ -22,7 +22,7 @@ CLI = os.path.join(OUT, "pma")
 
 
 def _headers():
-    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     hs.append(os.path.join(INCLUDE, "pma.h"))
     return hs
 
