@@ -56,10 +56,10 @@ ALGO_BYTES = {
     "edt_pass_x": 3.0,          # 1 B mask read + 2 B distance written
     "edt_pass_y": 6.0,          # 2 B read + 4 B write
     "edt_pass_z": 8.0,          # 4 B read + 4 B write
-    "balls_candidates": 16.0,   # 2 x (4 B EDT read) + 8 B key init write
-    "balls_tile_gather": 20.0,  # 4 B EDT read + 16 B (radius, centre x, y, z) written
-    "uf_hook": 12.0,            # 4 B crad read + 4 B parent read + 4 B parent write
-    "geo_bucket": 17.0,         # per settled voxel: 1 B mask + 8 B read + 8 B write (float64)
+    "balls_candidates": 6.0,    # 4 B EDT read + 1 B flag written and read by the selection
+    "balls_tile_gather": 12.0,  # 4 B EDT read + 8 B key (radius and centre) written
+    "uf_hook": 8.0,             # 4 B crad read + 4 B parent read; few parents are written
+    "geo_bucket": 20.0,         # per settled voxel: 8 B distance read and written (float64) + 4 B cavity id
     "level_sets": 0.0,          # plateau graph work, not per voxel
     "ws_generations": 24.0,     # 4 B crad read + 4 B claim write + 2 x 8 B frontier entry
 }

@@ -29,9 +29,9 @@
 // a 704 x 768 x 811 spinodal) took 18 ms in the count and again in the fill; the groups' lists have a
 // quarter of the entries, and the split reads them in order. That spinodal, ms: kept centres 13 -> 2.9 (bricks),
 // floors and counts 23 -> 4.6 (groups; a quarter of the centres for the floors, 9 -> 2.5), fill 19 -> 7.0
-// and split 7.9, gather 117 -> 38 (least key by 32-bit reductions and 2 x 4 x 4 boxes 82, centres by
+// and split 7.3, gather 117 -> 38 (least key by 32-bit reductions and 2 x 4 x 4 boxes 82, centres by
 // descending radius 73, the box of the lanes still open 44, lists in the order of the radii 41, four CTAs
-// an SM 38); stage 170 -> 66. A gather that filters its group's list itself took 68 ms, one that keeps the
+// an SM 38); stage 170 -> 65. A gather that filters its group's list itself took 68 ms, one that keeps the
 // lists' own order 45, lists in chunks of 1024 44.
 #include <thrust/iterator/counting_iterator.h>
 

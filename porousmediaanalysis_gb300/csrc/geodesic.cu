@@ -148,8 +148,9 @@ __device__ __forceinline__ unsigned long long geo_dilate(F mask, int x, int z) {
 // unsigned integers (their bits order as the values do): solid reads as infinity, unreached as
 // the largest finite value. The least neighbour per step weight is found first and only three
 // sums are formed (rounding is monotone).
-// What bounds it: the bricks' loads (27 KB of a float64 brick with its halo, once for each of the
-// about 25 steps that the front takes through a brick: 330 B a voxel) and the block's barriers.
+// What bounds it: the block's barriers and the bricks' loads (27 KB of a float64 brick with its halo, once
+// for each of the about 25 steps that the front takes through a brick: 330 B a voxel). A mid-front step at
+// 512^3: 30 and 25 % of the cycles between two instructions, issue slots 49 % and DRAM 42 % busy.
 // Five blocks an SM (48 registers, the loads of a whole brick in flight); six spill (1024^3 spinodal,
 // float64: 121 against 157 ms). Before and after, ms: that volume 253 -> 121 (a step of 14000
 // bricks 130 us, 2.9 TB/s of brick loads); 301 x 257 x 411 field, float32, D3Q7 10.2 -> 6.6.
@@ -306,8 +307,9 @@ __global__ void __launch_bounds__(kBrickThreads, 5)
             if (nz >= 0 && nz < b.BZ && nx >= 0 && nx < b.BX && ny >= 0 && ny < b.BY)
                 geo_list(b, static_cast<uint32_t>((nz * b.BX + nx) * b.BY + ny), k + 1, epoch0);
         }
-        // no barrier: what the next brick's loads overwrite was read before the last one, and the
-        // thread that clears s_next is one of those that just read it
+        // no barrier: what the next brick's loads overwrite was read before the last one, and s_next is read
+        // by the warp whose first thread clears it, behind votes of the whole warp (put's): every lane has
+        // branched on its bit by then
     }
     for (int o = 16; o > 0; o >>= 1) my_settled += __shfl_xor_sync(0xFFFFFFFFu, my_settled, o);
     my_walls = __reduce_or_sync(0xFFFFFFFFu, my_walls);

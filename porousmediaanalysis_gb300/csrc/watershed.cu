@@ -388,7 +388,8 @@ __device__ __forceinline__ WsStrip ws_strip(unsigned long long c, unsigned long 
     return k;
 }
 
-// Lane i: the strip's i-th node (at most six); lane k: the touch bits of the strip's k-th 32 events.
+// Lane i: the strip's i-th node (at most four with kStrip 2); lane k: the touch bits of the strip's k-th 32 events.
+static_assert((26 + kStrip * 32 + 26) / 27 <= 32, "a lane per node of a strip");
 struct WsAhead {
     uint32_t v, p, touched;
 };
@@ -771,7 +772,7 @@ __device__ __noinline__ uint32_t ws_small_generation(const WsState& s, WsSmallSh
     if (tid < m) sh.won[tid] = 0;
     __syncthreads();
     const uint32_t nev = m * 27, seq0 = first * 27;
-    // claims, as ws_claim_event; bit k of touched: this thread's k-th event touched an unclaimed
+    // claims, as ws_claim_strip; bit k of touched: this thread's k-th event touched an unclaimed
     // voxel. Two events a turn, their loads in flight together.
     uint32_t touched = 0;
 #pragma unroll 1
@@ -816,7 +817,7 @@ __device__ __noinline__ uint32_t ws_small_generation(const WsState& s, WsSmallSh
     }
     if (cl) cg::this_cluster().sync();
     else __syncthreads();
-    // resolve the touches, as ws_resolve_event; a claim of the same depth sets its stencil
+    // resolve the touches, as ws_resolve_strip; a claim of the same depth sets its stencil
     // position's bit in its node's word
 #pragma unroll 1
     for (unsigned k = 0; k * kSmallThreads + warp * 32 < nev; k += 2) {
